@@ -14,7 +14,6 @@
 #include "field.cuh"
 #include "inverse.cuh"
 #include "lazy.cuh"
-#include "lazy64.cuh"
 
 namespace h2b {
 
@@ -243,55 +242,6 @@ H2B_DEV void xyzzl_madd(G1XyzzL& acc, const FqL& qx, const FqL& qy)
     acc.ZZZ = zz.b;
 }
 
-// dbl-2008-s-1 and add-2008-s in limb form with out-of-line latency-oriented
-// products, for the single-thread tails of the MSM (window combination, final
-// doubling chain): one warp runs them, so latency sets the time; each
-// product's own critical path is short and the formula's code stays small
-// (fully inlined formulas measured twice as slow there).
-H2B_DEV G1XyzzL xyzzl_dbl(const G1XyzzL& p)
-{
-    if (is_inf(p) || fl_is_zero_mod(p.Y)) return xyzzl_inf();
-    const FqL U = fl_add(p.Y, p.Y);
-    const FqL V = fl_sqr_ilp(U);
-    const FqL xx = fl_sqr_ilp(p.X);
-    const FqL W = fl_mul_ilp(U, V);
-    const FqL S = fl_mul_ilp(p.X, V);
-    const FqL M = fl_add(fl_add(xx, xx), xx);
-    G1XyzzL r;
-    r.ZZ = fl_mul_ilp(V, p.ZZ);
-    r.ZZZ = fl_mul_ilp(W, p.ZZZ);
-    r.X = fl_sub(fl_sqr_ilp(M), fl_add(S, S));
-    r.Y = fl_sub(fl_mul_ilp(M, fl_sub(S, r.X)), fl_mul_ilp(W, p.Y));
-    return r;
-}
-
-H2B_DEV void xyzzl_add(G1XyzzL& acc, const G1XyzzL& q)
-{
-    if (is_inf(q)) return;
-    if (is_inf(acc)) { acc = q; return; }
-    const FqL U1 = fl_mul_ilp(acc.X, q.ZZ);
-    const FqL U2 = fl_mul_ilp(q.X, acc.ZZ);
-    const FqL S1 = fl_mul_ilp(acc.Y, q.ZZZ);
-    const FqL S2 = fl_mul_ilp(q.Y, acc.ZZZ);
-    const FqL P = fl_sub(U2, U1);
-    const FqL R = fl_sub(S2, S1);
-    if (fl_is_zero_mod(P)) {
-        acc = fl_is_zero_mod(R) ? xyzzl_dbl(acc) : xyzzl_inf();
-        return;
-    }
-    const FqL PP = fl_sqr_ilp(P);
-    const FqL RR = fl_sqr_ilp(R);
-    const FqL zz = fl_mul_ilp(acc.ZZ, q.ZZ);
-    const FqL zzz = fl_mul_ilp(acc.ZZZ, q.ZZZ);
-    const FqL PPP = fl_mul_ilp(P, PP);
-    const FqL Q = fl_mul_ilp(U1, PP);
-    const FqL X3 = fl_sub(fl_sub(RR, PPP), fl_add(Q, Q));
-    acc.Y = fl_sub(fl_mul_ilp(R, fl_sub(Q, X3)), fl_mul_ilp(S1, PPP));
-    acc.X = X3;
-    acc.ZZ = fl_mul_ilp(zz, PP);
-    acc.ZZZ = fl_mul_ilp(zzz, PPP);
-}
-
 // ---- XYZZ in the lazy form (R = 2^261), for the bucket accumulation -------
 // Bounds (multiples of p) that every step relies on are written beside it;
 // products follow (1 + 0.0059 a b) p (lazy.cuh).  The accumulator keeps
@@ -373,139 +323,109 @@ static __device__ __noinline__ void st_xyzzz(G1Xyzz* dst, const G1XyzzZ p, const
     st_xyzz(dst, r);
 }
 
-// ---- XYZZ in the FP64 lazy form (R' = 2^260), accumulate variant 6 -------
-// The same formulas as the R = 2^261 form above; products follow
-// (1 + 0.0118 a b) p, so the accumulator bounds are X < 5.4p, Y < 3.45p,
-// ZZ and ZZZ < 1.2p (stable from one addition to the next); affine inputs
-// are qx < p and qy < 2p.
+// ---- XYZZ with coordinates in [0, 2p) ---------------------------------------
+// The memory image with residues in [0, 2p): products without their closing
+// subtraction (mont_mul_eo_lazy: 1.76p), sums and differences corrected by
+// 2p.  Every function takes and returns coordinates below 2p; infinity is the
+// all-zero ZZ (no product of nonzero residues is 0, and the exceptional cases
+// write zeros).  INL: products inline (the bucket accumulation) or one shared
+// out-of-line body per product (the tails, whose code must stay small).
 
-typedef Fd<FqCfg> FqD;
-
-struct G1XyzzD {
-    FqD X, Y, ZZ, ZZZ;
-};
-
-H2B_DEV G1XyzzD xyzzd_inf()
+template <bool INL>
+H2B_DEV Fq qmul(const Fq& a, const Fq& b)
 {
-    G1XyzzD r;
-    r.X = fd_zero<FqCfg>(); r.Y = fd_zero<FqCfg>(); r.ZZ = fd_zero<FqCfg>(); r.ZZZ = fd_zero<FqCfg>();
+    return INL ? mont_mul_eo_lazy<FqCfg>(a, b) : mont_mul_lazy_outline<FqCfg>(a, b);
+}
+
+template <bool INL>
+H2B_DEV Fq qsqr(const Fq& a)
+{
+    return INL ? mont_sqr_eo_lazy<FqCfg>(a) : mont_sqr_lazy_outline<FqCfg>(a);
+}
+
+H2B_DEV Fq qadd(const Fq& a, const Fq& b) { return add2p<FqCfg>(a, b); }
+H2B_DEV Fq qsub(const Fq& a, const Fq& b) { return sub2p<FqCfg>(a, b); }
+
+// the canonical memory image (infinity stays ZZ = 0)
+H2B_DEV G1Xyzz xyzze_canonical(const G1Xyzz& a)
+{
+    G1Xyzz r;
+    r.X = canon2p<FqCfg>(a.X); r.Y = canon2p<FqCfg>(a.Y);
+    r.ZZ = canon2p<FqCfg>(a.ZZ); r.ZZZ = canon2p<FqCfg>(a.ZZZ);
+    return r;
+}
+H2B_DEV void st_xyzze(G1Xyzz* p, const G1Xyzz& a) { st_xyzz(p, xyzze_canonical(a)); }
+
+// 2 q for an affine q that is not infinity (y != 0 on this curve: the group order is odd)
+template <bool INL>
+__device__ __noinline__ G1Xyzz xyzze_dbl_affine(const Fq qx, const Fq qy)
+{
+    const Fq U = qadd(qy, qy), V = qsqr<INL>(U), xx = qsqr<INL>(qx);
+    const Fq W = qmul<INL>(U, V), S = qmul<INL>(qx, V), M = qadd(qadd(xx, xx), xx);
+    G1Xyzz r;
+    r.X = qsub(qsqr<INL>(M), qadd(S, S));
+    r.Y = qsub(qmul<INL>(M, qsub(S, r.X)), qmul<INL>(W, qy));
+    r.ZZ = V;
+    r.ZZZ = W;
     return r;
 }
 
-H2B_DEV bool is_inf(const G1XyzzD& p) { return fd_is_zero(p.ZZ); }
-
-// 2 q for an affine q (qx < p, qy < 2p, qy != 0): dbl-2008-s-1 with Z = 1.
-H2B_DEV G1XyzzD xyzzd_dbl_affine(const FqD& qx, const FqD& qy)
+// dbl-2008-s-1 (a = 0)
+template <bool INL>
+H2B_DEV G1Xyzz xyzze_dbl(const G1Xyzz& p)
 {
-    const FqD U = fd_add(qy, qy);                              // < 4p
-    const Fd2<FqCfg> vx = fd_mul2(U, U, qx, qx);               // V < 1.19p, xx < 1.012p
-    const Fd2<FqCfg> ws = fd_mul2(U, vx.a, qx, vx.a);          // W < 1.057p, S < 1.015p
-    const FqD M = fd_add(fd_add(vx.b, vx.b), vx.b);            // < 3.04p
-    const Fd2<FqCfg> mm = fd_mul2(M, M, ws.a, qy);             // MM < 1.11p, W y < 1.025p
-    G1XyzzD r;
-    r.X = fd_sub<FqCfg, 3>(mm.a, fd_add(ws.b, ws.b));          // 2S < 2.03p; X3 < 4.11p
-    const FqD t1 = fd_mul_call(M, fd_sub<FqCfg, 5>(ws.b, r.X)); // S - X3 + 5p < 6.02p; t1 < 1.22p
-    r.Y = fd_sub<FqCfg, 2>(t1, mm.b);                          // < 3.22p
-    r.ZZ = vx.a;                                               // < 1.19p
-    r.ZZZ = ws.a;                                              // < 1.057p
+    if (is_inf(p)) return xyzz_inf();
+    const Fq U = qadd(p.Y, p.Y), V = qsqr<INL>(U), xx = qsqr<INL>(p.X);
+    const Fq W = qmul<INL>(U, V), S = qmul<INL>(p.X, V), M = qadd(qadd(xx, xx), xx);
+    G1Xyzz r;
+    r.ZZ = qmul<INL>(V, p.ZZ);
+    r.ZZZ = qmul<INL>(W, p.ZZZ);
+    r.X = qsub(qsqr<INL>(M), qadd(S, S));
+    r.Y = qsub(qmul<INL>(M, qsub(S, r.X)), qmul<INL>(W, p.Y));
     return r;
 }
 
-// madd-2008-s: acc += (qx, qy), q affine and not infinity.  PP == 0 mod p
-// exactly when P is, so the equal-x test reads the square.
-H2B_DEV void xyzzd_madd(G1XyzzD& acc, const FqD& qx, const FqD& qy)
+// madd-2008-s: acc += (qx, qy), an affine point that is not infinity
+template <bool INL>
+H2B_DEV void xyzze_madd(G1Xyzz& acc, const Fq& qx, const Fq& qy)
 {
     if (is_inf(acc)) {
-        acc.X = qx; acc.Y = qy; acc.ZZ = fd_one<FqCfg>(); acc.ZZZ = fd_one<FqCfg>();
+        acc.X = qx; acc.Y = qy; acc.ZZ = Fq::one(); acc.ZZZ = Fq::one();
         return;
     }
-    const Fd2<FqCfg> us = fd_mul2(qx, acc.ZZ, qy, acc.ZZZ);   // U2 < 1.015p, S2 < 1.03p
-    const FqD P = fd_sub<FqCfg, 6>(us.a, acc.X);               // X1 < 5.4p; P < 7.02p
-    const FqD R = fd_sub<FqCfg, 4>(us.b, acc.Y);               // Y1 < 3.45p; R < 5.03p
-    const Fd2<FqCfg> sq = fd_mul2(P, P, R, R);                 // PP < 1.59p, RR < 1.3p
-    if (fd_is_zero_mod(sq.a)) {
-        acc = fd_is_zero_mod(sq.b) ? xyzzd_dbl_affine(qx, qy) : xyzzd_inf();
+    const Fq P = qsub(qmul<INL>(qx, acc.ZZ), acc.X);
+    const Fq R = qsub(qmul<INL>(qy, acc.ZZZ), acc.Y);
+    if (is_zero2p<FqCfg>(P)) {
+        acc = is_zero2p<FqCfg>(R) ? xyzze_dbl_affine<false>(qx, qy) : xyzz_inf();
         return;
     }
-    const Fd2<FqCfg> pq = fd_mul2(P, sq.a, acc.X, sq.a);       // PPP < 1.14p, Q < 1.11p
-    const FqD X3 = fd_sub<FqCfg, 4>(sq.b, fd_add(pq.a, fd_add(pq.b, pq.b)));  // PPP + 2Q < 3.36p; X3 < 5.3p
-    const Fd2<FqCfg> yy = fd_mul2(R, fd_sub<FqCfg, 6>(pq.b, X3), acc.Y, pq.a); // Q - X3 + 6p < 7.11p;
-                                                                              // < 1.43p, < 1.05p
-    const Fd2<FqCfg> zz = fd_mul2(acc.ZZ, sq.a, acc.ZZZ, pq.a); // < 1.03p, < 1.02p
-    acc.Y = fd_sub<FqCfg, 2>(yy.a, yy.b);                     // < 3.43p
-    acc.X = X3;
-    acc.ZZ = zz.a;
-    acc.ZZZ = zz.b;
+    const Fq PP = qsqr<INL>(P);
+    const Fq PPP = qmul<INL>(P, PP), Q = qmul<INL>(acc.X, PP);
+    acc.ZZ = qmul<INL>(acc.ZZ, PP);
+    acc.ZZZ = qmul<INL>(acc.ZZZ, PPP);
+    acc.X = qsub(qsub(qsqr<INL>(R), PPP), qadd(Q, Q));
+    acc.Y = qsub(qmul<INL>(R, qsub(Q, acc.X)), qmul<INL>(acc.Y, PPP));
 }
 
-// Two independent madd-2008-s additions, a0 += q0 and a1 += q1, whose
-// products share out-of-line calls four at a time (the latency of one chain
-// hides behind the other).  When an accumulator is at infinity or a
-// square reads zero (equal x: a doubling or P + (-P)) the two additions run
-// one after the other through xyzzd_madd instead; no accumulator has been
-// written when that is decided.  Bounds as in xyzzd_madd.
-H2B_DEV void xyzzd_madd_x2(G1XyzzD& a0, const FqD& q0x, const FqD& q0y, G1XyzzD& a1, const FqD& q1x,
-                           const FqD& q1y)
+// add-2008-s: acc += q
+template <bool INL>
+H2B_DEV void xyzze_add(G1Xyzz& acc, const G1Xyzz& q)
 {
-    if (is_inf(a0) || is_inf(a1)) {
-        xyzzd_madd(a0, q0x, q0y);
-        xyzzd_madd(a1, q1x, q1y);
+    if (is_inf(q)) return;
+    if (is_inf(acc)) { acc = q; return; }
+    const Fq U1 = qmul<INL>(acc.X, q.ZZ), S1 = qmul<INL>(acc.Y, q.ZZZ);
+    const Fq P = qsub(qmul<INL>(q.X, acc.ZZ), U1), R = qsub(qmul<INL>(q.Y, acc.ZZZ), S1);
+    if (is_zero2p<FqCfg>(P)) {
+        if (is_zero2p<FqCfg>(R)) acc = xyzze_dbl<INL>(acc);
+        else acc = xyzz_inf();
         return;
     }
-    const Fd4<FqCfg> us = fd_mul4(q0x, a0.ZZ, q0y, a0.ZZZ, q1x, a1.ZZ, q1y, a1.ZZZ);
-    const FqD P0 = fd_sub<FqCfg, 6>(us.a, a0.X), R0 = fd_sub<FqCfg, 4>(us.b, a0.Y);
-    const FqD P1 = fd_sub<FqCfg, 6>(us.c, a1.X), R1 = fd_sub<FqCfg, 4>(us.d, a1.Y);
-    const Fd4<FqCfg> sq = fd_mul4(P0, P0, R0, R0, P1, P1, R1, R1);
-    if (fd_is_zero_mod(sq.a) || fd_is_zero_mod(sq.c)) {
-        xyzzd_madd(a0, q0x, q0y);
-        xyzzd_madd(a1, q1x, q1y);
-        return;
-    }
-    const Fd4<FqCfg> pq = fd_mul4(P0, sq.a, a0.X, sq.a, P1, sq.c, a1.X, sq.c);
-    const FqD X30 = fd_sub<FqCfg, 4>(sq.b, fd_add(pq.a, fd_add(pq.b, pq.b)));
-    const FqD X31 = fd_sub<FqCfg, 4>(sq.d, fd_add(pq.c, fd_add(pq.d, pq.d)));
-    const Fd4<FqCfg> yy = fd_mul4(R0, fd_sub<FqCfg, 6>(pq.b, X30), a0.Y, pq.a, R1, fd_sub<FqCfg, 6>(pq.d, X31), a1.Y,
-                                  pq.c);
-    const Fd4<FqCfg> zz = fd_mul4(a0.ZZ, sq.a, a0.ZZZ, pq.a, a1.ZZ, sq.c, a1.ZZZ, pq.c);
-    a0.Y = fd_sub<FqCfg, 2>(yy.a, yy.b);
-    a0.X = X30;
-    a0.ZZ = zz.a;
-    a0.ZZZ = zz.b;
-    a1.Y = fd_sub<FqCfg, 2>(yy.c, yy.d);
-    a1.X = X31;
-    a1.ZZ = zz.c;
-    a1.ZZZ = zz.d;
-}
-
-// Canonical memory image of the accumulator (infinity stays ZZ = 0): four
-// products by 2^256 mod p (each below 1.07p), then conditional subtractions.
-static __device__ __noinline__ G1Xyzz xyzzd_canonical(const G1XyzzD p)
-{
-    const FqD r256 = fd_r256<FqCfg>();
-    const Fd4<FqCfg> a = fd_mul4(p.X, r256, p.Y, r256, p.ZZ, r256, p.ZZZ, r256);
-    G1Xyzz r;
-    r.X = fd_canonical(a.a); r.Y = fd_canonical(a.b);
-    r.ZZ = fd_canonical(a.c); r.ZZZ = fd_canonical(a.d);
-    return r;
-}
-
-// The sum of two accumulators, stored in the canonical memory image.
-static __device__ __noinline__ void st_xyzzd_pair(G1Xyzz* dst, const G1XyzzD p0, const G1XyzzD p1)
-{
-    G1Xyzz r = xyzzd_canonical(p0);
-    if (!is_inf(p1)) xyzz_add(r, xyzzd_canonical(p1));
-    st_xyzz(dst, r);
-}
-
-static __device__ __noinline__ void st_xyzzd(G1Xyzz* dst, const G1XyzzD p)
-{
-    const FqD r256 = fd_r256<FqCfg>();
-    const Fd2<FqCfg> a = fd_mul2(p.X, r256, p.Y, r256);
-    const Fd2<FqCfg> b = fd_mul2(p.ZZ, r256, p.ZZZ, r256);
-    G1Xyzz r;
-    r.X = fd_canonical(a.a); r.Y = fd_canonical(a.b);
-    r.ZZ = fd_canonical(b.a); r.ZZZ = fd_canonical(b.b);
-    st_xyzz(dst, r);
+    const Fq PP = qsqr<INL>(P);
+    const Fq PPP = qmul<INL>(P, PP), Q = qmul<INL>(U1, PP);
+    acc.ZZ = qmul<INL>(qmul<INL>(acc.ZZ, q.ZZ), PP);
+    acc.ZZZ = qmul<INL>(qmul<INL>(acc.ZZZ, q.ZZZ), PPP);
+    acc.X = qsub(qsub(qsqr<INL>(R), PPP), qadd(Q, Q));
+    acc.Y = qsub(qmul<INL>(R, qsub(Q, acc.X)), qmul<INL>(S1, PPP));
 }
 
 // ---- lane-parallel XYZZ formulas for one warp ------------------------------
@@ -518,76 +438,73 @@ static __device__ __noinline__ void st_xyzzd(G1Xyzz* dst, const G1XyzzD p)
 // product latencies instead of 9, an addition 4 instead of 14.  All 32 lanes
 // must call these with identical arguments; every lane ends with the result.
 
-H2B_DEV FqL lane_bcast(const FqL& v, int src)
+H2B_DEV Fq lane_bcast(const Fq& v, int src)
 {
-    FqL r;
+    Fq r;
 #pragma unroll
-    for (int i = 0; i < 9; i++) r.l[i] = __shfl_sync(0xffffffffu, v.l[i], src);
+    for (int i = 0; i < 8; i++) r.v[i] = __shfl_sync(0xffffffffu, v.v[i], src);
     return r;
 }
 
 // operand k of a level for lane slot s = lane mod 8 (slots past the last operand repeat it)
-H2B_DEV FqL lane_pick(int s, const FqL& a0, const FqL& a1, const FqL& a2, const FqL& a3, const FqL& a4,
-                      const FqL& a5)
+H2B_DEV Fq lane_pick(int s, const Fq& a0, const Fq& a1, const Fq& a2, const Fq& a3, const Fq& a4, const Fq& a5)
 {
-    FqL r;
+    Fq r;
 #pragma unroll
-    for (int i = 0; i < 9; i++)
-        r.l[i] = s == 0 ? a0.l[i] : s == 1 ? a1.l[i] : s == 2 ? a2.l[i] : s == 3 ? a3.l[i] : s == 4 ? a4.l[i]
-                                                                                                    : a5.l[i];
+    for (int i = 0; i < 8; i++)
+        r.v[i] = s == 0 ? a0.v[i] : s == 1 ? a1.v[i] : s == 2 ? a2.v[i] : s == 3 ? a3.v[i] : s == 4 ? a4.v[i]
+                                                                                                    : a5.v[i];
     return r;
 }
 
 H2B_DEV int lane_slot() { return (int)(threadIdx.x & 7); }
 
 // dbl-2008-s-1 in three levels: {U^2, X^2}, {U V, X V, V ZZ, M^2}, {W ZZZ, M (S - X3), W Y}.
-H2B_DEV G1XyzzL xyzzw_dbl(const G1XyzzL& p)
+H2B_DEV G1Xyzz xyzzw_dbl(const G1Xyzz& p)
 {
-    if (is_inf(p) || fl_is_zero_mod(p.Y)) return xyzzl_inf();
+    if (is_inf(p)) return xyzz_inf();
     const int s = lane_slot();
-    const FqL U = fl_add(p.Y, p.Y);
-    FqL a = (s & 1) ? p.X : U;
-    FqL r = fl_mul_ilp(a, a);
-    const FqL V = lane_bcast(r, 0), xx = lane_bcast(r, 1);
-    const FqL M = fl_add(fl_add(xx, xx), xx);
-    r = fl_mul_ilp(lane_pick(s, U, p.X, V, M, M, M), lane_pick(s, V, V, p.ZZ, M, M, M));
-    const FqL W = lane_bcast(r, 0), S = lane_bcast(r, 1);
-    G1XyzzL o;
+    const Fq U = qadd(p.Y, p.Y);
+    Fq r = qsqr<false>((s & 1) ? p.X : U);
+    const Fq V = lane_bcast(r, 0), xx = lane_bcast(r, 1);
+    const Fq M = qadd(qadd(xx, xx), xx);
+    r = qmul<false>(lane_pick(s, U, p.X, V, M, M, M), lane_pick(s, V, V, p.ZZ, M, M, M));
+    const Fq W = lane_bcast(r, 0), S = lane_bcast(r, 1);
+    G1Xyzz o;
     o.ZZ = lane_bcast(r, 2);
-    o.X = fl_sub(lane_bcast(r, 3), fl_add(S, S));
-    const FqL sx = fl_sub(S, o.X);
-    r = fl_mul_ilp(lane_pick(s, W, M, W, W, W, W), lane_pick(s, p.ZZZ, sx, p.Y, p.Y, p.Y, p.Y));
+    o.X = qsub(lane_bcast(r, 3), qadd(S, S));
+    const Fq sx = qsub(S, o.X);
+    r = qmul<false>(lane_pick(s, W, M, W, W, W, W), lane_pick(s, p.ZZZ, sx, p.Y, p.Y, p.Y, p.Y));
     o.ZZZ = lane_bcast(r, 0);
-    o.Y = fl_sub(lane_bcast(r, 1), lane_bcast(r, 2));
+    o.Y = qsub(lane_bcast(r, 1), lane_bcast(r, 2));
     return o;
 }
 
 // add-2008-s in four levels: {U1, U2, S1, S2, ZZ1 ZZ2, ZZZ1 ZZZ2}, {P^2, R^2},
 // {P PP, U1 PP, zz PP}, {R (Q - X3), S1 PPP, zzz PPP}.
-H2B_DEV void xyzzw_add(G1XyzzL& acc, const G1XyzzL& q)
+H2B_DEV void xyzzw_add(G1Xyzz& acc, const G1Xyzz& q)
 {
     if (is_inf(q)) return;
     if (is_inf(acc)) { acc = q; return; }
     const int s = lane_slot();
-    FqL r = fl_mul_ilp(lane_pick(s, acc.X, q.X, acc.Y, q.Y, acc.ZZ, acc.ZZZ),
+    Fq r = qmul<false>(lane_pick(s, acc.X, q.X, acc.Y, q.Y, acc.ZZ, acc.ZZZ),
                        lane_pick(s, q.ZZ, acc.ZZ, q.ZZZ, acc.ZZZ, q.ZZ, q.ZZZ));
-    const FqL U1 = lane_bcast(r, 0), S1 = lane_bcast(r, 2);
-    const FqL zz = lane_bcast(r, 4), zzz = lane_bcast(r, 5);
-    const FqL P = fl_sub(lane_bcast(r, 1), U1);
-    const FqL R = fl_sub(lane_bcast(r, 3), S1);
-    if (fl_is_zero_mod(P)) {
-        acc = fl_is_zero_mod(R) ? xyzzw_dbl(acc) : xyzzl_inf();
+    const Fq U1 = lane_bcast(r, 0), S1 = lane_bcast(r, 2);
+    const Fq zz = lane_bcast(r, 4), zzz = lane_bcast(r, 5);
+    const Fq P = qsub(lane_bcast(r, 1), U1), R = qsub(lane_bcast(r, 3), S1);
+    if (is_zero2p<FqCfg>(P)) {
+        if (is_zero2p<FqCfg>(R)) acc = xyzzw_dbl(acc);
+        else acc = xyzz_inf();
         return;
     }
-    FqL a = (s & 1) ? R : P;
-    r = fl_mul_ilp(a, a);
-    const FqL PP = lane_bcast(r, 0), RR = lane_bcast(r, 1);
-    r = fl_mul_ilp(lane_pick(s, P, U1, zz, zz, zz, zz), PP);
-    const FqL PPP = lane_bcast(r, 0), Q = lane_bcast(r, 1);
+    r = qsqr<false>((s & 1) ? R : P);
+    const Fq PP = lane_bcast(r, 0), RR = lane_bcast(r, 1);
+    r = qmul<false>(lane_pick(s, P, U1, zz, zz, zz, zz), PP);
+    const Fq PPP = lane_bcast(r, 0), Q = lane_bcast(r, 1);
     acc.ZZ = lane_bcast(r, 2);
-    const FqL X3 = fl_sub(fl_sub(RR, PPP), fl_add(Q, Q));
-    r = fl_mul_ilp(lane_pick(s, R, S1, zzz, zzz, zzz, zzz), lane_pick(s, fl_sub(Q, X3), PPP, PPP, PPP, PPP, PPP));
-    acc.Y = fl_sub(lane_bcast(r, 0), lane_bcast(r, 1));
+    const Fq X3 = qsub(qsub(RR, PPP), qadd(Q, Q));
+    r = qmul<false>(lane_pick(s, R, S1, zzz, zzz, zzz, zzz), lane_pick(s, qsub(Q, X3), PPP, PPP, PPP, PPP, PPP));
+    acc.Y = qsub(lane_bcast(r, 0), lane_bcast(r, 1));
     acc.ZZZ = lane_bcast(r, 2);
     acc.X = X3;
 }

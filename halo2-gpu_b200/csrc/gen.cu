@@ -52,7 +52,7 @@ __global__ void k_random_fr(Fr* __restrict__ out, uint64_t n, uint64_t seed, int
             }
             Fr r2 = Fr::r2();
             Fr r3 = r2 * r2;
-            r = d0 * r2 + d1 * r3;
+            r = r2 * d0 + r3 * d1;   // the reduced factor first (mont_mul_eo's bound)
         } else {
             Fr c = Fr::zero();
             if (cls == 1) { c.v[0] = (uint32_t)w[0]; c.v[1] = (uint32_t)(w[0] >> 32); }

@@ -61,6 +61,12 @@ static constexpr uint64_t ACC_MIN_K = 16;       // smallest chunk of the default
 static constexpr uint64_t MSM_PIPE_MIN = 1ull << 18;  // host scalars from here on are copied in pieces
 static constexpr int MSM_PIPE_PIECES = 8;
 
+#ifndef ACC_BLOCKS
+#define ACC_BLOCKS 4
+#endif
+#ifndef ACC_INLINE
+#define ACC_INLINE true
+#endif
 static int g_msm_window_override = 0;
 static int g_msm_acc_variant = 6;  // form and call structure of the accumulation kernel (0..6)
 static int g_msm_pair_rounds = 0;  // batch-affine pairing rounds before the XYZZ accumulation (0..3)
@@ -544,10 +550,32 @@ __global__ void __launch_bounds__(128, 3) k_msm_accumulate_z(const uint32_t* __r
     }
 }
 
-// The same accumulation in the FP64 lazy form (R' = 2^260, lazy64.cuh):
-// bases are read in the same x 2^261 storage form and halved modulo p on
-// load; buckets leave in the same canonical memory image.
-__global__ void __launch_bounds__(128, 3) k_msm_accumulate_d(const uint32_t* __restrict__ sorted,
+// x 2^261 mod p (canonical) -> x 2^256 mod p, canonical: v / 32 mod p as
+// (v + t p) / 32 with t = -v / p mod 32.
+__device__ __forceinline__ Fq from_r261(const Fq& v)
+{
+    const uint32_t t = (v.v[0] * FqCfg::N0) & 31u;
+    const uint32_t p[8] = {FqCfg::M0, FqCfg::M1, FqCfg::M2, FqCfg::M3, FqCfg::M4, FqCfg::M5, FqCfg::M6, FqCfg::M7};
+    uint32_t w[8];
+    uint64_t c = 0;
+#pragma unroll
+    for (int i = 0; i < 8; i++) {
+        c += (uint64_t)t * p[i] + v.v[i];
+        w[i] = (uint32_t)c;
+        c >>= 32;
+    }
+    Fq r;
+#pragma unroll
+    for (int i = 0; i < 7; i++) r.v[i] = __funnelshift_r(w[i], w[i + 1], 5);
+    r.v[7] = w[7] >> 5;                  // v + 31 p < 2^5 p < 2^259: the carry c joins the top word
+    r.v[7] |= (uint32_t)c << 27;
+    return r;
+}
+
+// The same accumulation with coordinates in [0, 2p) on the even/odd product:
+// bases are read in the x 2^261 storage form and divided by 32 on load;
+// buckets leave in the canonical memory image.
+__global__ void __launch_bounds__(128, ACC_BLOCKS) k_msm_accumulate_e(const uint32_t* __restrict__ sorted,
                                                              const uint32_t* __restrict__ offsets, uint64_t NB,
                                                              uint32_t K, const G1Affine* __restrict__ bases,
                                                              uint64_t phi_off, G1Xyzz* __restrict__ buckets,
@@ -567,11 +595,11 @@ __global__ void __launch_bounds__(128, 3) k_msm_accumulate_d(const uint32_t* __r
         uint64_t b = lo;
         uint32_t next = offsets[b + 1];
         bool head = offsets[b] < start;
-        G1XyzzD acc = xyzzd_inf();
+        G1Xyzz acc = xyzz_inf();
         for (uint32_t e = start; e < end; e++) {
             if (e == next) {
-                st_xyzzd(head ? &heads[t] : &buckets[b], acc);
-                acc = xyzzd_inf();
+                st_xyzze(head ? &heads[t] : &buckets[b], acc);
+                acc = xyzz_inf();
                 head = false;
                 do { b++; next = offsets[b + 1]; } while (next == e);
             }
@@ -585,84 +613,16 @@ __global__ void __launch_bounds__(128, 3) k_msm_accumulate_d(const uint32_t* __r
             const bool phi = (v & 1u) != 0;
             const G1Affine P = ld_affine(&bases[(v >> 1) + (phi ? phi_off : 0)]);    // phi(P) precomputed
             if (is_inf(P)) continue;
-            const FqD qx = fd_from_r261(P.x);                              // < p
-            FqD qy = fd_from_r261(P.y);                                    // < p
-            if (ent & SIGN_BIT) qy = fd_sub<FqCfg, 2>(fd_zero<FqCfg>(), qy);  // 2p - y < 2p
-            xyzzd_madd(acc, qx, qy);
+            const Fq qx = from_r261(P.x);
+            Fq qy = from_r261(P.y);
+            if (ent & SIGN_BIT) qy = qsub(Fq::zero(), qy);
+            xyzze_madd<ACC_INLINE>(acc, qx, qy);
         }
-        st_xyzzd(head ? &heads[t] : &buckets[b], acc);
+        st_xyzze(head ? &heads[t] : &buckets[b], acc);
     }
 }
 
 #if H2B_EXPERIMENTS
-// The FP64 lazy accumulation with two independent chains per thread: the
-// entries of a bucket segment alternate between two accumulators whose
-// additions share their out-of-line product calls (xyzzd_madd_x2), and the
-// two are added once when the segment's bucket (or chunk head) is stored.
-// Same chunks, bucket boundaries and outputs as k_msm_accumulate_d.  Measured
-// at 2^22 with the witness mix: 25.7 ms against 11.4 ms (255 registers and
-// spills halve the warps per SM; the second chain does not make up for it).
-__global__ void __launch_bounds__(128, 2) k_msm_accumulate_d2(const uint32_t* __restrict__ sorted,
-                                                              const uint32_t* __restrict__ offsets, uint64_t NB,
-                                                              uint32_t K, const G1Affine* __restrict__ bases,
-                                                              uint64_t phi_off, G1Xyzz* __restrict__ buckets,
-                                                              G1Xyzz* __restrict__ heads)
-{
-    const uint32_t M = offsets[NB];
-    const uint64_t nchunks = (M + (uint64_t)K - 1) / K;
-    auto load = [&](uint32_t e, FqD& qx, FqD& qy) -> bool {    // false for a point at infinity
-        const uint32_t ent = sorted[e];
-        const uint32_t v = ent & ~SIGN_BIT;
-        const G1Affine P = ld_affine(&bases[(v >> 1) + ((v & 1u) ? phi_off : 0)]);
-        if (is_inf(P)) return false;
-        qx = fd_from_r261(P.x);                                        // < p
-        qy = fd_from_r261(P.y);                                        // < p
-        if (ent & SIGN_BIT) qy = fd_sub<FqCfg, 2>(fd_zero<FqCfg>(), qy);  // 2p - y < 2p
-        return true;
-    };
-    for (uint64_t t = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; t < nchunks;
-         t += (uint64_t)gridDim.x * blockDim.x) {
-        const uint32_t start = (uint32_t)(t * K);
-        const uint32_t end = ((uint64_t)start + K < (uint64_t)M) ? start + K : M;
-        uint64_t lo = 0, hi = NB;  // offsets[lo] <= start < offsets[hi]
-        while (hi - lo > 1) {
-            uint64_t mid = (lo + hi) >> 1;
-            if (offsets[mid] <= start) lo = mid; else hi = mid;
-        }
-        uint64_t b = lo;
-        uint32_t next = offsets[b + 1];
-        bool head = offsets[b] < start;
-        G1XyzzD a0 = xyzzd_inf(), a1 = xyzzd_inf();
-        uint32_t e = start;
-        while (e < end) {
-            if (e == next) {
-                st_xyzzd_pair(head ? &heads[t] : &buckets[b], a0, a1);
-                a0 = xyzzd_inf();
-                a1 = xyzzd_inf();
-                head = false;
-                do { b++; next = offsets[b + 1]; } while (next == e);
-            }
-            const uint32_t seg = next < end ? next : end;
-            for (; e + 1 < seg; e += 2) {
-                FqD x0, y0, x1, y1;
-                const bool f0 = load(e, x0, y0), f1 = load(e + 1, x1, y1);
-                if (f0 && f1) {
-                    xyzzd_madd_x2(a0, x0, y0, a1, x1, y1);
-                } else {
-                    if (f0) xyzzd_madd(a0, x0, y0);
-                    if (f1) xyzzd_madd(a1, x1, y1);
-                }
-            }
-            if (e < seg) {
-                FqD x0, y0;
-                if (load(e, x0, y0)) xyzzd_madd(a0, x0, y0);
-                e++;
-            }
-        }
-        st_xyzzd_pair(head ? &heads[t] : &buckets[b], a0, a1);
-    }
-}
-
 // ---- pairing rounds (batch-affine bucket additions) -----------------------
 // Round r adds the points of every bucket pairwise in affine coordinates:
 // entries (2j, 2j+1) of a bucket become output point j (an odd last entry is
@@ -864,9 +824,9 @@ __global__ void k_msm_fixup(const uint32_t* __restrict__ offsets, uint64_t NB, u
             if (idx < max_dense) dense[idx] = (uint32_t)gb;
             continue;
         }
-        G1XyzzL acc = xyzzl_from(ld_xyzz(&buckets[gb]));
-        for (uint32_t t = t0 + 1; t <= t1; t++) xyzzl_add(acc, xyzzl_from(ld_xyzz(&heads[t])));
-        st_xyzz(&buckets[gb], xyzzl_to(acc));
+        G1Xyzz acc = ld_xyzz(&buckets[gb]);
+        for (uint32_t t = t0 + 1; t <= t1; t++) xyzze_add<false>(acc, ld_xyzz(&heads[t]));
+        st_xyzze(&buckets[gb], acc);
     }
 }
 
@@ -876,20 +836,20 @@ __global__ void k_msm_fixup(const uint32_t* __restrict__ offsets, uint64_t NB, u
 template <class Get>
 __device__ G1Xyzz block_sum_xyzz(uint64_t n, Get get)
 {
-    __shared__ G1XyzzL red[256];
-    G1XyzzL acc = xyzzl_inf();
-    for (uint64_t i = threadIdx.x; i < n; i += blockDim.x) xyzzl_add(acc, xyzzl_from(get(i)));
+    __shared__ G1Xyzz red[256];
+    G1Xyzz acc = xyzz_inf();
+    for (uint64_t i = threadIdx.x; i < n; i += blockDim.x) xyzze_add<false>(acc, get(i));
     red[threadIdx.x] = acc;
     __syncthreads();
     for (int h = blockDim.x >> 1; h > 0; h >>= 1) {
         if ((int)threadIdx.x < h) {
-            G1XyzzL a = red[threadIdx.x];
-            xyzzl_add(a, red[threadIdx.x + h]);
+            G1Xyzz a = red[threadIdx.x];
+            xyzze_add<false>(a, red[threadIdx.x + h]);
             red[threadIdx.x] = a;
         }
         __syncthreads();
     }
-    G1Xyzz r = xyzzl_to(red[0]);
+    G1Xyzz r = red[0];
     __syncthreads();
     return r;
 }
@@ -910,7 +870,7 @@ __global__ void __launch_bounds__(256) k_msm_dense_pieces(const uint32_t* __rest
         uint64_t len = t1 - t0;  // heads t0+1 .. t1
         uint64_t b0 = len * p / DENSE_PIECES, b1 = len * (p + 1) / DENSE_PIECES;
         G1Xyzz r = block_sum_xyzz(b1 - b0, [&](uint64_t j) { return ld_xyzz(&heads[t0 + 1 + b0 + j]); });
-        if (threadIdx.x == 0) st_xyzz(&pieces[it], r);
+        if (threadIdx.x == 0) st_xyzze(&pieces[it], r);
         __syncthreads();
     }
 }
@@ -927,7 +887,7 @@ __global__ void __launch_bounds__(DENSE_PIECES) k_msm_dense_merge(const uint64_t
         for (int h = DENSE_PIECES / 2; h > 0; h >>= 1) {
             if ((int)threadIdx.x < h) {
                 G1Xyzz a = red[threadIdx.x];
-                xyzz_add(a, red[threadIdx.x + h]);
+                xyzze_add<false>(a, red[threadIdx.x + h]);
                 red[threadIdx.x] = a;
             }
             __syncthreads();
@@ -935,8 +895,8 @@ __global__ void __launch_bounds__(DENSE_PIECES) k_msm_dense_merge(const uint64_t
         if (threadIdx.x == 0) {
             uint32_t gb = dense[i];
             G1Xyzz acc = ld_xyzz(&buckets[gb]);
-            xyzz_add(acc, red[0]);
-            st_xyzz(&buckets[gb], acc);
+            xyzze_add<false>(acc, red[0]);
+            st_xyzze(&buckets[gb], acc);
         }
         __syncthreads();
     }
@@ -957,13 +917,13 @@ __global__ void __launch_bounds__(128) k_msm_segments(const G1Xyzz* __restrict__
          id += (uint64_t)gridDim.x * blockDim.x) {
         uint64_t w = id / S, s = id % S;
         const G1Xyzz* B = buckets + w * H + s * L;
-        G1XyzzL run = xyzzl_inf(), acc = xyzzl_inf();
+        G1Xyzz run = xyzz_inf(), acc = xyzz_inf();
         for (int j = (int)L - 1; j >= 0; j--) {
-            xyzzl_add(run, xyzzl_from(ld_xyzz(&B[j])));
-            xyzzl_add(acc, run);
+            xyzze_add<false>(run, ld_xyzz(&B[j]));
+            xyzze_add<false>(acc, run);
         }
-        st_xyzz(&segacc[id], xyzzl_to(acc));
-        st_xyzz(&segrun[id], xyzzl_to(run));
+        st_xyzze(&segacc[id], acc);
+        st_xyzze(&segrun[id], run);
     }
 }
 
@@ -990,7 +950,7 @@ __global__ void __launch_bounds__(256) k_msm_bitsums(const G1Xyzz* __restrict__ 
         uint64_t s = ((j & ~lo_mask) << 1) | (1ull << k) | (j & lo_mask);
         return ld_xyzz(&segrun[(uint64_t)w * S + s]);
     });
-    if (threadIdx.x == 0) st_xyzz(&out[blockIdx.x], r);
+    if (threadIdx.x == 0) st_xyzze(&out[blockIdx.x], r);
 }
 
 // CTA (w, k): the BP partials of bit sum (w, k).
@@ -998,7 +958,7 @@ __global__ void __launch_bounds__(256) k_msm_bitparts(const G1Xyzz* __restrict__
                                                       G1Xyzz* __restrict__ bits)
 {
     G1Xyzz r = block_sum_xyzz(BP, [&](uint64_t j) { return ld_xyzz(&parts[(uint64_t)blockIdx.x * BP + j]); });
-    if (threadIdx.x == 0) st_xyzz(&bits[blockIdx.x], r);
+    if (threadIdx.x == 0) st_xyzze(&bits[blockIdx.x], r);
 }
 
 // One warp per window (warps loop when there are more windows than warps in
@@ -1009,14 +969,14 @@ __global__ void k_msm_wincombine(const G1Xyzz* __restrict__ bits, int W, int nbi
     const int warps = (int)(gridDim.x * (blockDim.x >> 5));
     for (int w = (int)(blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5)); w < W; w += warps) {
         const G1Xyzz* T = bits + (uint64_t)w * (nbits + 1);
-        G1XyzzL r = xyzzl_inf();
+        G1Xyzz r = xyzz_inf();
         for (int k = nbits - 1; k >= 0; k--) {
             r = xyzzw_dbl(r);
-            xyzzw_add(r, xyzzl_from(ld_xyzz(&T[k])));
+            xyzzw_add(r, ld_xyzz(&T[k]));
         }
         for (int d = 0; d < log_l; d++) r = xyzzw_dbl(r);
-        xyzzw_add(r, xyzzl_from(ld_xyzz(&T[nbits])));
-        if ((threadIdx.x & 31) == 0) st_xyzz(&wins[w], xyzzl_to(r));
+        xyzzw_add(r, ld_xyzz(&T[nbits]));
+        if ((threadIdx.x & 31) == 0) st_xyzze(&wins[w], r);
     }
 }
 
@@ -1027,16 +987,16 @@ __global__ void k_msm_final(const G1Xyzz* __restrict__ wins, int W, int c, G1Jac
 {
     __shared__ G1Xyzz sh[FINAL_MAX_W];
     for (int w = (int)(threadIdx.x >> 5); w < W; w += (int)(blockDim.x >> 5)) {
-        G1XyzzL x = xyzzl_from(ld_xyzz(&wins[w]));
+        G1Xyzz x = ld_xyzz(&wins[w]);
         for (int d = 0; d < c * w; d++) x = xyzzw_dbl(x);
-        if ((threadIdx.x & 31) == 0) sh[w] = xyzzl_to(x);
+        if ((threadIdx.x & 31) == 0) sh[w] = x;
     }
     __syncthreads();
     if (threadIdx.x < 32) {
-        G1XyzzL acc = xyzzl_inf();
-        for (int i = 0; i < W; i++) xyzzw_add(acc, xyzzl_from(sh[i]));
+        G1Xyzz acc = xyzz_inf();
+        for (int i = 0; i < W; i++) xyzzw_add(acc, sh[i]);
         if (threadIdx.x == 0) {
-            G1Jac j = xyzz_to_jac_affine(xyzzl_to(acc));
+            G1Jac j = xyzz_to_jac_affine(xyzze_canonical(acc));
             st(&out->X, j.X);
             st(&out->Y, j.Y);
             st(&out->Z, j.Z);
@@ -1161,14 +1121,9 @@ static RustError msm_finish(const MsmPlan& p, const MsmScratch& s, const G1Affin
     const uint64_t chunks = (p.cap[p.R] + p.Kf - 1) / p.Kf;
     const unsigned acc_grid = grid_for(chunks, 128, 148u * 32u);
     if (lazy && g_msm_acc_variant == 6)
-        k_msm_accumulate_d<<<acc_grid, 128, 0, st>>>(s.sorted, off, p.NB, p.Kf, p.tn ? d_bases : s.rbases,
+        k_msm_accumulate_e<<<acc_grid, 128, 0, st>>>(s.sorted, off, p.NB, p.Kf, p.tn ? d_bases : s.rbases,
                                                      p.tn ? (uint64_t)p.W * p.tn : p.n, s.buckets, s.heads,
                                                      g_msm_prefetch);
-#if H2B_EXPERIMENTS
-    else if (lazy && g_msm_acc_variant == 7)
-        k_msm_accumulate_d2<<<acc_grid, 128, 0, st>>>(s.sorted, off, p.NB, p.Kf, p.tn ? d_bases : s.rbases,
-                                                      p.tn ? (uint64_t)p.W * p.tn : p.n, s.buckets, s.heads);
-#endif
     else if (lazy)
         k_msm_accumulate_z<<<acc_grid, 128, 0, st>>>(s.sorted, off, p.NB, p.Kf, p.tn ? d_bases : s.rbases,
                                                      p.tn ? (uint64_t)p.W * p.tn : p.n, s.buckets, s.heads);
@@ -1255,7 +1210,7 @@ RustError msm_run_merged(const MsmPlan& p, const MsmScratch& s, uint32_t J, cons
     const uint64_t chunks = (p.max_entries + p.Kf - 1) / p.Kf;
     const unsigned acc_grid = grid_for(chunks, 128, 148u * 32u);
     if (g_msm_acc_variant == 6)
-        k_msm_accumulate_d<<<acc_grid, 128, 0, st>>>(s.sorted, s.offsets, p.NB, p.Kf, table, (uint64_t)p.W * p.tn,
+        k_msm_accumulate_e<<<acc_grid, 128, 0, st>>>(s.sorted, s.offsets, p.NB, p.Kf, table, (uint64_t)p.W * p.tn,
                                                      s.buckets, s.heads, g_msm_prefetch);
     else
         k_msm_accumulate_z<<<acc_grid, 128, 0, st>>>(s.sorted, s.offsets, p.NB, p.Kf, table, (uint64_t)p.W * p.tn,

@@ -306,12 +306,10 @@ constexpr int NTT_THREADS = 512;
 // of S * 2^nst).  A CTA owns G = 2^lG consecutive groups.  Every size is a
 // power of two, so all index arithmetic is shifts and masks on 32 bits
 // (n <= 2^31).
-// Blocks per SM for the pass: the FP64 product needs more live registers.
-#if H2B_MUL_F64
-constexpr int NTT_MIN_BLOCKS = 2;
-#else
-constexpr int NTT_MIN_BLOCKS = 3;
+#ifndef NTT4_BLOCKS
+#define NTT4_BLOCKS 2
 #endif
+constexpr int NTT_MIN_BLOCKS = 2;  // blocks per SM of the radix-2 pass
 
 template <bool DIT>
 __global__ void __launch_bounds__(NTT_THREADS, NTT_MIN_BLOCKS) k_ntt_pass(NttBatch B, const Fr* __restrict__ tw, int logn, int s0,
@@ -439,17 +437,13 @@ struct NttTile4 {
 // canonicalisation per element at the store (field.cuh, residues in [0, 2p)).
 __device__ __forceinline__ Fr lz_mul(const Fr& a, const Fr& b)
 {
-#if H2B_MUL_F64
-    return mont_mul_f64_lazy<FrCfg>(a, b);
-#else
-    return a * b;
-#endif
+    return mont_mul_eo_lazy<FrCfg>(a, b);
 }
 __device__ __forceinline__ Fr lz_add(const Fr& a, const Fr& b) { return add2p<FrCfg>(a, b); }
 __device__ __forceinline__ Fr lz_sub(const Fr& a, const Fr& b) { return sub2p<FrCfg>(a, b); }
 
 template <bool DIT>
-__global__ void __launch_bounds__(NTT4_THREADS, 2) k_ntt_pass4(NttBatch B, const Fr* __restrict__ tw, int logn,
+__global__ void __launch_bounds__(NTT4_THREADS, NTT4_BLOCKS) k_ntt_pass4(NttBatch B, const Fr* __restrict__ tw, int logn,
                                                                int s0, int nst, int lS, int lG)
 {
     const Fr* src = B.src[blockIdx.y];
