@@ -428,86 +428,159 @@ H2B_DEV void xyzze_add(G1Xyzz& acc, const G1Xyzz& q)
     acc.Y = qsub(qmul<INL>(R, qsub(Q, acc.X)), qmul<INL>(S1, PPP));
 }
 
-// ---- lane-parallel XYZZ formulas for one warp ------------------------------
-// A serial tail (the window doubling chain, the Horner combination of bit
-// sums, the sum of window results) runs one point formula after another, and
-// one thread needs about 1200 cycles per dependent product.  Here the whole
-// warp holds the same operands and its lanes compute the independent products
-// of one formula level at once (lane i mod 8 takes product i of the level),
-// then every lane reads the results back by shuffle.  A doubling becomes 3
-// product latencies instead of 9, an addition 4 instead of 14.  All 32 lanes
-// must call these with identical arguments; every lane ends with the result.
+// ---- one warp per point: formulas over shared-memory slots --------------------
+// A serial tail (doubling a window or bit sum many times, the sums of the
+// results) is one dependent product after another.  Here a warp keeps its
+// values in slots of shared memory; a level lets lane i take the i-th product
+// of a formula (operands and result by slot number, five bits per lane in a
+// literal), so a level costs one product's latency (860 cycles) and the
+// exchange two 32-byte reads and one write per lane.  All values are below 2p.
 
-H2B_DEV Fq lane_bcast(const Fq& v, int src)
+H2B_DEV Fq sl_get(const Fq* sl, int i) { return ld(&sl[i]); }
+
+// lane i < n: slot[(o >> 5 i) & 31] = slot[(a >> 5 i) & 31] * slot[(b >> 5 i) & 31]
+H2B_DEV void sl_mul(Fq* sl, int n, uint32_t a, uint32_t b, uint32_t o)
 {
+    const int lane = (int)(threadIdx.x & 31);
+    __syncwarp();
     Fq r;
+    if (lane < n) r = mont_mul_eo_lazy<FqCfg>(sl[(a >> (5 * lane)) & 31], sl[(b >> (5 * lane)) & 31]);
+    __syncwarp();
+    if (lane < n) st(&sl[(o >> (5 * lane)) & 31], r);
+    __syncwarp();
+}
+
+// (ca a + cb b + cc c) mod p, below 1.1p, for a, b, c <= 2p and ca + cb + cc <= 266:
+// the sum stays below 2^264, and the quotient estimate from its bits above
+// 2^248 is at most one short (2^280 / p rounded down is 88753990).
+H2B_DEV Fq qlin(uint32_t ca, const Fq& a, uint32_t cb, const Fq& b, uint32_t cc, const Fq& c)
+{
+    uint32_t w[9];
+    uint64_t x = 0;
 #pragma unroll
-    for (int i = 0; i < 8; i++) r.v[i] = __shfl_sync(0xffffffffu, v.v[i], src);
+    for (int i = 0; i < 8; i++) {
+        x += (uint64_t)ca * a.v[i] + (uint64_t)cb * b.v[i] + (uint64_t)cc * c.v[i];
+        w[i] = (uint32_t)x;
+        x >>= 32;
+    }
+    w[8] = (uint32_t)x;
+    const uint32_t q = __umulhi((w[7] >> 24) | (w[8] << 8), 88753990u);
+    Fq r;
+    int64_t y = 0;
+#pragma unroll
+    for (int i = 0; i < 8; i++) {
+        y += (int64_t)w[i] - (int64_t)((uint64_t)q * mword<FqCfg>(i) & 0xffffffffu);
+        r.v[i] = (uint32_t)y;
+        y >>= 32;
+        y -= (int64_t)((uint64_t)q * mword<FqCfg>(i) >> 32);
+    }
     return r;
 }
 
-// operand k of a level for lane slot s = lane mod 8 (slots past the last operand repeat it)
-H2B_DEV Fq lane_pick(int s, const Fq& a0, const Fq& a1, const Fq& a2, const Fq& a3, const Fq& a4, const Fq& a5)
+// 2p - a (a <= 2p): the complement that turns a subtraction into an addition for qlin
+H2B_DEV Fq qneg2(const Fq& a)
 {
     Fq r;
+    int64_t y = 0;
 #pragma unroll
-    for (int i = 0; i < 8; i++)
-        r.v[i] = s == 0 ? a0.v[i] : s == 1 ? a1.v[i] : s == 2 ? a2.v[i] : s == 3 ? a3.v[i] : s == 4 ? a4.v[i]
-                                                                                                    : a5.v[i];
+    for (int i = 0; i < 8; i++) {
+        y += (int64_t)m2word<FqCfg>(i) - (int64_t)a.v[i];
+        r.v[i] = (uint32_t)y;
+        y >>= 32;
+    }
     return r;
 }
 
-H2B_DEV int lane_slot() { return (int)(threadIdx.x & 7); }
-
-// dbl-2008-s-1 in three levels: {U^2, X^2}, {U V, X V, V ZZ, M^2}, {W ZZZ, M (S - X3), W Y}.
-H2B_DEV G1Xyzz xyzzw_dbl(const G1Xyzz& p)
+// 2^m times the XYZZ point in slots 0..3 (X, Y, ZZ, ZZZ; not infinity), in place.
+// The x coordinate alone goes through the doublings: with x = X / Z,
+//   X' = X^4 - 24 X Z^3,  Z' = 4 X^3 Z + 12 Z^4      (b = 3)
+// which is two levels deep instead of the three of dbl-2008-s-1.  With
+// C = X^3 Z and D = Z^4 the y coordinate is multiplied by
+//   (2 C^2 + 120 C D - 144 D^2) / Z'^2
+// at every doubling, whose numerators and denominators are collected by two
+// further lanes one and two steps behind.  No point of this curve has order
+// two (the group order is an odd prime), so Z never vanishes.
+// Slots used: 0..15.
+H2B_DEV void sl_dbl_many(Fq* sl, int m)
 {
-    if (is_inf(p)) return xyzz_inf();
-    const int s = lane_slot();
-    const Fq U = qadd(p.Y, p.Y);
-    Fq r = qsqr<false>((s & 1) ? p.X : U);
-    const Fq V = lane_bcast(r, 0), xx = lane_bcast(r, 1);
-    const Fq M = qadd(qadd(xx, xx), xx);
-    r = qmul<false>(lane_pick(s, U, p.X, V, M, M, M), lane_pick(s, V, V, p.ZZ, M, M, M));
-    const Fq W = lane_bcast(r, 0), S = lane_bcast(r, 1);
-    G1Xyzz o;
-    o.ZZ = lane_bcast(r, 2);
-    o.X = qsub(lane_bcast(r, 3), qadd(S, S));
-    const Fq sx = qsub(S, o.X);
-    r = qmul<false>(lane_pick(s, W, M, W, W, W, W), lane_pick(s, p.ZZZ, sx, p.Y, p.Y, p.Y, p.Y));
-    o.ZZZ = lane_bcast(r, 0);
-    o.Y = qsub(lane_bcast(r, 1), lane_bcast(r, 2));
-    return o;
+    if (m == 0) return;
+    const int lane = (int)(threadIdx.x & 31);
+    enum { X = 0, YN = 1, Z = 2, YD = 3, X2 = 4, Z2 = 5, XZ = 6, CC = 7, CD = 8, DD = 9, A = 10, B = 11, C = 12, D = 13,
+           M = 14, ONE = 15 };
+#define SL6(a, b, c, d, e, f) \
+    ((uint32_t)(a) | (uint32_t)(b) << 5 | (uint32_t)(c) << 10 | (uint32_t)(d) << 15 | (uint32_t)(e) << 20 | (uint32_t)(f) << 25)
+    if (lane == 0) st(&sl[M], Fq::one());
+    if (lane == 1) st(&sl[ONE], Fq::one());
+    if (lane == 2) st(&sl[C], Fq::one());
+    if (lane == 3) st(&sl[D], Fq::one());
+#pragma unroll 1
+    for (int i = 0; i <= m; i++) {
+        sl_mul(sl, 6, SL6(X, Z, X, C, C, D), SL6(X, Z, Z, C, D, D), SL6(X2, Z2, XZ, CC, CD, DD));
+        sl_mul(sl, 6, SL6(X2, XZ, XZ, Z2, YN, YD), SL6(X2, Z2, X2, Z2, M, i ? Z2 : ONE), SL6(A, B, C, D, YN, YD));
+        // lane 0: X' = A - 24 B; lane 1: Z' = 4 C + 12 D; lane 2: M = 2 CC + 120 CD - 144 DD of the step before
+        if (lane < 3) {
+            const Fq a = sl[lane == 0 ? A : lane == 1 ? C : CC];
+            Fq b = sl[lane == 0 ? B : lane == 1 ? D : CD];
+            const Fq c = qneg2(sl[DD]);
+            if (lane == 0) b = qneg2(b);
+            const Fq r = qlin(lane == 0 ? 1u : lane == 1 ? 4u : 2u, a, lane == 0 ? 24u : lane == 1 ? 12u : 120u, b,
+                              lane == 2 ? 144u : 0u, c);
+            if (lane == 2) { if (i) st(&sl[M], r); }
+            else if (i < m) st(&sl[lane == 0 ? X : Z], r);
+        }
+        __syncwarp();
+    }
+    // x = X / Z, y = YN M / YD: with t = Z YD, ZZ = t^2, ZZZ = t^3, X' = X YD t, Y' = (YN M) Z t^2
+    sl_mul(sl, 3, SL6(YN, Z, X, 0, 0, 0), SL6(M, YD, YD, 0, 0, 0), SL6(YN, A, B, 0, 0, 0));
+    sl_mul(sl, 3, SL6(A, B, YN, 0, 0, 0), SL6(A, A, Z, 0, 0, 0), SL6(C, X, D, 0, 0, 0));
+    sl_mul(sl, 2, SL6(C, D, 0, 0, 0, 0), SL6(A, C, 0, 0, 0, 0), SL6(YD, YN, 0, 0, 0, 0));
+    if (lane == 0) st(&sl[Z], sl_get(sl, C));
+    __syncwarp();
 }
 
-// add-2008-s in four levels: {U1, U2, S1, S2, ZZ1 ZZ2, ZZZ1 ZZZ2}, {P^2, R^2},
-// {P PP, U1 PP, zz PP}, {R (Q - X3), S1 PPP, zzz PPP}.
-H2B_DEV void xyzzw_add(G1Xyzz& acc, const G1Xyzz& q)
+// slots 0..3 += slots 4..7 (XYZZ points, add-2008-s in four product levels).  Slots used: 0..19.
+H2B_DEV void sl_add(Fq* sl)
 {
-    if (is_inf(q)) return;
-    if (is_inf(acc)) { acc = q; return; }
-    const int s = lane_slot();
-    Fq r = qmul<false>(lane_pick(s, acc.X, q.X, acc.Y, q.Y, acc.ZZ, acc.ZZZ),
-                       lane_pick(s, q.ZZ, acc.ZZ, q.ZZZ, acc.ZZZ, q.ZZ, q.ZZZ));
-    const Fq U1 = lane_bcast(r, 0), S1 = lane_bcast(r, 2);
-    const Fq zz = lane_bcast(r, 4), zzz = lane_bcast(r, 5);
-    const Fq P = qsub(lane_bcast(r, 1), U1), R = qsub(lane_bcast(r, 3), S1);
-    if (is_zero2p<FqCfg>(P)) {
-        if (is_zero2p<FqCfg>(R)) acc = xyzzw_dbl(acc);
-        else acc = xyzz_inf();
+    const int lane = (int)(threadIdx.x & 31);
+    __syncwarp();
+    if (sl_get(sl, 6).is_zero()) return;
+    if (sl_get(sl, 2).is_zero()) {
+        Fq t;
+        if (lane < 4) t = sl_get(sl, 4 + lane);
+        __syncwarp();
+        if (lane < 4) st(&sl[lane], t);
+        __syncwarp();
         return;
     }
-    r = qsqr<false>((s & 1) ? R : P);
-    const Fq PP = lane_bcast(r, 0), RR = lane_bcast(r, 1);
-    r = qmul<false>(lane_pick(s, P, U1, zz, zz, zz, zz), PP);
-    const Fq PPP = lane_bcast(r, 0), Q = lane_bcast(r, 1);
-    acc.ZZ = lane_bcast(r, 2);
-    const Fq X3 = qsub(qsub(RR, PPP), qadd(Q, Q));
-    r = qmul<false>(lane_pick(s, R, S1, zzz, zzz, zzz, zzz), lane_pick(s, qsub(Q, X3), PPP, PPP, PPP, PPP, PPP));
-    acc.Y = qsub(lane_bcast(r, 0), lane_bcast(r, 1));
-    acc.ZZZ = lane_bcast(r, 2);
-    acc.X = X3;
+    enum { X1 = 0, Y1 = 1, ZZ1 = 2, ZZZ1 = 3, XX2 = 4, YY2 = 5, ZZ2 = 6, ZZZ2 = 7, U1 = 8, U2 = 9, S1 = 10, S2 = 11,
+           P = 12, RR = 13, PP = 14, R2 = 15, PPP = 16, QQ = 17, T = 18, W = 19 };
+    sl_mul(sl, 6, SL6(X1, XX2, Y1, YY2, ZZ1, ZZZ1), SL6(ZZ2, ZZ1, ZZZ2, ZZZ1, ZZ2, ZZZ2), SL6(U1, U2, S1, S2, ZZ1, ZZZ1));
+    if (lane < 2) st(&sl[lane ? RR : P], qsub(sl[lane ? S2 : U2], sl[lane ? S1 : U1]));
+    __syncwarp();
+    if (is_zero2p<FqCfg>(sl_get(sl, P))) {     // equal x: a doubling or P + (-P); slots 4..7 still hold the second point
+        const bool dbl = is_zero2p<FqCfg>(sl_get(sl, RR));
+        __syncwarp();
+        if (lane == 0) {
+            G1Xyzz q;
+            q.X = sl[XX2]; q.Y = sl[YY2]; q.ZZ = sl[ZZ2]; q.ZZZ = sl[ZZZ2];
+            q = dbl ? xyzze_dbl<false>(q) : xyzz_inf();
+            st(&sl[X1], q.X); st(&sl[Y1], q.Y); st(&sl[ZZ1], q.ZZ); st(&sl[ZZZ1], q.ZZZ);
+        }
+        __syncwarp();
+        return;
+    }
+    sl_mul(sl, 2, SL6(P, RR, 0, 0, 0, 0), SL6(P, RR, 0, 0, 0, 0), SL6(PP, R2, 0, 0, 0, 0));
+    sl_mul(sl, 3, SL6(P, U1, ZZ1, 0, 0, 0), SL6(PP, PP, PP, 0, 0, 0), SL6(PPP, QQ, ZZ1, 0, 0, 0));
+    if (lane == 0) {
+        const Fq q = sl[QQ], x = qsub(qsub(sl[R2], sl[PPP]), qadd(q, q));
+        st(&sl[X1], x);
+        st(&sl[T], qsub(q, x));
+    }
+    sl_mul(sl, 3, SL6(RR, S1, ZZZ1, 0, 0, 0), SL6(T, PPP, PPP, 0, 0, 0), SL6(T, W, ZZZ1, 0, 0, 0));
+    if (lane == 0) st(&sl[Y1], qsub(sl[T], sl[W]));
+    __syncwarp();
 }
+#undef SL6
 
 H2B_DEV G1Affine affine_neg(const G1Affine& p)
 {

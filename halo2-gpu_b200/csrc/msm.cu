@@ -233,7 +233,7 @@ void msm_plan_scratch(const MsmPlan& p, ScratchPlan& sp, bool scalar_host, bool 
     sp.add_n<G1Xyzz>((uint64_t)p.Wr * p.S);           // segment plain sums
     sp.add_n<G1Xyzz>((uint64_t)std::max(p.W, p.Wr) * (p.NBITS + 1));  // per-bit sums
     if (p.BP > 1) sp.add_n<G1Xyzz>((uint64_t)p.Wr * (p.NBITS + 1) * p.BP);  // their parts
-    sp.add_n<G1Xyzz>(std::max(p.W, p.Wr));                            // window sums
+    sp.add_n<G1Xyzz>(std::max(p.W, p.Wr));                            // counters of the last reduction step
     sp.add_n<G1Jac>(1);                               // result
     if (p.R >= 1) sp.add_n<G1Affine>(p.cap[1]);       // round outputs 1, 3
     if (p.R >= 2) sp.add_n<G1Affine>(p.cap[2]);       // round output 2
@@ -269,7 +269,8 @@ MsmScratch msm_carve(const MsmPlan& p, ScratchArena& ar, bool scalar_host, bool 
     s.segrun = ar.take_n<G1Xyzz>((uint64_t)p.Wr * p.S);
     s.bits = ar.take_n<G1Xyzz>((uint64_t)std::max(p.W, p.Wr) * (p.NBITS + 1));
     s.bitparts = p.BP > 1 ? ar.take_n<G1Xyzz>((uint64_t)p.Wr * (p.NBITS + 1) * p.BP) : nullptr;
-    s.wins = ar.take_n<G1Xyzz>(std::max(p.W, p.Wr));
+    // a counter per bit sum: at most 20 (NBITS + 1) a window, 128 bytes set aside for each
+    s.tailctr = (uint32_t*)ar.take_n<G1Xyzz>(std::max(p.W, p.Wr));
     s.result = ar.take_n<G1Jac>(1);
     s.pts[0] = p.R >= 1 ? ar.take_n<G1Affine>(p.cap[1]) : nullptr;
     s.pts[1] = p.R >= 2 ? ar.take_n<G1Affine>(p.cap[2]) : nullptr;
@@ -910,8 +911,11 @@ __global__ void __launch_bounds__(DENSE_PIECES) k_msm_dense_merge(const uint64_t
 // 3. Thread w: W_w = T + L * sum_k 2^k T_k (Horner over the bits).
 __global__ void __launch_bounds__(128) k_msm_segments(const G1Xyzz* __restrict__ buckets, int W, uint32_t H,
                                                       uint32_t L, uint32_t S, G1Xyzz* __restrict__ segacc,
-                                                      G1Xyzz* __restrict__ segrun)
+                                                      G1Xyzz* __restrict__ segrun, uint32_t* __restrict__ ctr,
+                                                      uint32_t nctr)
 {
+    if (blockIdx.x == 0)
+        for (uint32_t i = threadIdx.x; i < nctr; i += blockDim.x) ctr[i] = 0;
     uint64_t total = (uint64_t)W * S;
     for (uint64_t id = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; id < total;
          id += (uint64_t)gridDim.x * blockDim.x) {
@@ -961,46 +965,72 @@ __global__ void __launch_bounds__(256) k_msm_bitparts(const G1Xyzz* __restrict__
     if (threadIdx.x == 0) st_xyzze(&bits[blockIdx.x], r);
 }
 
-// One warp per window (warps loop when there are more windows than warps in
-// the grid), the Horner steps on the lane-parallel formulas.
-__global__ void k_msm_wincombine(const G1Xyzz* __restrict__ bits, int W, int nbits, int log_l,
-                                 G1Xyzz* __restrict__ wins)
-{
-    const int warps = (int)(gridDim.x * (blockDim.x >> 5));
-    for (int w = (int)(blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5)); w < W; w += warps) {
-        const G1Xyzz* T = bits + (uint64_t)w * (nbits + 1);
-        G1Xyzz r = xyzz_inf();
-        for (int k = nbits - 1; k >= 0; k--) {
-            r = xyzzw_dbl(r);
-            xyzzw_add(r, ld_xyzz(&T[k]));
-        }
-        for (int d = 0; d < log_l; d++) r = xyzzw_dbl(r);
-        xyzzw_add(r, ld_xyzz(&T[nbits]));
-        if ((threadIdx.x & 31) == 0) st_xyzze(&wins[w], r);
-    }
-}
+// A merged run over a window table: window j of the reduction is job j's
+// whole sum (the table already holds the window multiples), so each job has
+// its own result; otherwise all windows of a run sum into one.
+struct MsmOuts {
+    G1Jac* p[MSM_MERGE_MAX];
+};
 
-// 2^(c*w) * W_w with one warp per window (lane-parallel doublings), then the
-// sum over windows and the affine conversion by the first warp.
-constexpr int FINAL_MAX_W = 64;
-__global__ void k_msm_final(const G1Xyzz* __restrict__ wins, int W, int c, G1Jac* __restrict__ out)
+// The reduction's last step: result = sum over windows w of
+// 2^(c w) (T_w + sum_k 2^(log_l + k) T_{w,k}).  One warp (one CTA) takes one
+// bit sum, doubles it by its whole weight on the x coordinate alone
+// (sl_dbl_many: the chain of a bit sum of the top window is as long as the
+// window doublings it replaces, but all of them run at once on their own SMs)
+// and the points are then added up pairwise: of two siblings the CTA that
+// arrives second adds the other's point and goes on, so no CTA waits for
+// another.  The last one of a group converts to the affine image.
+// Node i of a level stands at leaf i << level; a pair's counter is its right
+// child's leaf index.  Counters start at zero (k_msm_segments).
+// The chain is bound by product latency, two per doubling.  Measured at
+// c = 16, 8 windows: Horner over bit sums per window, then the window
+// doublings with one warp per window on one SM, 567 us; this kernel 290 us.
+__global__ void __launch_bounds__(32) k_msm_tail(G1Xyzz* bits, int nbits, int c, int log_l, uint32_t leaves,
+                                                 uint32_t* ctr, const __grid_constant__ MsmOuts outs)
 {
-    __shared__ G1Xyzz sh[FINAL_MAX_W];
-    for (int w = (int)(threadIdx.x >> 5); w < W; w += (int)(blockDim.x >> 5)) {
-        G1Xyzz x = ld_xyzz(&wins[w]);
-        for (int d = 0; d < c * w; d++) x = xyzzw_dbl(x);
-        if ((threadIdx.x & 31) == 0) sh[w] = x;
-    }
-    __syncthreads();
-    if (threadIdx.x < 32) {
-        G1Xyzz acc = xyzz_inf();
-        for (int i = 0; i < W; i++) xyzzw_add(acc, sh[i]);
-        if (threadIdx.x == 0) {
-            G1Jac j = xyzz_to_jac_affine(xyzze_canonical(acc));
-            st(&out->X, j.X);
-            st(&out->Y, j.Y);
-            st(&out->Z, j.Z);
+    __shared__ Fq sl[20];
+    const int lane = (int)threadIdx.x;
+    const uint32_t group = blockIdx.x / leaves;
+    uint32_t i = blockIdx.x % leaves;
+    G1Xyzz* pts = bits + (uint64_t)group * leaves;
+    uint32_t* gctr = ctr + (uint64_t)group * leaves;
+    const int w = (int)(i / (uint32_t)(nbits + 1)), k = (int)(i % (uint32_t)(nbits + 1));
+    // the four coordinates of a point are consecutive: lane j < 4 moves coordinate j
+    if (lane < 4) st(&sl[lane], ld(&pts[i].X + lane));
+    __syncwarp();
+    if (!sl_get(sl, 2).is_zero()) sl_dbl_many(sl, c * w + (k < nbits ? log_l + k : 0));
+    uint32_t cnt = leaves;
+    for (int level = 0; cnt > 1; level++) {
+        const uint32_t sib = i ^ 1u;
+        if (sib < cnt) {
+            if (lane < 4) st(&pts[i << level].X + lane, sl_get(sl, lane));
+            __threadfence();
+            __syncwarp();
+            uint32_t old = 0;
+            if (lane == 0) old = atomicAdd(&gctr[(i | 1u) << level], 1u);
+            old = __shfl_sync(0xffffffffu, old, 0);
+            if (old == 0) return;               // the sibling's CTA will take this point
+            __threadfence();
+            if (lane < 4) {
+                const uint4* q = reinterpret_cast<const uint4*>(&pts[sib << level].X + lane);
+                uint4* d = reinterpret_cast<uint4*>(&sl[4 + lane]);
+                d[0] = __ldcg(q);
+                d[1] = __ldcg(q + 1);
+            }
+            __syncwarp();
+            sl_add(sl);
         }
+        i >>= 1;
+        cnt = (cnt + 1) >> 1;
+    }
+    if (lane == 0) {
+        G1Xyzz r;
+        r.X = sl[0]; r.Y = sl[1]; r.ZZ = sl[2]; r.ZZZ = sl[3];
+        const G1Jac j = xyzz_to_jac_affine(xyzze_canonical(r));
+        G1Jac* out = outs.p[group];
+        st(&out->X, j.X);
+        st(&out->Y, j.Y);
+        st(&out->Z, j.Z);
     }
 }
 
@@ -1011,22 +1041,6 @@ __global__ void k_write_inf(G1Jac* out)
         st(&out->Y, Fq::one());
         st(&out->Z, Fq::zero());
     }
-}
-
-// A merged run over a window table: window j of the reduction is job j's
-// whole sum (the table already holds the window multiples), so each job's
-// result is its window sum in the reference's affine image, one lane per job.
-struct MsmOuts {
-    G1Jac* p[MSM_MERGE_MAX];
-};
-__global__ void k_msm_final_each(const G1Xyzz* __restrict__ wins, uint32_t J, const __grid_constant__ MsmOuts outs)
-{
-    const uint32_t j = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
-    if (j >= J || (threadIdx.x & 31) != 0) return;
-    const G1Jac r = xyzz_to_jac_affine(ld_xyzz(&wins[j]));
-    st(&outs.p[j]->X, r.X);
-    st(&outs.p[j]->Y, r.Y);
-    st(&outs.p[j]->Z, r.Z);
 }
 
 // Per-bit sums of the segment sums (reduction step 2), in BP parts per sum
@@ -1151,14 +1165,16 @@ static RustError msm_finish(const MsmPlan& p, const MsmScratch& s, const G1Affin
     k_msm_dense_merge<<<148, DENSE_PIECES, 0, st>>>(p.max_dense, s.buckets, s.dense, s.pieces);
     H2B_LAUNCHED("k_msm_dense_merge");
     uint64_t nseg = (uint64_t)p.Wr * p.S;
-    k_msm_segments<<<grid_for(nseg, 128, sm_cap), 128, 0, st>>>(s.buckets, p.Wr, p.H, p.L, p.S, s.segacc, s.segrun);
+    k_msm_segments<<<grid_for(nseg, 128, sm_cap), 128, 0, st>>>(s.buckets, p.Wr, p.H, p.L, p.S, s.segacc, s.segrun,
+                                                                s.tailctr, (uint32_t)p.Wr * (uint32_t)(p.NBITS + 1));
     H2B_LAUNCHED("k_msm_segments");
     H2B_TRY(msm_bitsums(p, s, st));
-    k_msm_wincombine<<<(p.Wr + 7) / 8, 32 * std::min(p.Wr, 8), 0, st>>>(s.bits, p.Wr, p.NBITS, p.LOGL, s.wins);
-    H2B_LAUNCHED("k_msm_wincombine");
-    k_msm_final<<<1, 32 * std::min(p.Wr, 8), 0, st>>>(s.wins, p.Wr, p.c, s.result);
+    MsmOuts o;
+    o.p[0] = s.result;
+    const uint32_t leaves = (uint32_t)p.Wr * (uint32_t)(p.NBITS + 1);
+    k_msm_tail<<<leaves, 32, 0, st>>>(s.bits, p.NBITS, p.c, p.LOGL, leaves, s.tailctr, o);
     prof_end(PROF_MSM_TOTAL, st);
-    H2B_LAUNCHED("k_msm_final");
+    H2B_LAUNCHED("k_msm_tail");
     return ok();
 }
 
@@ -1225,16 +1241,16 @@ RustError msm_run_merged(const MsmPlan& p, const MsmScratch& s, uint32_t J, cons
     k_msm_dense_merge<<<148, DENSE_PIECES, 0, st>>>(p.max_dense, s.buckets, s.dense, s.pieces);
     H2B_LAUNCHED("k_msm_dense_merge");
     const uint64_t nseg = (uint64_t)p.Wr * p.S;
-    k_msm_segments<<<grid_for(nseg, 128, sm_cap), 128, 0, st>>>(s.buckets, p.Wr, p.H, p.L, p.S, s.segacc, s.segrun);
+    k_msm_segments<<<grid_for(nseg, 128, sm_cap), 128, 0, st>>>(s.buckets, p.Wr, p.H, p.L, p.S, s.segacc, s.segrun,
+                                                                s.tailctr, (uint32_t)p.Wr * (uint32_t)(p.NBITS + 1));
     H2B_LAUNCHED("k_msm_segments");
     H2B_TRY(msm_bitsums(p, s, st));
-    k_msm_wincombine<<<(p.Wr + 7) / 8, 32 * std::min(p.Wr, 8), 0, st>>>(s.bits, p.Wr, p.NBITS, p.LOGL, s.wins);
-    H2B_LAUNCHED("k_msm_wincombine");
     MsmOuts o;
     for (uint32_t j = 0; j < J; j++) o.p[j] = outs[j];
-    k_msm_final_each<<<(J + 7) / 8, 256, 0, st>>>(s.wins, J, o);
+    const uint32_t leaves = (uint32_t)(p.NBITS + 1);
+    k_msm_tail<<<J * leaves, 32, 0, st>>>(s.bits, p.NBITS, 0, p.LOGL, leaves, s.tailctr, o);
     prof_end(PROF_MSM_TOTAL, st);
-    H2B_LAUNCHED("k_msm_final_each");
+    H2B_LAUNCHED("k_msm_tail");
     return ok();
 }
 

@@ -47,7 +47,7 @@ struct MsmScratch {
     G1Xyzz* segrun;
     G1Xyzz* bits;
     G1Xyzz* bitparts;    // per-part bit sums (BP > 1)
-    G1Xyzz* wins;
+    uint32_t* tailctr;   // arrival counters of the last reduction step
     G1Jac* result;
     G1Affine* rbases;    // plain bases P_i, then phi(P_i), in the lazy x 2^261 form (no pairing rounds)
     G1Affine* pts[2];    // pairing-round outputs (ping-pong)
