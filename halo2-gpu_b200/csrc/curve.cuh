@@ -155,93 +155,6 @@ H2B_DEV void xyzz_add(G1Xyzz& acc, const G1Xyzz& q)
     acc.ZZZ = acc.ZZZ * q.ZZZ * PPP;
 }
 
-// ---- XYZZ in 29-bit limb form (MSM bucket accumulation) -------------------
-// Same madd-2008-s formula over Fl<FqCfg>: coordinates stay below 2p in limb
-// form between products, so a bucket addition converts only the loaded point
-// (and the accumulator when it is stored).
-
-typedef Fl<FqCfg> FqL;
-
-struct G1XyzzL {
-    FqL X, Y, ZZ, ZZZ;
-};
-
-H2B_DEV G1XyzzL xyzzl_inf()
-{
-    G1XyzzL r;
-    r.X = fl_zero<FqCfg>(); r.Y = fl_zero<FqCfg>(); r.ZZ = fl_zero<FqCfg>(); r.ZZZ = fl_zero<FqCfg>();
-    return r;
-}
-
-H2B_DEV bool is_inf(const G1XyzzL& p) { return fl_is_zero(p.ZZ); }
-
-H2B_DEV G1XyzzL xyzzl_from(const G1Xyzz& p)
-{
-    G1XyzzL r;
-    r.X = to_l(p.X); r.Y = to_l(p.Y); r.ZZ = to_l(p.ZZ); r.ZZZ = to_l(p.ZZZ);
-    return r;
-}
-
-// Canonical XYZZ (infinity keeps ZZ = 0).
-H2B_DEV G1Xyzz xyzzl_to(const G1XyzzL& p)
-{
-    G1Xyzz r;
-    r.X = from_l(p.X); r.Y = from_l(p.Y); r.ZZ = from_l(p.ZZ); r.ZZZ = from_l(p.ZZZ);
-    return r;
-}
-
-// Product helpers by call structure: MODE 0 pairs two independent products
-// per out-of-line call, MODE 1 inlines every product, MODE 2 makes one
-// out-of-line call per product.
-template <int MODE>
-H2B_DEV Fl2<FqCfg> xl_mul2(const FqL& a0, const FqL& b0, const FqL& a1, const FqL& b1)
-{
-    if (MODE == 0) return fl_mul2(a0, b0, a1, b1);
-    Fl2<FqCfg> r;
-    if (MODE == 1) { r.a = mul29(a0, b0); r.b = mul29(a1, b1); }
-    else { r.a = fl_mul(a0, b0); r.b = fl_mul(a1, b1); }
-    return r;
-}
-
-template <int MODE>
-H2B_DEV Fl2<FqCfg> xl_sqr2(const FqL& a0, const FqL& a1)
-{
-    if (MODE == 0) return fl_sqr2(a0, a1);
-    Fl2<FqCfg> r;
-    if (MODE == 1) { r.a = sqr29(a0); r.b = sqr29(a1); }
-    else { r.a = fl_sqr(a0); r.b = fl_sqr(a1); }
-    return r;
-}
-
-// madd-2008-s: acc += (qx, qy), an affine point that is not infinity.
-template <int MODE = 0>
-H2B_DEV void xyzzl_madd(G1XyzzL& acc, const FqL& qx, const FqL& qy)
-{
-    if (is_inf(acc)) {
-        acc.X = qx; acc.Y = qy; acc.ZZ = to_l(Fq::one()); acc.ZZZ = acc.ZZ;
-        return;
-    }
-    // products grouped in independent pairs: 8M + 2S in five pairs
-    const Fl2<FqCfg> us = xl_mul2<MODE>(qx, acc.ZZ, qy, acc.ZZZ);     // U2, S2
-    const FqL P = fl_sub(us.a, acc.X);
-    const FqL R = fl_sub(us.b, acc.Y);
-    if (fl_is_zero_mod(P)) {
-        G1Affine q;
-        q.x = from_l(qx); q.y = from_l(qy);
-        acc = fl_is_zero_mod(R) ? xyzzl_from(xyzz_dbl_affine(q)) : xyzzl_inf();
-        return;
-    }
-    const Fl2<FqCfg> sq = xl_sqr2<MODE>(P, R);                        // PP, R^2
-    const Fl2<FqCfg> pq = xl_mul2<MODE>(P, sq.a, acc.X, sq.a);        // PPP, Q
-    const FqL X3 = fl_sub(fl_sub(sq.b, pq.a), fl_add(pq.b, pq.b));
-    const Fl2<FqCfg> yy = xl_mul2<MODE>(R, fl_sub(pq.b, X3), acc.Y, pq.a);
-    const Fl2<FqCfg> zz = xl_mul2<MODE>(acc.ZZ, sq.a, acc.ZZZ, pq.a); // ZZ*PP, ZZZ*PPP
-    acc.Y = fl_sub(yy.a, yy.b);
-    acc.X = X3;
-    acc.ZZ = zz.a;
-    acc.ZZZ = zz.b;
-}
-
 // ---- XYZZ in the lazy form (R = 2^261), for the bucket accumulation -------
 // Bounds (multiples of p) that every step relies on are written beside it;
 // products follow (1 + 0.0059 a b) p (lazy.cuh).  The accumulator keeps
@@ -455,25 +368,40 @@ H2B_DEV void sl_mul(Fq* sl, int n, uint32_t a, uint32_t b, uint32_t o)
 // 2^248 is at most one short (2^280 / p rounded down is 88753990).
 H2B_DEV Fq qlin(uint32_t ca, const Fq& a, uint32_t cb, const Fq& b, uint32_t cc, const Fq& c)
 {
-    uint32_t w[9];
-    uint64_t x = 0;
+    // limb products first (independent), then one carry chain each way
+    uint32_t lo[8], hi[8], w[9];
 #pragma unroll
     for (int i = 0; i < 8; i++) {
-        x += (uint64_t)ca * a.v[i] + (uint64_t)cb * b.v[i] + (uint64_t)cc * c.v[i];
-        w[i] = (uint32_t)x;
-        x >>= 32;
+        const uint64_t x = (uint64_t)ca * a.v[i] + (uint64_t)cb * b.v[i] + (uint64_t)cc * c.v[i];
+        lo[i] = (uint32_t)x;
+        hi[i] = (uint32_t)(x >> 32);
     }
-    w[8] = (uint32_t)x;
+    w[0] = lo[0];
+    asm("add.cc.u32 %0, %8, %16;\n\taddc.cc.u32 %1, %9, %17;\n\taddc.cc.u32 %2, %10, %18;\n\t"
+        "addc.cc.u32 %3, %11, %19;\n\taddc.cc.u32 %4, %12, %20;\n\taddc.cc.u32 %5, %13, %21;\n\t"
+        "addc.cc.u32 %6, %14, %22;\n\taddc.u32 %7, %15, 0;"
+        : "=&r"(w[1]), "=&r"(w[2]), "=&r"(w[3]), "=&r"(w[4]), "=&r"(w[5]), "=&r"(w[6]), "=&r"(w[7]), "=&r"(w[8])
+        : "r"(hi[0]), "r"(hi[1]), "r"(hi[2]), "r"(hi[3]), "r"(hi[4]), "r"(hi[5]), "r"(hi[6]), "r"(hi[7]), "r"(lo[1]),
+          "r"(lo[2]), "r"(lo[3]), "r"(lo[4]), "r"(lo[5]), "r"(lo[6]), "r"(lo[7]));
     const uint32_t q = __umulhi((w[7] >> 24) | (w[8] << 8), 88753990u);
-    Fq r;
-    int64_t y = 0;
 #pragma unroll
     for (int i = 0; i < 8; i++) {
-        y += (int64_t)w[i] - (int64_t)((uint64_t)q * mword<FqCfg>(i) & 0xffffffffu);
-        r.v[i] = (uint32_t)y;
-        y >>= 32;
-        y -= (int64_t)((uint64_t)q * mword<FqCfg>(i) >> 32);
+        const uint64_t x = (uint64_t)q * mword<FqCfg>(i);
+        lo[i] = (uint32_t)x;
+        hi[i] = (uint32_t)(x >> 32);
     }
+    asm("add.cc.u32 %0, %0, %7;\n\taddc.cc.u32 %1, %1, %8;\n\taddc.cc.u32 %2, %2, %9;\n\t"
+        "addc.cc.u32 %3, %3, %10;\n\taddc.cc.u32 %4, %4, %11;\n\taddc.cc.u32 %5, %5, %12;\n\taddc.u32 %6, %6, %13;"
+        : "+r"(lo[1]), "+r"(lo[2]), "+r"(lo[3]), "+r"(lo[4]), "+r"(lo[5]), "+r"(lo[6]), "+r"(lo[7])
+        : "r"(hi[0]), "r"(hi[1]), "r"(hi[2]), "r"(hi[3]), "r"(hi[4]), "r"(hi[5]), "r"(hi[6]));
+    Fq r;
+    asm("sub.cc.u32 %0, %8, %16;\n\tsubc.cc.u32 %1, %9, %17;\n\tsubc.cc.u32 %2, %10, %18;\n\t"
+        "subc.cc.u32 %3, %11, %19;\n\tsubc.cc.u32 %4, %12, %20;\n\tsubc.cc.u32 %5, %13, %21;\n\t"
+        "subc.cc.u32 %6, %14, %22;\n\tsubc.u32 %7, %15, %23;"
+        : "=&r"(r.v[0]), "=&r"(r.v[1]), "=&r"(r.v[2]), "=&r"(r.v[3]), "=&r"(r.v[4]), "=&r"(r.v[5]), "=&r"(r.v[6]),
+          "=&r"(r.v[7])
+        : "r"(w[0]), "r"(w[1]), "r"(w[2]), "r"(w[3]), "r"(w[4]), "r"(w[5]), "r"(w[6]), "r"(w[7]), "r"(lo[0]), "r"(lo[1]),
+          "r"(lo[2]), "r"(lo[3]), "r"(lo[4]), "r"(lo[5]), "r"(lo[6]), "r"(lo[7]));
     return r;
 }
 
@@ -481,13 +409,14 @@ H2B_DEV Fq qlin(uint32_t ca, const Fq& a, uint32_t cb, const Fq& b, uint32_t cc,
 H2B_DEV Fq qneg2(const Fq& a)
 {
     Fq r;
-    int64_t y = 0;
-#pragma unroll
-    for (int i = 0; i < 8; i++) {
-        y += (int64_t)m2word<FqCfg>(i) - (int64_t)a.v[i];
-        r.v[i] = (uint32_t)y;
-        y >>= 32;
-    }
+    asm("sub.cc.u32 %0, %16, %8;\n\tsubc.cc.u32 %1, %17, %9;\n\tsubc.cc.u32 %2, %18, %10;\n\t"
+        "subc.cc.u32 %3, %19, %11;\n\tsubc.cc.u32 %4, %20, %12;\n\tsubc.cc.u32 %5, %21, %13;\n\t"
+        "subc.cc.u32 %6, %22, %14;\n\tsubc.u32 %7, %23, %15;"
+        : "=&r"(r.v[0]), "=&r"(r.v[1]), "=&r"(r.v[2]), "=&r"(r.v[3]), "=&r"(r.v[4]), "=&r"(r.v[5]), "=&r"(r.v[6]),
+          "=&r"(r.v[7])
+        : "r"(a.v[0]), "r"(a.v[1]), "r"(a.v[2]), "r"(a.v[3]), "r"(a.v[4]), "r"(a.v[5]), "r"(a.v[6]), "r"(a.v[7]),
+          "n"(m2word<FqCfg>(0)), "n"(m2word<FqCfg>(1)), "n"(m2word<FqCfg>(2)), "n"(m2word<FqCfg>(3)),
+          "n"(m2word<FqCfg>(4)), "n"(m2word<FqCfg>(5)), "n"(m2word<FqCfg>(6)), "n"(m2word<FqCfg>(7)));
     return r;
 }
 

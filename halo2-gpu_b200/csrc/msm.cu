@@ -23,10 +23,10 @@
 //              writes finished buckets directly and the partial sum of the
 //              bucket it started in the middle of to a per-chunk slot.
 //  5. fixup:   each bucket adds the per-chunk partials it spans; buckets that
-//              span many chunks are summed by a CTA-wide tree instead.
-//  6. reduce:  per window, buckets are cut into segments; each segment does
-//              the running-sum trick and scales by its offset, a CTA tree
-//              sums the segments, then 2^(c*w) * W_w is summed over windows.
+//              span many chunks get warps of their own.
+//  6. reduce:  per window, the buckets are folded bit by bit of their index
+//              into c - 1 bit sums and a total; every one of them is doubled
+//              by its whole weight on its own SM, and they are added up.
 //  7. output:  XYZZ -> the reference's Jacobian image {x, y, 1} (or (0,1,0)).
 #include <algorithm>
 #include "abi.cuh"
@@ -40,48 +40,33 @@ extern "C" RustError h2b_exec_fork(cudaStream_t parent, uint32_t n, cudaStream_t
 
 namespace h2b {
 
-// H2B_EXPERIMENTS=1 also builds the accumulation forms and the batch-affine
-// pairing rounds that measured slower than the default (A/B comparisons);
-// the shipped library leaves them out.
-#ifndef H2B_EXPERIMENTS
-#define H2B_EXPERIMENTS 0
-#endif
 static constexpr int GLV_BITS = 127;
 // 32-bit sorted-entry offsets: 2 halves x 8 windows x n < 2^32
 static constexpr uint64_t MSM_MAX_LENGTH = 1ull << 27;
 static constexpr uint32_t SIGN_BIT = 0x80000000u;
 // widest window the tuning override accepts (22 bits: 6 windows per GLV half)
 static constexpr int MSM_MAX_WINDOW = 22;
-// segment sums per CTA of a bit sum before it is split (reduction step 2)
-static constexpr uint32_t BITSUM_ITEMS = 4096;
-static constexpr uint32_t DENSE_LIMIT = 32;     // chunks per bucket summed serially in fixup
-static constexpr int DENSE_PIECES = 32;          // CTAs per dense bucket
-static constexpr uint64_t ACC_TARGET_CHUNKS = 148ull * 3 * 128 * 4;  // accumulation threads x 4
-static constexpr uint64_t ACC_MIN_K = 16;       // smallest chunk of the default plan
+static constexpr uint32_t FOLD_THREADS = 320;     // most threads of a reduction CTA
+// accumulation threads resident at once: 148 SMs x 4 CTAs x 128
+static constexpr uint32_t ACC_RESIDENT = 148u * 4u * 128u;
+static constexpr uint32_t ACC_MIN_K = 4;          // smallest chunk
+// Largest chunk of an MSM that runs alone: larger ones leave fewer heads to the
+// fixup, smaller ones even out the ends of the accumulation (2^22 witness mix
+// 8.14 ms at 64, 8.07 at 96 and 128, 8.12 at 192).
+static constexpr uint32_t ACC_MAX_K = 96;
+static constexpr uint32_t ACC_MAX_K_SHARED = 128; // and of one of several that run at once
+static constexpr uint32_t HEADS_PIECE = 32;       // chunk heads per warp of a long bucket
+static constexpr uint32_t HEADS_PIECES_MAX = 1024;
 static constexpr uint64_t MSM_PIPE_MIN = 1ull << 18;  // host scalars from here on are copied in pieces
 static constexpr int MSM_PIPE_PIECES = 8;
 
-#ifndef ACC_BLOCKS
-#define ACC_BLOCKS 4
-#endif
-#ifndef ACC_INLINE
-#define ACC_INLINE true
-#endif
 static int g_msm_window_override = 0;
-static int g_msm_acc_variant = 6;  // form and call structure of the accumulation kernel (0..6)
-static int g_msm_pair_rounds = 0;  // batch-affine pairing rounds before the XYZZ accumulation (0..3)
-constexpr int PR_T = 128;          // pairing rounds: threads per CTA
-constexpr int PR_E = 8;            // pairing rounds: input entries per thread (at most 4 additions)
-static uint64_t pr_ctas(uint64_t entries) { return (entries + (uint64_t)PR_T * PR_E - 1) / ((uint64_t)PR_T * PR_E); }
+static int g_msm_acc_variant = 6;  // form of the accumulation kernel: 6 or 0
 
 uint64_t fq_batch_invert_scratch(uint64_t n);
 int tune_value(int param, int log_n);  // tune.cu
 RustError fq_batch_invert(Fq* d, uint64_t n, void* scratch, uint64_t scratch_bytes, cudaStream_t st);
 
-void msm_set_pair_rounds(int rounds)
-{
-    if (rounds >= 0 && rounds <= (H2B_EXPERIMENTS ? 3 : 0)) g_msm_pair_rounds = rounds;
-}
 static int g_msm_chunk_override = 0;
 static uint32_t g_msm_prefetch = 2;   // entries ahead whose point the accumulation prefetches into L2 (0: none)
 
@@ -107,15 +92,18 @@ static int choose_c(uint64_t n, bool plain = false)
     if (plain) {
         const int tuned = tune_value(0, lg);
         if (tuned) return tuned;
-        // plain-base widths from autotuner runs on B200 (witness-like scalar
-        // mix): 16 bits from 2^20 (5.40 -> 4.36 ms with the chunk rule below),
-        // 13 bits from 2^14 (2^16: 1.79 -> 1.45 ms); 17 to 20 bits measured
-        // slower from 2^20 to 2^22 (2^22: 11.30 ms at 16, 13.4-19.6 ms wider)
-        if (lg >= 20) return 16;
-        if (lg >= 19) return 15;
+        // Plain-base widths, measured on B200 (uniform / witness-mix scalars, us).
+        // What is left over for the top window matters as much as the width:
+        // 7, 9 and 14 bits leave one bit of the 127, whose one or two buckets
+        // hold half of all entries each.
+        //   1000 points:  8 bits 387 / 442, 10 bits 452 / 462
+        //   2^13: 8 bits 464 / 514, 13 bits 514 / 526
+        //   2^16: 13 bits 751 / 685, 12 bits 803 / 716, 16 bits 929 / 944
+        //   2^18: 13 bits 1522 / 1138, 16 bits 1527 / 1302
+        //   2^19: 16 bits 2267 / 1755, 13 bits 2553 / 1761
+        if (lg >= 19) return 16;
         if (lg >= 14) return 13;
-        if (lg >= 10) return 10;
-        return 7;
+        return 8;
     }
     // Window tables: every window's digits land in one bucket set of 2^(c-1)
     // buckets, so a narrow window makes few, long buckets (2^18 points at 13
@@ -132,8 +120,9 @@ static int choose_c(uint64_t n, bool plain = false)
 }
 
 // tn > 0: precomputed window table of tn points per window; all windows then
-// share one bucket set and the reduction has a single window.
-static MsmPlan plan_core(uint64_t n, int c, uint64_t tn, uint32_t concurrent = 1)
+// share one bucket set and the reduction has a single window (one per job of
+// a merged run).
+static MsmPlan plan_core(uint64_t n, int c, uint64_t tn, uint32_t concurrent = 1, uint32_t jobs = 1)
 {
     MsmPlan p;
     p.n = n;
@@ -144,54 +133,50 @@ static MsmPlan plan_core(uint64_t n, int c, uint64_t tn, uint32_t concurrent = 1
     p.W = (GLV_BITS + c - 1) / c;
     if (GLV_BITS - c * (p.W - 1) > c - 1) p.W++;
     p.H = 1u << (c - 1);
-    p.Wr = tn ? 1 : p.W;
+    p.Wr = tn ? (int)jobs : p.W;
     p.NB = (uint64_t)p.Wr * p.H;
     p.nv = 2 * n;
     p.max_entries = p.nv * (uint64_t)p.W;
-    // Entries per accumulation chunk (one thread walks a chunk): 128 when the
-    // entries give at least ACC_TARGET_CHUNKS chunks (k >= 20 at every
-    // window size), fewer for a small MSM so that about ACC_TARGET_CHUNKS
-    // threads still run (148 SMs x 3 CTAs x 128 threads, 4 chunks each).
-    // MSMs that run `concurrent` at a time share that target.  A smaller K
-    // adds chunk heads that the fixup sums serially per bucket, so K must
-    // not drop where buckets are long: on the 64-job batch (16 streams) a
-    // fixed K = 32 took 133 ms over a window table against 85 ms at 128.
-    const uint64_t k_fit = p.max_entries / std::max<uint64_t>(1, ACC_TARGET_CHUNKS / std::max(concurrent, 1u));
-    // A tuned chunk size applies to an MSM that runs alone (batched MSMs keep
-    // the formula, which accounts for the MSMs running beside them).
-    // A plain-base MSM that runs alone takes half the fitted chunk, at most
-    // 64 (B200 autotuner runs: 2^22 128 -> 64 entries 11.89 -> 11.45 ms;
-    // 2^20 at 16 bits chose 32 entries): twice the chunks hide more of the
-    // accumulation's latency than the extra chunk heads cost the fixup.  Not
-    // over a window table: its single bucket set holds W times longer
-    // buckets, which at 64 entries span more than DENSE_LIMIT chunks and take
-    // the dense path (k = 22 prover-shaped proof 398 -> 438 ms).
+    // Entries per accumulation chunk (one thread walks a chunk; chunk_entries
+    // below fixes it on the device from the entries that are really there): a
+    // tuned or overriding size as it is, else the fewest whole waves of
+    // resident threads whose chunks stay within the cap.  MSMs that run
+    // `concurrent` at a time share the resident threads and take larger
+    // chunks, whose fewer heads cost the fixup less.  A tuned size applies to
+    // a plain-base MSM that runs alone.
     const bool alone_plain = concurrent <= 1 && tn == 0;
     const int tuned_k = alone_plain ? tune_value(1, floor_log2(n)) : 0;
-    const uint64_t k_rule = alone_plain ? std::min<uint64_t>(64, std::max<uint64_t>(ACC_MIN_K, k_fit / 2))
-                                        : std::min<uint64_t>(128, std::max<uint64_t>(ACC_MIN_K, k_fit));
-    p.K = g_msm_chunk_override > 0 ? (uint32_t)g_msm_chunk_override
-          : tuned_k > 0            ? (uint32_t)tuned_k
-                                   : (uint32_t)k_rule;
-    // pairing rounds: round r leaves at most cap[r-1]/2 + NB/2 entries
-    p.R = tn ? 0 : g_msm_pair_rounds;
-    p.cap[0] = p.max_entries;
-    for (int r = 1; r <= 3; r++) p.cap[r] = p.cap[r - 1] / 2 + p.NB / 2 + 1;
-    p.Kf = p.R > 0 ? std::max<uint32_t>(8u, p.K >> p.R) : p.K;
-    const uint64_t final_entries = p.cap[p.R];
-    p.max_chunks = (final_entries + p.Kf - 1) / p.Kf + 1;
-    // segments per window for the running-sum reduction (L buckets each)
-    uint32_t L = p.H >= 256 ? 8u : (p.H >= 4 ? 4u : 1u);
-    p.L = L;
-    p.LOGL = 31 - __builtin_clz(L);
-    p.S = p.H / L;
-    p.NBITS = p.S > 1 ? 31 - __builtin_clz(p.S) : 0;
-    // a bit sum of more than BITSUM_ITEMS segment sums is split over CTAs
-    // (wide windows over a table: one bucket set of 2^(c-1) buckets, a
-    // single reduction window, so only NBITS + 1 bit sums to spread)
-    p.BP = std::max<uint32_t>(1u, (p.S + BITSUM_ITEMS - 1) / BITSUM_ITEMS);
-    // a bucket spanning more than DENSE_LIMIT chunks holds > DENSE_LIMIT*K entries
-    p.max_dense = final_entries / ((uint64_t)DENSE_LIMIT * p.Kf) + 1;
+    p.chunk.fixed = g_msm_chunk_override > 0 ? (uint32_t)g_msm_chunk_override : (uint32_t)std::max(tuned_k, 0);
+    p.chunk.threads = std::max<uint32_t>(ACC_RESIDENT / std::max(concurrent, 1u), 128u);
+    p.chunk.cap = concurrent <= 1 ? ACC_MAX_K : ACC_MAX_K_SHARED;
+    // more entries never make fewer chunks than one wave less: the bound over
+    // every entry count up to max_entries
+    p.max_chunks = p.chunk.fixed ? p.max_entries / p.chunk.fixed + 2
+                                 : std::min<uint64_t>(p.max_entries / ACC_MIN_K,
+                                                      (p.max_entries / ((uint64_t)p.chunk.threads * p.chunk.cap) + 1) *
+                                                          p.chunk.threads) + 2;
+    // Bits folded by each pass of the bucket reduction: nine at first (one CTA
+    // of 256 threads per 512 buckets), then as many as keep a pass's first
+    // step within one addition per thread (FOLD_THREADS).
+    p.passes = 0;
+    int arrays = 1, left = c - 1;
+    do {
+        int m = std::min(left, 9);
+        while (m > 1 && (uint32_t)arrays << (m - 1) > FOLD_THREADS) m--;
+        p.fold[p.passes++] = m;
+        arrays += m;
+        left -= m;
+    } while (left > 0);
+    p.leaves = (uint64_t)p.Wr * c;                     // c - 1 bit sums and the total per window
+    // Lanes per bucket that sum its chunk heads: enough to occupy the GPU when
+    // the buckets are few, no more than the heads an average bucket has.  A
+    // bucket with more than `limit` heads goes to warps of its own instead.
+    const uint64_t avg = p.max_chunks / p.NB + 1;
+    p.fix_lanes = 1;
+    while (p.fix_lanes < 32 && p.NB * p.fix_lanes < 32768 && p.fix_lanes < avg) p.fix_lanes *= 2;
+    p.fix_limit = p.fix_lanes * (uint32_t)std::min<uint64_t>(std::max<uint64_t>(2 * avg / p.fix_lanes + 2, 4), 16);
+    p.max_dense = p.max_chunks / p.fix_limit + 1;
+    p.max_items = p.max_chunks / HEADS_PIECE + p.max_dense + 1;
     return p;
 }
 
@@ -209,10 +194,21 @@ MsmPlan msm_plan_shared(uint64_t n, uint64_t tn, uint32_t concurrent)
 // the sort, the accumulation and the bucket reduction run once for all jobs.
 MsmPlan msm_plan_merged(uint64_t n_total, uint64_t tn, uint32_t J)
 {
-    MsmPlan p = plan_core(n_total, choose_c(tn), tn);
-    p.Wr = (int)J;
-    p.NB = (uint64_t)J * p.H;
+    MsmPlan p = plan_core(n_total, choose_c(tn), tn, 1, J);
     return p;
+}
+
+// Points that the even (k = 0) or odd passes of the bucket reduction write at
+// most: 1 + (bits folded so far) arrays of one element per block left.
+static uint64_t msm_fold_points(const MsmPlan& p, int k)
+{
+    uint64_t most = 0;
+    int done = 0;
+    for (int i = 0; i < p.passes; i++) {
+        done += p.fold[i];
+        if ((i & 1) == k) most = std::max<uint64_t>(most, (uint64_t)p.Wr * (1 + done) * (p.H >> done));
+    }
+    return most;
 }
 
 void msm_plan_scratch(const MsmPlan& p, ScratchPlan& sp, bool scalar_host, bool bases_host)
@@ -227,27 +223,12 @@ void msm_plan_scratch(const MsmPlan& p, ScratchPlan& sp, bool scalar_host, bool 
     sp.add_n<uint32_t>(p.max_entries);                // sorted entries
     sp.add_n<G1Xyzz>(p.NB);                           // bucket sums
     sp.add_n<G1Xyzz>(p.max_chunks);                   // chunk head partials
-    sp.add_n<uint32_t>(p.max_dense + 1);              // dense list + count
-    sp.add_n<G1Xyzz>(p.max_dense * DENSE_PIECES);     // dense pieces
-    sp.add_n<G1Xyzz>((uint64_t)p.Wr * p.S);           // segment weighted sums
-    sp.add_n<G1Xyzz>((uint64_t)p.Wr * p.S);           // segment plain sums
-    sp.add_n<G1Xyzz>((uint64_t)std::max(p.W, p.Wr) * (p.NBITS + 1));  // per-bit sums
-    if (p.BP > 1) sp.add_n<G1Xyzz>((uint64_t)p.Wr * (p.NBITS + 1) * p.BP);  // their parts
-    sp.add_n<G1Xyzz>(std::max(p.W, p.Wr));                            // counters of the last reduction step
+    sp.add_n<uint32_t>(p.max_dense + 2);              // long buckets, their count, their pieces' count
+    sp.add_n<uint2>(p.max_items);                     // their pieces
+    for (int k = 0; k < 2; k++) sp.add_n<G1Xyzz>(msm_fold_points(p, k));  // outputs of the reduction passes
+    sp.add_n<uint32_t>(p.leaves);                     // counters of the last reduction step
     sp.add_n<G1Jac>(1);                               // result
-    if (p.R >= 1) sp.add_n<G1Affine>(p.cap[1]);       // round outputs 1, 3
-    if (p.R >= 2) sp.add_n<G1Affine>(p.cap[2]);       // round output 2
-    for (int r = 0; r < p.R; r++) sp.add_n<uint32_t>(p.NB + 1);  // round offsets
-    if (p.R >= 1) {                                   // sized for round 1, reused by later rounds
-        const uint64_t ctas = pr_ctas(p.cap[0]);
-        sp.add_n<Fq>(ctas * PR_T * 4);                // denominator prefixes
-        sp.add_n<uint2>(ctas * PR_T * 4);             // jobs
-        sp.add_n<uint32_t>(ctas * PR_T);              // jobs per thread
-        sp.add_n<Fq>(ctas * 2 * PR_T);                // product trees
-        sp.add_n<Fq>(ctas);                           // CTA totals
-        sp.add(fq_batch_invert_scratch(ctas));
-    }
-    if (p.tn == 0 && p.R == 0) sp.add_n<G1Affine>(2 * p.n);  // P_i and phi(P_i) in the lazy form (x 2^261)
+    if (p.tn == 0) sp.add_n<G1Affine>(2 * p.n);  // P_i and phi(P_i) in the lazy form (x 2^261)
 }
 
 MsmScratch msm_carve(const MsmPlan& p, ScratchArena& ar, bool scalar_host, bool bases_host)
@@ -263,31 +244,12 @@ MsmScratch msm_carve(const MsmPlan& p, ScratchArena& ar, bool scalar_host, bool 
     s.sorted = ar.take_n<uint32_t>(p.max_entries);
     s.buckets = ar.take_n<G1Xyzz>(p.NB);
     s.heads = ar.take_n<G1Xyzz>(p.max_chunks);
-    s.dense = ar.take_n<uint32_t>(p.max_dense + 1);
-    s.pieces = ar.take_n<G1Xyzz>(p.max_dense * DENSE_PIECES);
-    s.segacc = ar.take_n<G1Xyzz>((uint64_t)p.Wr * p.S);
-    s.segrun = ar.take_n<G1Xyzz>((uint64_t)p.Wr * p.S);
-    s.bits = ar.take_n<G1Xyzz>((uint64_t)std::max(p.W, p.Wr) * (p.NBITS + 1));
-    s.bitparts = p.BP > 1 ? ar.take_n<G1Xyzz>((uint64_t)p.Wr * (p.NBITS + 1) * p.BP) : nullptr;
-    // a counter per bit sum: at most 20 (NBITS + 1) a window, 128 bytes set aside for each
-    s.tailctr = (uint32_t*)ar.take_n<G1Xyzz>(std::max(p.W, p.Wr));
+    s.dense = ar.take_n<uint32_t>(p.max_dense + 2);
+    s.items = ar.take_n<uint2>(p.max_items);
+    for (int k = 0; k < 2; k++) s.fold[k] = ar.take_n<G1Xyzz>(msm_fold_points(p, k));
+    s.tailctr = ar.take_n<uint32_t>(p.leaves);
     s.result = ar.take_n<G1Jac>(1);
-    s.pts[0] = p.R >= 1 ? ar.take_n<G1Affine>(p.cap[1]) : nullptr;
-    s.pts[1] = p.R >= 2 ? ar.take_n<G1Affine>(p.cap[2]) : nullptr;
-    for (int r = 0; r < 3; r++) s.roff[r] = r < p.R ? ar.take_n<uint32_t>(p.NB + 1) : nullptr;
-    s.pr_pref = nullptr; s.pr_job = nullptr; s.pr_nj = nullptr; s.pr_tree = nullptr; s.pr_tot = nullptr;
-    s.pr_inv_scratch = nullptr; s.pr_inv_bytes = 0;
-    if (p.R >= 1) {
-        const uint64_t ctas = pr_ctas(p.cap[0]);
-        s.pr_pref = ar.take_n<Fq>(ctas * PR_T * 4);
-        s.pr_job = ar.take_n<uint2>(ctas * PR_T * 4);
-        s.pr_nj = ar.take_n<uint32_t>(ctas * PR_T);
-        s.pr_tree = ar.take_n<Fq>(ctas * 2 * PR_T);
-        s.pr_tot = ar.take_n<Fq>(ctas);
-        s.pr_inv_bytes = fq_batch_invert_scratch(ctas);
-        s.pr_inv_scratch = ar.take(s.pr_inv_bytes);
-    }
-    s.rbases = (p.tn == 0 && p.R == 0) ? ar.take_n<G1Affine>(2 * p.n) : nullptr;
+    s.rbases = p.tn == 0 ? ar.take_n<G1Affine>(2 * p.n) : nullptr;
     return s;
 }
 
@@ -426,59 +388,6 @@ __global__ void k_msm_glv_hist(const Fr* __restrict__ sc, uint4* __restrict__ vs
     }
 }
 
-#if H2B_EXPERIMENTS
-// One thread per chunk of K sorted entries; the running bucket sum stays in
-// 29-bit limb form and is packed to the canonical 8 x 32 image when stored.
-// PTS: the entries are the affine points themselves (bases[e]), as left by
-// the pairing rounds, instead of signed (GLV) indices into the bases.
-template <int MODE, bool PTS>
-__global__ void __launch_bounds__(128, MODE == 1 ? 2 : (MODE >= 3 ? MODE + 1 : 3)) k_msm_accumulate(const uint32_t* __restrict__ sorted,
-                                                        const uint32_t* __restrict__ offsets, uint64_t NB, uint32_t K,
-                                                        const G1Affine* __restrict__ bases, G1Xyzz* __restrict__ buckets,
-                                                        G1Xyzz* __restrict__ heads)
-{
-    const uint32_t M = offsets[NB];
-    const uint64_t nchunks = (M + (uint64_t)K - 1) / K;
-    for (uint64_t t = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; t < nchunks;
-         t += (uint64_t)gridDim.x * blockDim.x) {
-        const uint32_t start = (uint32_t)(t * K);
-        const uint32_t end = ((uint64_t)start + K < (uint64_t)M) ? start + K : M;
-        uint64_t lo = 0, hi = NB;  // offsets[lo] <= start < offsets[hi]
-        while (hi - lo > 1) {
-            uint64_t mid = (lo + hi) >> 1;
-            if (offsets[mid] <= start) lo = mid; else hi = mid;
-        }
-        uint64_t b = lo;
-        uint32_t next = offsets[b + 1];
-        bool head = offsets[b] < start;
-        G1XyzzL acc = xyzzl_inf();
-        for (uint32_t e = start; e < end; e++) {
-            if (e == next) {
-                if (head) st_xyzz(&heads[t], xyzzl_to(acc)); else st_xyzz(&buckets[b], xyzzl_to(acc));
-                acc = xyzzl_inf();
-                head = false;
-                do { b++; next = offsets[b + 1]; } while (next == e);
-            }
-            if (PTS) {  // contiguous affine points left by the pairing rounds
-                const G1Affine P = ld_affine(&bases[e]);
-                if (is_inf(P)) continue;
-                xyzzl_madd<MODE>(acc, to_l(P.x), to_l(P.y));
-                continue;
-            }
-            const uint32_t ent = sorted[e];
-            const uint32_t v = ent & ~SIGN_BIT;
-            G1Affine P = ld_affine(&bases[v >> 1]);
-            if (is_inf(P)) continue;
-            if (ent & SIGN_BIT) P.y = fneg(P.y);
-            FqL qx = to_l(P.x);
-            if (v & 1u) qx = fl_mul(qx, to_l(glv::beta()));  // phi(P)
-            xyzzl_madd<MODE>(acc, qx, to_l(P.y));
-        }
-        if (head) st_xyzz(&heads[t], xyzzl_to(acc)); else st_xyzz(&buckets[b], xyzzl_to(acc));
-    }
-}
-
-#endif  // H2B_EXPERIMENTS
 
 // Bases (affine, memory image x 2^256 mod p) -> canonical x 2^261 mod p, the
 // form the lazy accumulation reads; infinity (0, 0) stays (0, 0).
@@ -499,6 +408,17 @@ __global__ void k_to_r261(const G1Affine* in, G1Affine* out, uint64_t n, G1Affin
     }
 }
 
+// Entries per chunk for M sorted entries (MsmChunk: the plan's rule).
+__device__ __forceinline__ uint32_t chunk_entries(const MsmChunk& k, uint32_t M)
+{
+    if (k.fixed) return k.fixed;
+    const uint32_t wave = k.threads * k.cap;               // entries of one wave of the largest chunks
+    const uint32_t waves = M / wave + (M % wave != 0);
+    const uint32_t threads = k.threads * (waves ? waves : 1u);
+    const uint32_t n = M / threads + (M % threads != 0);
+    return n < ACC_MIN_K ? ACC_MIN_K : n;
+}
+
 // The accumulation in the lazy form (curve.cuh, lazy.cuh): same chunking,
 // bucket boundaries and outputs as k_msm_accumulate, over bases in the
 // x 2^261 form.  The accumulator's additions and subtractions are one-step
@@ -508,13 +428,14 @@ __global__ void k_to_r261(const G1Affine* in, G1Affine* out, uint64_t n, G1Affin
 // bases: phi_off = n; window tables: W n, after all slices).
 __global__ void __launch_bounds__(128, 3) k_msm_accumulate_z(const uint32_t* __restrict__ sorted,
                                                              const uint32_t* __restrict__ offsets, uint64_t NB,
-                                                             uint32_t K, const G1Affine* __restrict__ bases,
+                                                             const MsmChunk kc, const G1Affine* __restrict__ bases,
                                                              uint64_t phi_off, G1Xyzz* __restrict__ buckets,
                                                              G1Xyzz* __restrict__ heads)
 {
     const FqZ one = fz_from_words(to_r261(Fq::one()));           // 1 in the lazy form (2^261 mod p)
     const FqZ r256 = fz_from_words(Fq::one());                    // 2^256 mod p, for the stores
     const uint32_t M = offsets[NB];
+    const uint32_t K = chunk_entries(kc, M);
     const uint64_t nchunks = (M + (uint64_t)K - 1) / K;
     for (uint64_t t = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; t < nchunks;
          t += (uint64_t)gridDim.x * blockDim.x) {
@@ -576,13 +497,14 @@ __device__ __forceinline__ Fq from_r261(const Fq& v)
 // The same accumulation with coordinates in [0, 2p) on the even/odd product:
 // bases are read in the x 2^261 storage form and divided by 32 on load;
 // buckets leave in the canonical memory image.
-__global__ void __launch_bounds__(128, ACC_BLOCKS) k_msm_accumulate_e(const uint32_t* __restrict__ sorted,
+__global__ void __launch_bounds__(128, 4) k_msm_accumulate_e(const uint32_t* __restrict__ sorted,
                                                              const uint32_t* __restrict__ offsets, uint64_t NB,
-                                                             uint32_t K, const G1Affine* __restrict__ bases,
+                                                             const MsmChunk kc, const G1Affine* __restrict__ bases,
                                                              uint64_t phi_off, G1Xyzz* __restrict__ buckets,
                                                              G1Xyzz* __restrict__ heads, uint32_t pf)
 {
     const uint32_t M = offsets[NB];
+    const uint32_t K = chunk_entries(kc, M);
     const uint64_t nchunks = (M + (uint64_t)K - 1) / K;
     for (uint64_t t = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; t < nchunks;
          t += (uint64_t)gridDim.x * blockDim.x) {
@@ -617,217 +539,119 @@ __global__ void __launch_bounds__(128, ACC_BLOCKS) k_msm_accumulate_e(const uint
             const Fq qx = from_r261(P.x);
             Fq qy = from_r261(P.y);
             if (ent & SIGN_BIT) qy = qsub(Fq::zero(), qy);
-            xyzze_madd<ACC_INLINE>(acc, qx, qy);
+            xyzze_madd<true>(acc, qx, qy);
         }
         st_xyzze(head ? &heads[t] : &buckets[b], acc);
     }
 }
 
-#if H2B_EXPERIMENTS
-// ---- pairing rounds (batch-affine bucket additions) -----------------------
-// Round r adds the points of every bucket pairwise in affine coordinates:
-// entries (2j, 2j+1) of a bucket become output point j (an odd last entry is
-// copied), so each round halves every bucket.  lambda = (y2 - y1) / (x2 - x1)
-// (or 3 x1^2 / (2 y1) for equal points) needs one inversion per addition; all
-// denominators share inversions through Montgomery's trick, so an addition
-// costs about 6 products against 10 for an XYZZ mixed addition, and the
-// additions of a thread are independent of each other.  Infinity inputs pass
-// the other point through; P + (-P) gives infinity, written as (0, 0) like an
-// input base.  A round is three launches: forward products with a product
-// tree per CTA, one batch inversion of all CTA totals, backward pass.  (An
-// inversion inside each CTA would put a long serial binary GCD behind every
-// 512 additions.)
 
-__device__ __forceinline__ void st_affine(G1Affine* p, const G1Affine& a)
+// pieces of a long bucket with m chunk heads (one warp each)
+__device__ __forceinline__ uint32_t head_pieces(uint32_t m)
 {
-    st(&p->x, a.x);
-    st(&p->y, a.y);
+    const uint32_t n = (m + HEADS_PIECE - 1) / HEADS_PIECE;
+    return n < HEADS_PIECES_MAX ? n : HEADS_PIECES_MAX;
 }
 
-template <bool FIRST>
-__device__ __forceinline__ G1Affine pr_load(const uint32_t* __restrict__ sorted, const G1Affine* __restrict__ src,
-                                            uint32_t e)
+// Adds the chunk heads of each bucket to what the bucket's first chunk left
+// in it, G lanes per bucket (a serial share each, then a tree).  A bucket with
+// more than `limit` heads is listed instead, with its pieces, for
+// k_msm_heads.  Latency-bound unless the buckets are many: one lane per bucket
+// took 161 us for 4096 buckets of 19 heads.
+template <int G>
+__global__ void __launch_bounds__(128) k_msm_fixup(const uint32_t* __restrict__ offsets, uint64_t NB, const MsmChunk kc,
+                                                   G1Xyzz* __restrict__ buckets, const G1Xyzz* __restrict__ heads,
+                                                   uint32_t limit, uint32_t* __restrict__ dense, uint64_t max_dense,
+                                                   uint2* __restrict__ items, uint64_t max_items)
 {
-    if (!FIRST) return ld_affine(&src[e]);
-    const uint32_t ent = sorted[e];
-    const uint32_t v = ent & ~SIGN_BIT;
-    G1Affine P = ld_affine(&src[v >> 1]);
-    if (is_inf(P)) return P;
-    if (v & 1u) P.x = P.x * glv::beta();  // phi(P)
-    if (ent & SIGN_BIT) P.y = fneg(P.y);
-    return P;
-}
-
-// Denominator and numerator of lambda for P1 + P2 (both finite, P2 != -P1).
-__device__ __forceinline__ void pr_slope_terms(const G1Affine& P1, const G1Affine& P2, FqL& d, FqL& num)
-{
-    const FqL x1 = to_l(P1.x), y1 = to_l(P1.y);
-    if (P1.x != P2.x) {
-        d = fl_sub(to_l(P2.x), x1);
-        num = fl_sub(to_l(P2.y), y1);
-    } else {
-        d = fl_add(y1, y1);
-        const FqL xx = fl_sqr(x1);
-        num = fl_add(fl_add(xx, xx), xx);
-    }
-}
-
-// Forward half.  A thread owns PR_E input entries; every entry at an even
-// position of its bucket starts an addition with the next entry (at most 4
-// per thread).  Running products of the denominators go to g_pref, the jobs
-// to g_job / g_nj, the CTA's product tree over the thread totals to g_tree
-// (nodes 1 .. 2T-1) and its root to g_tot[cta].  CTAs past the last entry
-// only set g_tot[cta] = 1.
-template <bool FIRST>
-__global__ void __launch_bounds__(PR_T) k_msm_pair_fwd(const uint32_t* __restrict__ sorted,
-                                                       const G1Affine* __restrict__ src,
-                                                       const uint32_t* __restrict__ in_off, uint64_t NB,
-                                                       const uint32_t* __restrict__ out_off,
-                                                       G1Affine* __restrict__ out_pts, Fq* __restrict__ g_pref,
-                                                       uint2* __restrict__ g_job, uint32_t* __restrict__ g_nj,
-                                                       Fq* __restrict__ g_tree, Fq* __restrict__ g_tot)
-{
-    __shared__ FqL tree[2 * PR_T];
-    const int t = threadIdx.x;
-    const uint32_t M = in_off[NB];
-    const uint64_t cta = blockIdx.x;
-    const uint64_t cta_start = cta * PR_T * PR_E;
-    if (cta_start >= M) {
-        if (t == 0) st(&g_tot[cta], Fq::one());
-        return;  // the whole CTA leaves before any barrier
-    }
-    const uint64_t gt = cta * PR_T + t;
-    const uint64_t s64 = cta_start + (uint64_t)t * PR_E;
-    uint32_t nj = 0;
-    FqL acc = to_l(Fq::one());
-    if (s64 < M) {
-        const uint32_t s = (uint32_t)s64;
-        const uint32_t end = (s64 + PR_E < M) ? s + PR_E : M;
-        uint64_t lo = 0, hi = NB;  // in_off[lo] <= s < in_off[hi]
-        while (hi - lo > 1) {
-            const uint64_t mid = (lo + hi) >> 1;
-            if (in_off[mid] <= s) lo = mid; else hi = mid;
-        }
-        uint64_t b = lo;
-        uint32_t bstart = in_off[b], bnext = in_off[b + 1];
-        for (uint32_t e = s; e < end; e++) {
-            while (e >= bnext) { b++; bstart = bnext; bnext = in_off[b + 1]; }
-            const uint32_t local = e - bstart;
-            if (local & 1u) continue;
-            const uint32_t o = out_off[b] + (local >> 1);
-            const G1Affine P1 = pr_load<FIRST>(sorted, src, e);
-            if (e + 1 >= bnext) { st_affine(&out_pts[o], P1); continue; }
-            const G1Affine P2 = pr_load<FIRST>(sorted, src, e + 1);
-            if (is_inf(P1) || is_inf(P2)) { st_affine(&out_pts[o], is_inf(P1) ? P2 : P1); continue; }
-            if (P1.x == P2.x && P1.y != P2.y) {  // P2 = -P1
-                G1Affine z;
-                z.x = Fq::zero(); z.y = Fq::zero();
-                st_affine(&out_pts[o], z);
-                continue;
+    __shared__ G1Xyzz red[G > 1 ? 128 : 1];
+    const uint32_t K = chunk_entries(kc, offsets[NB]);
+    const uint32_t lane = threadIdx.x & 31, j = lane % G;
+    const uint64_t warps = (uint64_t)gridDim.x * (blockDim.x >> 5);
+    constexpr uint32_t PER = 32 / G;                 // buckets per warp
+    for (uint64_t base = ((uint64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5)) * PER; base < NB;
+         base += warps * PER) {                      // uniform within the warp
+        const uint64_t gb = base + lane / G;
+        uint32_t t0 = 0, t1 = 0;
+        bool take = false;
+        if (gb < NB) {
+            const uint32_t s = offsets[gb], e = offsets[gb + 1];
+            if (s == e) {
+                if (j == 0) st_xyzz(&buckets[gb], xyzz_inf());
+            } else {
+                t0 = s / K;
+                t1 = (e - 1) / K;
+                if (t1 - t0 > limit) {
+                    if (j == 0) {
+                        const uint32_t n = head_pieces(t1 - t0), at = atomicAdd(&dense[max_dense + 1], n);
+                        dense[atomicAdd(&dense[max_dense], 1u)] = (uint32_t)gb;
+                        for (uint32_t p = 0; p < n && at + p < max_items; p++) items[at + p] = make_uint2((uint32_t)gb, p);
+                    }
+                } else {
+                    take = t1 > t0;
+                }
             }
-            FqL d, num;
-            pr_slope_terms(P1, P2, d, num);
-            acc = nj == 0 ? d : fl_mul(acc, d);
-            st(&g_pref[gt * 4 + nj], from_l(acc));
-            g_job[gt * 4 + nj] = make_uint2(e, o);
-            nj++;
         }
-    }
-    g_nj[gt] = nj;
-    tree[PR_T + t] = acc;
-    __syncthreads();
-    for (int w = PR_T / 2; w >= 1; w >>= 1) {
-        if (t < w) tree[w + t] = fl_mul(tree[2 * (w + t)], tree[2 * (w + t) + 1]);
-        __syncthreads();
-    }
-    for (int i = t + 1; i < 2 * PR_T; i += PR_T) st(&g_tree[cta * 2 * PR_T + i], from_l(tree[i]));
-    if (t == 0) st(&g_tot[cta], from_l(tree[1]));
-}
-
-// Backward half: the inverted CTA total (g_tot[cta]) goes down the stored
-// tree to every thread, which walks its jobs in reverse, recovers each
-// denominator's inverse from its prefix, and writes P1 + P2.
-template <bool FIRST>
-__global__ void __launch_bounds__(PR_T) k_msm_pair_bwd(const uint32_t* __restrict__ sorted,
-                                                       const G1Affine* __restrict__ src,
-                                                       const uint32_t* __restrict__ in_off, uint64_t NB,
-                                                       G1Affine* __restrict__ out_pts, const Fq* __restrict__ g_pref,
-                                                       const uint2* __restrict__ g_job,
-                                                       const uint32_t* __restrict__ g_nj,
-                                                       const Fq* __restrict__ g_tree, const Fq* __restrict__ g_tot)
-{
-    __shared__ FqL tree[2 * PR_T];
-    const int t = threadIdx.x;
-    const uint32_t M = in_off[NB];
-    const uint64_t cta = blockIdx.x;
-    if (cta * PR_T * PR_E >= M) return;  // the whole CTA
-    const uint64_t gt = cta * PR_T + t;
-    for (int i = t + 1; i < 2 * PR_T; i += PR_T) tree[i] = to_l(ld(&g_tree[cta * 2 * PR_T + i]));
-    __syncthreads();
-    if (t == 0) tree[1] = to_l(ld(&g_tot[cta]));
-    __syncthreads();
-    for (int w = 1; w < PR_T; w <<= 1) {
-        if (t < w) {
-            const int k = w + t;
-            const FqL inv = tree[k], l = tree[2 * k], r = tree[2 * k + 1];
-            const Fl2<FqCfg> lr = fl_mul2(inv, r, inv, l);
-            tree[2 * k] = lr.a;
-            tree[2 * k + 1] = lr.b;
+        G1Xyzz acc = xyzz_inf();
+        if (take) {
+            if (j == 0) acc = ld_xyzz(&buckets[gb]);
+            for (uint32_t t = t0 + 1 + j; t <= t1; t += G) xyzze_add<false>(acc, ld_xyzz(&heads[t]));
         }
-        __syncthreads();
-    }
-    FqL inv = tree[PR_T + t];
-    const int nj = (int)g_nj[gt];
-    for (int k = nj - 1; k >= 0; k--) {
-        const uint2 job = g_job[gt * 4 + k];
-        const G1Affine P1 = pr_load<FIRST>(sorted, src, job.x);
-        const G1Affine P2 = pr_load<FIRST>(sorted, src, job.x + 1);
-        FqL d, num;
-        pr_slope_terms(P1, P2, d, num);
-        FqL inv_d;
-        if (k > 0) {
-            const Fl2<FqCfg> r = fl_mul2(inv, to_l(ld(&g_pref[gt * 4 + k - 1])), inv, d);
-            inv_d = r.a;
-            inv = r.b;
-        } else {
-            inv_d = inv;
+        if (G > 1) {
+            red[threadIdx.x] = acc;
+#pragma unroll 1
+            for (int h = G / 2; h > 0; h >>= 1) {
+                __syncwarp();
+                if (take && j < (uint32_t)h) {
+                    xyzze_add<false>(acc, red[threadIdx.x + h]);
+                    red[threadIdx.x] = acc;
+                }
+            }
+            __syncwarp();
         }
-        const FqL x1 = to_l(P1.x), y1 = to_l(P1.y);
-        const FqL lam = fl_mul(num, inv_d);
-        const FqL x3 = fl_sub(fl_sub(fl_sqr(lam), x1), to_l(P2.x));
-        const FqL y3 = fl_sub(fl_mul(lam, fl_sub(x1, x3)), y1);
-        G1Affine R;
-        R.x = from_l(x3);
-        R.y = from_l(y3);
-        st_affine(&out_pts[job.y], R);
+        if (take && j == 0) st_xyzze(&buckets[gb], acc);
     }
 }
 
-// Per-bucket entry counts after a pairing round: ceil(count / 2).
-__global__ void k_msm_half_counts(const uint32_t* __restrict__ in_off, uint64_t NB, uint32_t* __restrict__ out_cnt)
+// One warp per piece of a long bucket: the sum of its slice of chunk heads,
+// left in place of the slice's first head (or added to the bucket when the
+// piece is the only one).
+__global__ void __launch_bounds__(128) k_msm_heads(const uint32_t* __restrict__ offsets, uint64_t NB, const MsmChunk kc,
+                                                   G1Xyzz* __restrict__ buckets, G1Xyzz* heads,
+                                                   const uint32_t* __restrict__ dense, uint64_t max_dense,
+                                                   const uint2* __restrict__ items)
 {
-    for (uint64_t b = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; b < NB; b += (uint64_t)gridDim.x * blockDim.x)
-        out_cnt[b] = (in_off[b + 1] - in_off[b] + 1) >> 1;
-}
-
-#endif  // H2B_EXPERIMENTS
-
-__global__ void k_msm_fixup(const uint32_t* __restrict__ offsets, uint64_t NB, uint32_t K, G1Xyzz* __restrict__ buckets,
-                            const G1Xyzz* __restrict__ heads, uint32_t* __restrict__ dense, uint64_t max_dense)
-{
-    for (uint64_t gb = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; gb < NB; gb += (uint64_t)gridDim.x * blockDim.x) {
-        uint32_t s = offsets[gb], e = offsets[gb + 1];
-        if (s == e) { st_xyzz(&buckets[gb], xyzz_inf()); continue; }
-        uint32_t t0 = s / K, t1 = (e - 1) / K;
-        if (t1 == t0) continue;
-        if (t1 - t0 > DENSE_LIMIT) {
-            uint32_t idx = atomicAdd(&dense[max_dense], 1u);
-            if (idx < max_dense) dense[idx] = (uint32_t)gb;
-            continue;
+    __shared__ G1Xyzz red[128];
+    const uint32_t n = dense[max_dense + 1];
+    if (blockIdx.x * (blockDim.x >> 5) >= n) return;
+    const uint32_t K = chunk_entries(kc, offsets[NB]);
+    const uint32_t lane = threadIdx.x & 31;
+    for (uint32_t it = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); it < n;
+         it += gridDim.x * (blockDim.x >> 5)) {
+        const uint2 item = items[it];
+        const uint32_t t0 = offsets[item.x] / K, t1 = (offsets[item.x + 1] - 1) / K, m = t1 - t0;
+        const uint32_t P = head_pieces(m);
+        const uint32_t b0 = (uint32_t)((uint64_t)m * item.y / P), b1 = (uint32_t)((uint64_t)m * (item.y + 1) / P);
+        G1Xyzz acc = xyzz_inf();
+        for (uint32_t i = b0 + lane; i < b1; i += 32) xyzze_add<false>(acc, ld_xyzz(&heads[t0 + 1 + i]));
+        red[threadIdx.x] = acc;
+#pragma unroll 1
+        for (int h = 16; h > 0; h >>= 1) {
+            __syncwarp();
+            if (lane < (uint32_t)h) {
+                xyzze_add<false>(acc, red[threadIdx.x + h]);
+                red[threadIdx.x] = acc;
+            }
         }
-        G1Xyzz acc = ld_xyzz(&buckets[gb]);
-        for (uint32_t t = t0 + 1; t <= t1; t++) xyzze_add<false>(acc, ld_xyzz(&heads[t]));
-        st_xyzze(&buckets[gb], acc);
+        if (lane == 0) {
+            if (P > 1) {
+                st_xyzze(&heads[t0 + 1 + b0], acc);
+            } else {
+                xyzze_add<false>(acc, ld_xyzz(&buckets[item.x]));
+                st_xyzze(&buckets[item.x], acc);
+            }
+        }
+        __syncwarp();
     }
 }
 
@@ -842,7 +666,9 @@ __device__ G1Xyzz block_sum_xyzz(uint64_t n, Get get)
     for (uint64_t i = threadIdx.x; i < n; i += blockDim.x) xyzze_add<false>(acc, get(i));
     red[threadIdx.x] = acc;
     __syncthreads();
-    for (int h = blockDim.x >> 1; h > 0; h >>= 1) {
+    int h = blockDim.x >> 1;
+    while (h > 1 && (uint64_t)h >= n) h >>= 1;         // no sums above n
+    for (; h > 0; h >>= 1) {
         if ((int)threadIdx.x < h) {
             G1Xyzz a = red[threadIdx.x];
             xyzze_add<false>(a, red[threadIdx.x + h]);
@@ -855,114 +681,80 @@ __device__ G1Xyzz block_sum_xyzz(uint64_t n, Get get)
     return r;
 }
 
-// Dense buckets (spanning more than DENSE_LIMIT chunks): DENSE_PIECES CTAs
-// each tree-sum a slice of the bucket's chunk partials, then one warp per
-// bucket tree-sums the pieces into the bucket.
-__global__ void __launch_bounds__(256) k_msm_dense_pieces(const uint32_t* __restrict__ offsets, uint64_t NB,
-                                                          uint32_t K, const G1Xyzz* __restrict__ heads,
-                                                          const uint32_t* __restrict__ dense,
-                                                          G1Xyzz* __restrict__ pieces)
+// One CTA per long bucket of more than one piece: the pieces' sums into the bucket.
+__global__ void __launch_bounds__(256) k_msm_heads_merge(const uint32_t* __restrict__ offsets, uint64_t NB,
+                                                         const MsmChunk kc, G1Xyzz* __restrict__ buckets,
+                                                         const G1Xyzz* __restrict__ heads,
+                                                         const uint32_t* __restrict__ dense, uint64_t max_dense)
 {
-    const uint32_t items = dense[NB] * DENSE_PIECES;
-    for (uint32_t it = blockIdx.x; it < items; it += gridDim.x) {
-        uint32_t i = it / DENSE_PIECES, p = it % DENSE_PIECES;
-        uint32_t gb = dense[i];
-        uint32_t t0 = offsets[gb] / K, t1 = (offsets[gb + 1] - 1) / K;
-        uint64_t len = t1 - t0;  // heads t0+1 .. t1
-        uint64_t b0 = len * p / DENSE_PIECES, b1 = len * (p + 1) / DENSE_PIECES;
-        G1Xyzz r = block_sum_xyzz(b1 - b0, [&](uint64_t j) { return ld_xyzz(&heads[t0 + 1 + b0 + j]); });
-        if (threadIdx.x == 0) st_xyzze(&pieces[it], r);
-        __syncthreads();
-    }
-}
-
-__global__ void __launch_bounds__(DENSE_PIECES) k_msm_dense_merge(const uint64_t NB, G1Xyzz* __restrict__ buckets,
-                                                                  const uint32_t* __restrict__ dense,
-                                                                  const G1Xyzz* __restrict__ pieces)
-{
-    __shared__ G1Xyzz red[DENSE_PIECES];
-    const uint32_t cnt = dense[NB];
+    const uint32_t cnt = dense[max_dense];
+    if (blockIdx.x >= cnt) return;
+    const uint32_t K = chunk_entries(kc, offsets[NB]);
     for (uint32_t i = blockIdx.x; i < cnt; i += gridDim.x) {
-        red[threadIdx.x] = ld_xyzz(&pieces[(uint64_t)i * DENSE_PIECES + threadIdx.x]);
-        __syncthreads();
-        for (int h = DENSE_PIECES / 2; h > 0; h >>= 1) {
-            if ((int)threadIdx.x < h) {
-                G1Xyzz a = red[threadIdx.x];
-                xyzze_add<false>(a, red[threadIdx.x + h]);
-                red[threadIdx.x] = a;
-            }
-            __syncthreads();
-        }
+        const uint32_t gb = dense[i];
+        const uint32_t t0 = offsets[gb] / K, m = (offsets[gb + 1] - 1) / K - t0, P = head_pieces(m);
+        if (P <= 1) continue;
+        G1Xyzz r = block_sum_xyzz(P, [&](uint64_t p) {
+            return ld_xyzz(&heads[t0 + 1 + (uint32_t)((uint64_t)m * p / P)]);
+        });
         if (threadIdx.x == 0) {
-            uint32_t gb = dense[i];
-            G1Xyzz acc = ld_xyzz(&buckets[gb]);
-            xyzze_add<false>(acc, red[0]);
-            st_xyzze(&buckets[gb], acc);
+            xyzze_add<false>(r, ld_xyzz(&buckets[gb]));
+            st_xyzze(&buckets[gb], r);
         }
         __syncthreads();
     }
 }
 
-// Bucket reduction, W_w = sum_{j<H} (j+1) B_{w,j}, in three parallel steps.
-// 1. Thread (w, s), segment s = buckets s*L .. s*L+L-1:
-//      acc_s = sum_j (j - sL + 1) B_j      run_s = sum_j B_j
-// 2. CTA (w, k): k < NBITS: T_k = sum over s with bit k set of run_s;
-//                k = NBITS: T = sum_s acc_s.
-// 3. Thread w: W_w = T + L * sum_k 2^k T_k (Horner over the bits).
-__global__ void __launch_bounds__(128) k_msm_segments(const G1Xyzz* __restrict__ buckets, int W, uint32_t H,
-                                                      uint32_t L, uint32_t S, G1Xyzz* __restrict__ segacc,
-                                                      G1Xyzz* __restrict__ segrun, uint32_t* __restrict__ ctr,
-                                                      uint32_t nctr)
+// Bucket reduction, W_w = sum_{j<H} (j+1) B_{w,j} = sum_j B_j + sum_k 2^k T_k
+// with T_k the sum of the buckets whose index has bit k set.
+// Folding the top index bit of an array y of n sums gives its T as the upper
+// half of y and a new y of the pairwise sums of both halves; every T array
+// found so far is halved by the same step.  A pass folds `m` bits: CTA (w, blk)
+// takes 2^m consecutive elements of each of the `arrays` arrays of window w
+// (array 0 is y, the others are T arrays; `len` elements each) and writes one
+// element of each of the arrays + m arrays that result.
+// Two additions per bucket, all of them in parallel within a step, so the
+// depth is the number of bits: running sums over 8-bucket segments and then
+// per-bit sums of the segments (16 and 16 additions one after the other at
+// c = 16) took 146 + 212 us for 8 windows of 2^15 buckets and 104 + 210 us for
+// one; the two passes here 117 + 60 and 76 + 53 us.
+__global__ void __launch_bounds__(FOLD_THREADS) k_msm_fold(const G1Xyzz* __restrict__ in, uint32_t arrays, uint32_t len,
+                                                           int m, G1Xyzz* __restrict__ out, uint32_t* __restrict__ ctr,
+                                                           uint32_t nctr)
 {
+    extern __shared__ uint4 fold_smem[];
+    G1Xyzz* sm = reinterpret_cast<G1Xyzz*>(fold_smem);
+    const uint32_t t = threadIdx.x;
+    const uint32_t blocks = len >> m, w = blockIdx.x / blocks, blk = blockIdx.x % blocks;
     if (blockIdx.x == 0)
-        for (uint32_t i = threadIdx.x; i < nctr; i += blockDim.x) ctr[i] = 0;
-    uint64_t total = (uint64_t)W * S;
-    for (uint64_t id = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; id < total;
-         id += (uint64_t)gridDim.x * blockDim.x) {
-        uint64_t w = id / S, s = id % S;
-        const G1Xyzz* B = buckets + w * H + s * L;
-        G1Xyzz run = xyzz_inf(), acc = xyzz_inf();
-        for (int j = (int)L - 1; j >= 0; j--) {
-            xyzze_add<false>(run, ld_xyzz(&B[j]));
-            xyzze_add<false>(acc, run);
+        for (uint32_t i = t; i < nctr; i += blockDim.x) ctr[i] = 0;
+    const G1Xyzz* src = in + (uint64_t)w * arrays * len + ((uint64_t)blk << m);
+    uint32_t A = arrays;
+#pragma unroll 1
+    for (int step = 0; step < m; step++) {
+        const int lh = m - 1 - step;                   // log2 of the halved length
+        const uint32_t half = 1u << lh, a = t >> lh, i = t & (half - 1);
+        const bool active = t < A << lh;
+        G1Xyzz x, y;
+        if (active) {
+            if (step == 0) {
+                x = ld_xyzz(&src[(uint64_t)a * len + i]);
+                y = ld_xyzz(&src[(uint64_t)a * len + i + half]);
+            } else {
+                x = sm[(a << (lh + 1)) + i];
+                y = sm[(a << (lh + 1)) + i + half];
+            }
         }
-        st_xyzze(&segacc[id], acc);
-        st_xyzze(&segrun[id], run);
+        __syncthreads();
+        if (active) {
+            if (a == 0) sm[(A << lh) + i] = y;         // the folded bit's T array
+            xyzze_add<false>(x, y);
+            sm[(a << lh) + i] = x;
+        }
+        __syncthreads();
+        A++;
     }
-}
-
-// CTA (w, k, part): part `part` of BP of bit sum (w, k); with BP = 1 the
-// CTA writes the bit sum itself, else its partial (out[(w, k) * BP + part]).
-__global__ void __launch_bounds__(256) k_msm_bitsums(const G1Xyzz* __restrict__ segacc,
-                                                     const G1Xyzz* __restrict__ segrun, uint32_t S, int nbits,
-                                                     uint32_t BP, G1Xyzz* __restrict__ out)
-{
-    const uint32_t wk = blockIdx.x / BP, part = blockIdx.x % BP;
-    const uint32_t w = wk / (nbits + 1);
-    const int k = (int)(wk % (nbits + 1));
-    // k == nbits: all S weighted sums; else the S/2 plain sums with bit k set,
-    // s = (hi << (k+1)) | (1 << k) | lo
-    const bool all = (k == nbits);
-    const uint64_t lo_mask = all ? 0 : (1ull << k) - 1;
-    const uint64_t items = all ? S : S / 2;
-    const uint64_t per = (items + BP - 1) / BP;
-    const uint64_t j0 = std::min<uint64_t>(items, (uint64_t)part * per);
-    const uint64_t j1 = std::min<uint64_t>(items, j0 + per);
-    G1Xyzz r = block_sum_xyzz(j1 - j0, [&](uint64_t jj) {
-        const uint64_t j = j0 + jj;
-        if (all) return ld_xyzz(&segacc[(uint64_t)w * S + j]);
-        uint64_t s = ((j & ~lo_mask) << 1) | (1ull << k) | (j & lo_mask);
-        return ld_xyzz(&segrun[(uint64_t)w * S + s]);
-    });
-    if (threadIdx.x == 0) st_xyzze(&out[blockIdx.x], r);
-}
-
-// CTA (w, k): the BP partials of bit sum (w, k).
-__global__ void __launch_bounds__(256) k_msm_bitparts(const G1Xyzz* __restrict__ parts, uint32_t BP,
-                                                      G1Xyzz* __restrict__ bits)
-{
-    G1Xyzz r = block_sum_xyzz(BP, [&](uint64_t j) { return ld_xyzz(&parts[(uint64_t)blockIdx.x * BP + j]); });
-    if (threadIdx.x == 0) st_xyzze(&bits[blockIdx.x], r);
+    if (t < A) st_xyzze(&out[((uint64_t)w * A + t) * blocks + blk], sm[t]);
 }
 
 // A merged run over a window table: window j of the reduction is job j's
@@ -972,33 +764,44 @@ struct MsmOuts {
     G1Jac* p[MSM_MERGE_MAX];
 };
 
+// bits folded by each pass of the reduction
+struct MsmFold {
+    int passes, bits[MSM_FOLD_PASSES];
+};
+
 // The reduction's last step: result = sum over windows w of
-// 2^(c w) (T_w + sum_k 2^(log_l + k) T_{w,k}).  One warp (one CTA) takes one
-// bit sum, doubles it by its whole weight on the x coordinate alone
+// 2^(c w) (sum_j B_{w,j} + sum_k 2^k T_{w,k}), `per` points a window.  One warp
+// (one CTA) takes one of them, doubles it by its whole weight on the x coordinate alone
 // (sl_dbl_many: the chain of a bit sum of the top window is as long as the
 // window doublings it replaces, but all of them run at once on their own SMs)
 // and the points are then added up pairwise: of two siblings the CTA that
 // arrives second adds the other's point and goes on, so no CTA waits for
 // another.  The last one of a group converts to the affine image.
 // Node i of a level stands at leaf i << level; a pair's counter is its right
-// child's leaf index.  Counters start at zero (k_msm_segments).
+// child's leaf index.  Counters start at zero (k_msm_fold).
 // The chain is bound by product latency, two per doubling.  Measured at
 // c = 16, 8 windows: Horner over bit sums per window, then the window
 // doublings with one warp per window on one SM, 567 us; this kernel 290 us.
-__global__ void __launch_bounds__(32) k_msm_tail(G1Xyzz* bits, int nbits, int c, int log_l, uint32_t leaves,
+__global__ void __launch_bounds__(32) k_msm_tail(G1Xyzz* sums, uint32_t per, MsmFold f, int c, uint32_t leaves,
                                                  uint32_t* ctr, const __grid_constant__ MsmOuts outs)
 {
     __shared__ Fq sl[20];
     const int lane = (int)threadIdx.x;
     const uint32_t group = blockIdx.x / leaves;
     uint32_t i = blockIdx.x % leaves;
-    G1Xyzz* pts = bits + (uint64_t)group * leaves;
+    G1Xyzz* pts = sums + (uint64_t)group * leaves;
     uint32_t* gctr = ctr + (uint64_t)group * leaves;
-    const int w = (int)(i / (uint32_t)(nbits + 1)), k = (int)(i % (uint32_t)(nbits + 1));
+    // leaf (w, a): the window's total (a = 0) or a bit sum; a pass appends its bits from the highest down
+    int dbl = c * (int)(i / per), a = (int)(i % per), base = 0;
+    for (int k = 0; k < f.passes && a > 0; k++) {
+        if (a <= f.bits[k]) dbl += base + f.bits[k] - a;
+        a -= f.bits[k];
+        base += f.bits[k];
+    }
     // the four coordinates of a point are consecutive: lane j < 4 moves coordinate j
     if (lane < 4) st(&sl[lane], ld(&pts[i].X + lane));
     __syncwarp();
-    if (!sl_get(sl, 2).is_zero()) sl_dbl_many(sl, c * w + (k < nbits ? log_l + k : 0));
+    if (!sl_get(sl, 2).is_zero()) sl_dbl_many(sl, dbl);
     uint32_t cnt = leaves;
     for (int level = 0; cnt > 1; level++) {
         const uint32_t sib = i ^ 1u;
@@ -1043,29 +846,58 @@ __global__ void k_write_inf(G1Jac* out)
     }
 }
 
-// Per-bit sums of the segment sums (reduction step 2), in BP parts per sum
-// when the segments are many.
-static RustError msm_bitsums(const MsmPlan& p, const MsmScratch& s, cudaStream_t st)
+// The first reduction pass takes 64 KB of shared memory (opt-in above 48 KB;
+// the attribute is the device's, so it is set on every call).
+static cudaError_t fold_smem_ready()
 {
-    const uint32_t nbs = (uint32_t)p.Wr * (uint32_t)(p.NBITS + 1);
-    k_msm_bitsums<<<nbs * p.BP, 256, 0, st>>>(s.segacc, s.segrun, p.S, p.NBITS, p.BP, p.BP > 1 ? s.bitparts : s.bits);
-    H2B_LAUNCHED("k_msm_bitsums");
-    if (p.BP > 1) {
-        k_msm_bitparts<<<nbs, 256, 0, st>>>(s.bitparts, p.BP, s.bits);
-        H2B_LAUNCHED("k_msm_bitparts");
+    return cudaFuncSetAttribute(k_msm_fold, cudaFuncAttributeMaxDynamicSharedMemorySize, 512 * (int)sizeof(G1Xyzz));
+}
+
+// Steps 5 to 7 from the accumulated buckets: chunk heads, bucket reduction, and
+// the results, one per group of `group_windows` reduction windows.
+static RustError msm_reduce(const MsmPlan& p, const MsmScratch& s, int group_windows, int c, const MsmOuts& outs,
+                            cudaStream_t st)
+{
+    const unsigned sm_cap = 148u * 16u;
+    const unsigned fix_grid = grid_for(p.NB * p.fix_lanes, 128, sm_cap);
+    switch (p.fix_lanes) {
+#define FIX(G)                                                                                                        \
+    case G:                                                                                                           \
+        k_msm_fixup<G><<<fix_grid, 128, 0, st>>>(s.offsets, p.NB, p.chunk, s.buckets, s.heads, p.fix_limit, s.dense,  \
+                                                 p.max_dense, s.items, p.max_items);                                  \
+        break;
+        FIX(1) FIX(2) FIX(4) FIX(8) FIX(16) FIX(32)
+#undef FIX
     }
+    H2B_LAUNCHED("k_msm_fixup");
+    k_msm_heads<<<148 * 8, 128, 0, st>>>(s.offsets, p.NB, p.chunk, s.buckets, s.heads, s.dense, p.max_dense, s.items);
+    H2B_LAUNCHED("k_msm_heads");
+    k_msm_heads_merge<<<148 * 4, 256, 0, st>>>(s.offsets, p.NB, p.chunk, s.buckets, s.heads, s.dense, p.max_dense);
+    H2B_LAUNCHED("k_msm_heads_merge");
+    const G1Xyzz* in = s.buckets;
+    uint32_t arrays = 1, len = p.H;
+    MsmFold f;
+    f.passes = p.passes;
+    for (int k = 0; k < p.passes; k++) {
+        const int m = p.fold[k];
+        f.bits[k] = m;
+        const uint32_t tasks = std::max(arrays << (m - 1), arrays + (uint32_t)m);
+        const size_t smem = sizeof(G1Xyzz) * ((size_t)(arrays + 1) << (m - 1));
+        H2B_CUDA(fold_smem_ready());
+        k_msm_fold<<<(unsigned)p.Wr * (len >> m), (tasks + 31) / 32 * 32, smem, st>>>(
+            in, arrays, len, m, s.fold[k & 1], s.tailctr, k == 0 ? (uint32_t)p.leaves : 0u);
+        H2B_LAUNCHED("k_msm_fold");
+        in = s.fold[k & 1];
+        arrays += (uint32_t)m;
+        len >>= m;
+    }
+    k_msm_tail<<<(unsigned)p.leaves, 32, 0, st>>>(s.fold[(p.passes - 1) & 1], (uint32_t)p.c, f, c,
+                                                  (uint32_t)group_windows * (uint32_t)p.c, s.tailctr, outs);
+    H2B_LAUNCHED("k_msm_tail");
     return ok();
 }
 
 // Runs steps 1-7 on device buffers; result (96 bytes) lands in s.result.
-// The lazy accumulation (window tables are stored in its form; plain bases
-// are converted by the split kernel) unless pairing rounds or an older
-// variant run.
-static bool msm_lazy(const MsmPlan& p)
-{
-    return p.R == 0 && (p.tn > 0 || g_msm_acc_variant == 0 || g_msm_acc_variant >= 6);
-}
-
 // Phases of one MSM on `st`: msm_begin clears the histogram, msm_split takes
 // points [lo, hi) through the GLV split (and base conversion) and the
 // histogram -- callers may feed the points in pieces as they arrive --, and
@@ -1074,7 +906,7 @@ static RustError msm_begin(const MsmPlan& p, const MsmScratch& s, cudaStream_t s
 {
     prof_begin(PROF_MSM_TOTAL, st);
     H2B_CUDA(cudaMemsetAsync(s.counts, 0, p.NB * sizeof(uint32_t), st));
-    H2B_CUDA(cudaMemsetAsync(s.dense + p.max_dense, 0, sizeof(uint32_t), st));
+    H2B_CUDA(cudaMemsetAsync(s.dense + p.max_dense, 0, 2 * sizeof(uint32_t), st));
     return ok();
 }
 
@@ -1085,96 +917,41 @@ static RustError msm_split(const MsmPlan& p, const MsmScratch& s, const Fr* d_sc
     const unsigned sm_cap = 148u * 16u;
     uint4* vsc = reinterpret_cast<uint4*>(s.canon);  // 2n x 16 B in the n x 32 B slot
     k_msm_glv_hist<<<grid_for(hi - lo, 256, sm_cap), 256, 0, st>>>(
-        d_scalars, vsc, lo, hi, d_bases, msm_lazy(p) && p.tn == 0 ? s.rbases : nullptr, p.n, p.c, p.W, p.H, s.counts,
+        d_scalars, vsc, lo, hi, d_bases, p.tn == 0 ? s.rbases : nullptr, p.n, p.c, p.W, p.H, s.counts,
         p.tn);
     H2B_LAUNCHED("k_msm_glv_hist");
     return ok();
+}
+
+// The bucket accumulation over points in the x 2^261 form.
+static void msm_accumulate(const MsmPlan& p, const MsmScratch& s, const G1Affine* pts, cudaStream_t st)
+{
+    const uint64_t phi = p.tn ? (uint64_t)p.W * p.tn : p.n;
+    const unsigned grid = grid_for(p.max_chunks, 128, 148u * 32u);
+    if (g_msm_acc_variant == 6)
+        k_msm_accumulate_e<<<grid, 128, 0, st>>>(s.sorted, s.offsets, p.NB, p.chunk, pts, phi, s.buckets, s.heads,
+                                                 g_msm_prefetch);
+    else
+        k_msm_accumulate_z<<<grid, 128, 0, st>>>(s.sorted, s.offsets, p.NB, p.chunk, pts, phi, s.buckets, s.heads);
 }
 
 static RustError msm_finish(const MsmPlan& p, const MsmScratch& s, const G1Affine* d_bases, cudaStream_t st)
 {
     const unsigned sm_cap = 148u * 16u;
     const uint4* vsc = reinterpret_cast<const uint4*>(s.canon);
-    const bool lazy = msm_lazy(p);
     H2B_CUDA(scan_u32(s.counts, p.NB, s.offsets, s.scan_tmp, st));
     H2B_CUDA(cudaMemcpyAsync(s.cursor, s.offsets, p.NB * sizeof(uint32_t), cudaMemcpyDeviceToDevice, st));
     k_msm_sort<true><<<grid_for(p.nv, 256, sm_cap), 256, 0, st>>>(vsc, 0, p.nv, p.c, p.W, p.H, s.cursor,
                                                                     s.sorted, p.tn, 0u);
     H2B_LAUNCHED("k_msm_sort<scatter>");
     prof_begin(PROF_MSM_ACCUMULATE, st);
-    // pairing rounds: sorted entries -> pts[0] -> pts[1] -> pts[0]
-    const uint32_t* off = s.offsets;
-#if H2B_EXPERIMENTS
-    const G1Affine* src = d_bases;
-    for (int r = 1; r <= p.R; r++) {
-        k_msm_half_counts<<<grid_for(p.NB, 256, sm_cap), 256, 0, st>>>(off, p.NB, s.counts);
-        H2B_LAUNCHED("k_msm_half_counts");
-        H2B_CUDA(scan_u32(s.counts, p.NB, s.roff[r - 1], s.scan_tmp, st));
-        G1Affine* dst = s.pts[(r - 1) & 1];
-        const uint64_t ctas = pr_ctas(p.cap[r - 1]);
-        const uint32_t* srt = r == 1 ? s.sorted : nullptr;
-        if (r == 1)
-            k_msm_pair_fwd<true><<<(unsigned)ctas, PR_T, 0, st>>>(srt, src, off, p.NB, s.roff[0], dst, s.pr_pref,
-                                                                  s.pr_job, s.pr_nj, s.pr_tree, s.pr_tot);
-        else
-            k_msm_pair_fwd<false><<<(unsigned)ctas, PR_T, 0, st>>>(srt, src, off, p.NB, s.roff[r - 1], dst,
-                                                                   s.pr_pref, s.pr_job, s.pr_nj, s.pr_tree, s.pr_tot);
-        H2B_LAUNCHED("k_msm_pair_fwd");
-        H2B_TRY(fq_batch_invert(s.pr_tot, ctas, s.pr_inv_scratch, s.pr_inv_bytes, st));
-        if (r == 1)
-            k_msm_pair_bwd<true><<<(unsigned)ctas, PR_T, 0, st>>>(srt, src, off, p.NB, dst, s.pr_pref, s.pr_job,
-                                                                  s.pr_nj, s.pr_tree, s.pr_tot);
-        else
-            k_msm_pair_bwd<false><<<(unsigned)ctas, PR_T, 0, st>>>(srt, src, off, p.NB, dst, s.pr_pref, s.pr_job,
-                                                                   s.pr_nj, s.pr_tree, s.pr_tot);
-        H2B_LAUNCHED("k_msm_pair_bwd");
-        off = s.roff[r - 1];
-        src = dst;
-    }
-#endif
-    const uint64_t chunks = (p.cap[p.R] + p.Kf - 1) / p.Kf;
-    const unsigned acc_grid = grid_for(chunks, 128, 148u * 32u);
-    if (lazy && g_msm_acc_variant == 6)
-        k_msm_accumulate_e<<<acc_grid, 128, 0, st>>>(s.sorted, off, p.NB, p.Kf, p.tn ? d_bases : s.rbases,
-                                                     p.tn ? (uint64_t)p.W * p.tn : p.n, s.buckets, s.heads,
-                                                     g_msm_prefetch);
-    else if (lazy)
-        k_msm_accumulate_z<<<acc_grid, 128, 0, st>>>(s.sorted, off, p.NB, p.Kf, p.tn ? d_bases : s.rbases,
-                                                     p.tn ? (uint64_t)p.W * p.tn : p.n, s.buckets, s.heads);
-#if H2B_EXPERIMENTS
-    else if (p.R > 0)
-        k_msm_accumulate<2, true><<<acc_grid, 128, 0, st>>>(nullptr, off, p.NB, p.Kf, src, s.buckets, s.heads);
-    else if (g_msm_acc_variant == 5)
-        k_msm_accumulate<0, false><<<acc_grid, 128, 0, st>>>(s.sorted, off, p.NB, p.Kf, src, s.buckets, s.heads);
-    else if (g_msm_acc_variant == 1)
-        k_msm_accumulate<1, false><<<acc_grid, 128, 0, st>>>(s.sorted, off, p.NB, p.Kf, src, s.buckets, s.heads);
-    else if (g_msm_acc_variant == 2)
-        k_msm_accumulate<2, false><<<acc_grid, 128, 0, st>>>(s.sorted, off, p.NB, p.Kf, src, s.buckets, s.heads);
-    else if (g_msm_acc_variant == 3)
-        k_msm_accumulate<3, false><<<acc_grid, 128, 0, st>>>(s.sorted, off, p.NB, p.Kf, src, s.buckets, s.heads);
-    else if (g_msm_acc_variant == 4)
-        k_msm_accumulate<4, false><<<acc_grid, 128, 0, st>>>(s.sorted, off, p.NB, p.Kf, src, s.buckets, s.heads);
-#endif
+    msm_accumulate(p, s, p.tn ? d_bases : s.rbases, st);
     prof_end(PROF_MSM_ACCUMULATE, st);
     H2B_LAUNCHED("k_msm_accumulate");
-    k_msm_fixup<<<grid_for(p.NB, 128, sm_cap), 128, 0, st>>>(off, p.NB, p.Kf, s.buckets, s.heads, s.dense,
-                                                            p.max_dense);
-    H2B_LAUNCHED("k_msm_fixup");
-    k_msm_dense_pieces<<<148 * 4, 256, 0, st>>>(off, p.max_dense, p.Kf, s.heads, s.dense, s.pieces);
-    H2B_LAUNCHED("k_msm_dense_pieces");
-    k_msm_dense_merge<<<148, DENSE_PIECES, 0, st>>>(p.max_dense, s.buckets, s.dense, s.pieces);
-    H2B_LAUNCHED("k_msm_dense_merge");
-    uint64_t nseg = (uint64_t)p.Wr * p.S;
-    k_msm_segments<<<grid_for(nseg, 128, sm_cap), 128, 0, st>>>(s.buckets, p.Wr, p.H, p.L, p.S, s.segacc, s.segrun,
-                                                                s.tailctr, (uint32_t)p.Wr * (uint32_t)(p.NBITS + 1));
-    H2B_LAUNCHED("k_msm_segments");
-    H2B_TRY(msm_bitsums(p, s, st));
     MsmOuts o;
     o.p[0] = s.result;
-    const uint32_t leaves = (uint32_t)p.Wr * (uint32_t)(p.NBITS + 1);
-    k_msm_tail<<<leaves, 32, 0, st>>>(s.bits, p.NBITS, p.c, p.LOGL, leaves, s.tailctr, o);
+    H2B_TRY(msm_reduce(p, s, p.Wr, p.c, o, st));
     prof_end(PROF_MSM_TOTAL, st);
-    H2B_LAUNCHED("k_msm_tail");
     return ok();
 }
 
@@ -1200,7 +977,7 @@ RustError msm_run_merged(const MsmPlan& p, const MsmScratch& s, uint32_t J, cons
     uint4* vsc = reinterpret_cast<uint4*>(s.canon);
     prof_begin(PROF_MSM_TOTAL, st);
     H2B_CUDA(cudaMemsetAsync(s.counts, 0, p.NB * sizeof(uint32_t), st));
-    H2B_CUDA(cudaMemsetAsync(s.dense + p.max_dense, 0, sizeof(uint32_t), st));
+    H2B_CUDA(cudaMemsetAsync(s.dense + p.max_dense, 0, 2 * sizeof(uint32_t), st));
     uint64_t at = 0;   // job j's virtual scalars start at vsc + 2 * at
     for (uint32_t j = 0; j < J; j++) {
         if (ns[j] == 0) continue;
@@ -1223,34 +1000,13 @@ RustError msm_run_merged(const MsmPlan& p, const MsmScratch& s, uint32_t J, cons
         at += ns[j];
     }
     prof_begin(PROF_MSM_ACCUMULATE, st);
-    const uint64_t chunks = (p.max_entries + p.Kf - 1) / p.Kf;
-    const unsigned acc_grid = grid_for(chunks, 128, 148u * 32u);
-    if (g_msm_acc_variant == 6)
-        k_msm_accumulate_e<<<acc_grid, 128, 0, st>>>(s.sorted, s.offsets, p.NB, p.Kf, table, (uint64_t)p.W * p.tn,
-                                                     s.buckets, s.heads, g_msm_prefetch);
-    else
-        k_msm_accumulate_z<<<acc_grid, 128, 0, st>>>(s.sorted, s.offsets, p.NB, p.Kf, table, (uint64_t)p.W * p.tn,
-                                                     s.buckets, s.heads);
+    msm_accumulate(p, s, table, st);
     prof_end(PROF_MSM_ACCUMULATE, st);
     H2B_LAUNCHED("k_msm_accumulate");
-    k_msm_fixup<<<grid_for(p.NB, 128, sm_cap), 128, 0, st>>>(s.offsets, p.NB, p.Kf, s.buckets, s.heads, s.dense,
-                                                            p.max_dense);
-    H2B_LAUNCHED("k_msm_fixup");
-    k_msm_dense_pieces<<<148 * 4, 256, 0, st>>>(s.offsets, p.max_dense, p.Kf, s.heads, s.dense, s.pieces);
-    H2B_LAUNCHED("k_msm_dense_pieces");
-    k_msm_dense_merge<<<148, DENSE_PIECES, 0, st>>>(p.max_dense, s.buckets, s.dense, s.pieces);
-    H2B_LAUNCHED("k_msm_dense_merge");
-    const uint64_t nseg = (uint64_t)p.Wr * p.S;
-    k_msm_segments<<<grid_for(nseg, 128, sm_cap), 128, 0, st>>>(s.buckets, p.Wr, p.H, p.L, p.S, s.segacc, s.segrun,
-                                                                s.tailctr, (uint32_t)p.Wr * (uint32_t)(p.NBITS + 1));
-    H2B_LAUNCHED("k_msm_segments");
-    H2B_TRY(msm_bitsums(p, s, st));
     MsmOuts o;
     for (uint32_t j = 0; j < J; j++) o.p[j] = outs[j];
-    const uint32_t leaves = (uint32_t)(p.NBITS + 1);
-    k_msm_tail<<<J * leaves, 32, 0, st>>>(s.bits, p.NBITS, 0, p.LOGL, leaves, s.tailctr, o);
+    H2B_TRY(msm_reduce(p, s, 1, 0, o, st));
     prof_end(PROF_MSM_TOTAL, st);
-    H2B_LAUNCHED("k_msm_tail");
     return ok();
 }
 
@@ -1509,26 +1265,20 @@ extern "C" RustError h2b_msm_device_table(const void* d_scalars, const void* d_t
 
 extern "C" void h2b_msm_set_tuning(int window_bits, int chunk) { msm_set_tuning(window_bits, chunk); }
 
-// Form and call structure of the bucket-accumulation kernel: 6 = the lazy
-// R' = 2^260 form on the FP64 pipe (default; window tables use it too);
-// 0 = the lazy R = 2^261 form of 29-bit limbs with one-step carries on the
-// integer multiply pipe (window tables use it for every choice but 6).
-// Built with H2B_EXPERIMENTS=1 only, the normalised R = 2^256 limb form with
-// 5 = two products per out-of-line call, 1 = all products inline, 2 = one
-// product per call, 3 and 4 = one product per call with at most 128 / 96
-// registers, and 7 = the FP64 lazy form with two accumulation chains per
-// thread (25.7 ms at 2^22).  Measured at 2^22 with the witness-like scalar mix: 6 takes
-// 12.26 ms, 0 13.56 ms.  Results are identical; only speed differs.  A value
-// that is not built leaves the setting unchanged (read it back with
+// Form of the bucket-accumulation kernel: 6 = coordinates in [0, 2p) on the
+// even/odd product (default), 0 = the lazy R = 2^261 form of 29-bit limbs with
+// one-step carries.  Measured at 2^22 with the witness-like scalar mix, the
+// whole MSM: 6 8.07 ms, 0 13.6 ms.  Results are identical; only speed differs.
+// Any other value leaves the setting unchanged (read it back with
 // h2b_msm_get_accumulate_variant).
 extern "C" void h2b_msm_set_accumulate_variant(int v)
 {
-    if (v == 0 || v == 6 || (H2B_EXPERIMENTS && v >= 1 && v <= 7)) g_msm_acc_variant = v;
+    if (v == 0 || v == 6) g_msm_acc_variant = v;
 }
 
 extern "C" int h2b_msm_get_accumulate_variant(void) { return g_msm_acc_variant; }
 
-// Distance (sorted entries ahead, 0..64) at which the FP64 accumulation
+// Distance (sorted entries ahead, 0..64) at which the accumulation
 // prefetches the next points into L2; 0 turns it off.  Same results.
 extern "C" void h2b_msm_set_prefetch(int distance)
 {
@@ -1536,16 +1286,10 @@ extern "C" void h2b_msm_set_prefetch(int distance)
 }
 extern "C" int h2b_msm_get_prefetch(void) { return (int)g_msm_prefetch; }
 
-extern "C" int h2b_msm_get_pair_rounds(void) { return g_msm_pair_rounds; }
-
-// Batch-affine pairing rounds run before the XYZZ bucket accumulation
-// (0..3; rounds above 0 are built with H2B_EXPERIMENTS=1 only, otherwise
-// the setting stays 0).  Default 0: on B200 a pairing addition (forward pass, shared
-// inversion, backward pass) measured about 0.5 ns per addition against
-// 0.3 ns for an XYZZ mixed addition (2^20 points, witness scalar mix).
-// Results are identical; speed and the workspace size differ (the
-// workspace-size queries follow this setting).
-extern "C" void h2b_msm_set_pair_rounds(int rounds) { msm_set_pair_rounds(rounds); }
+// Batch-affine pairing rounds before the XYZZ accumulation are not built (0.5 ns
+// per addition against 0.15 ns for an XYZZ mixed addition): the setting stays 0.
+extern "C" int h2b_msm_get_pair_rounds(void) { return 0; }
+extern "C" void h2b_msm_set_pair_rounds(int) {}
 
 // Number of nonzero signed window digits (= sorted entries = bucket
 // additions) the MSM of these scalars performs; written to *d_count (u64).

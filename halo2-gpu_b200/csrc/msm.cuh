@@ -7,27 +7,33 @@
 
 namespace h2b {
 
+// Entries per accumulation chunk: `fixed` if set, else the fewest whole waves
+// of `threads` chunks of at most `cap` entries, evened out.
+struct MsmChunk {
+    uint32_t fixed, threads, cap;
+};
+
+constexpr int MSM_FOLD_PASSES = 6;
+
 struct MsmPlan {
     uint64_t n;
     int c;           // window bits
     int W;           // windows
     uint32_t H;      // buckets per window = 2^(c-1)
-    uint64_t NB;     // W * H
-    uint32_t K;      // sorted entries per accumulation chunk
+    uint64_t NB;     // Wr * H
     uint64_t nv;     // virtual (GLV half) scalars = 2n
     uint64_t max_entries;
+    MsmChunk chunk;
     uint64_t max_chunks;
-    uint32_t L;      // buckets per reduction segment
-    int LOGL;        // log2(L)
-    uint32_t S;      // segments per window
-    int NBITS;       // log2(S)
-    uint64_t max_dense;  // capacity of the dense-bucket list
-    int R;               // pairing rounds before the XYZZ accumulation
-    uint64_t cap[4];     // entry capacity after round r (cap[0] = max_entries)
-    uint32_t Kf;         // entries per XYZZ accumulation chunk after the rounds
-    uint64_t tn;         // points per window slice of a precomputed table (0: plain bases)
-    int Wr;              // windows in the bucket reduction (W, or 1 with a table)
-    uint32_t BP;         // CTAs per bit sum of the reduction (partials summed by a second kernel when > 1)
+    uint32_t fix_lanes;  // lanes that sum a bucket's chunk heads
+    uint32_t fix_limit;  // heads beyond which a bucket is listed instead
+    uint64_t max_dense;  // capacity of that list
+    uint64_t max_items;  // and of the list of its pieces
+    int passes;      // passes of the bucket reduction
+    int fold[MSM_FOLD_PASSES];  // index bits that each folds
+    uint64_t leaves; // Wr c: the points the last step doubles and adds up
+    uint64_t tn;     // points per window slice of a precomputed table (0: plain bases)
+    int Wr;          // windows in the bucket reduction (W; with a table 1, or one per merged job)
 };
 
 struct MsmScratch {
@@ -42,23 +48,11 @@ struct MsmScratch {
     G1Xyzz* buckets;
     G1Xyzz* heads;
     uint32_t* dense;
-    G1Xyzz* pieces;
-    G1Xyzz* segacc;
-    G1Xyzz* segrun;
-    G1Xyzz* bits;
-    G1Xyzz* bitparts;    // per-part bit sums (BP > 1)
+    uint2* items;
+    G1Xyzz* fold[2];     // outputs of the reduction passes, alternating
     uint32_t* tailctr;   // arrival counters of the last reduction step
     G1Jac* result;
-    G1Affine* rbases;    // plain bases P_i, then phi(P_i), in the lazy x 2^261 form (no pairing rounds)
-    G1Affine* pts[2];    // pairing-round outputs (ping-pong)
-    uint32_t* roff[3];   // per-round bucket offsets (NB + 1 each)
-    Fq* pr_pref;         // pairing rounds: per-job denominator prefixes
-    uint2* pr_job;       // pairing rounds: per-job (input entry, output slot)
-    uint32_t* pr_nj;     // pairing rounds: jobs per thread
-    Fq* pr_tree;         // pairing rounds: per-CTA product trees
-    Fq* pr_tot;          // pairing rounds: per-CTA totals (inverted in place)
-    void* pr_inv_scratch;
-    uint64_t pr_inv_bytes;
+    G1Affine* rbases;    // plain bases P_i, then phi(P_i), in the x 2^261 form
 };
 
 // Plan for an MSM that runs beside `concurrent` - 1 others (batches): same
@@ -80,6 +74,5 @@ MsmPlan msm_plan_merged(uint64_t n_total, uint64_t tn, uint32_t J);
 RustError msm_run_merged(const MsmPlan& p, const MsmScratch& s, uint32_t J, const Fr* const* scalars,
                          const uint64_t* ns, const G1Affine* table, G1Jac* const* outs, cudaStream_t st);
 void msm_set_tuning(int window_bits, int chunk);
-void msm_set_pair_rounds(int rounds);
 
 } // namespace h2b
