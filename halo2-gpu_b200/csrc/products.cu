@@ -34,45 +34,60 @@ namespace h2b {
 constexpr int BI_T = 256;
 constexpr int BI_E = 8;
 constexpr int BI_TILE = BI_T * BI_E;  // elements per CTA
-constexpr size_t BI_SMEM = (size_t)(BI_E - 1) * BI_T * 32 + (size_t)2 * BI_T * 32;
+constexpr size_t BI_SMEM = (size_t)(BI_E + 1) * BI_T * 32;
+// Tiles of the product kernels (lookup, permutation, and the finish of the
+// host-staged form): 128 threads of 8 elements, one inversion per tile.  The
+// inversion is as many instructions as 80 products of a warp, so tiles must not
+// be short, and CTAs must be small and many, so that others work while one
+// inverts: 2^20 rows, all arguments of a proof, 1.33 ms; 1.41 ms at 256 x 8,
+// 1.47 ms at 128 x 4, 1.50 ms at 128 x 16.  Below 2^17 rows the GPU is not full
+// and the serial rows of a thread are what counts: two per thread (2^16 rows
+// 502 -> 427 us, 2^12 470 -> 373 us; at 2^18 it would be 595 -> 668 us).
+constexpr int PR_T = 128, PR_LOG_T = 7, PR_E = 8, PR_E_SMALL = 2;
+constexpr uint64_t PR_SMALL = 1ull << 17;
+constexpr size_t pr_smem(int E) { return (size_t)(E + 1) * PR_T * 32; }
 
-// Block Montgomery trick.  Thread t owns tile elements j*BI_T + t (j < BI_E).
+// Block Montgomery trick.  Thread t owns tile elements j*T + t (j < E).
 //   fwd(i)   -> x_i (may stash x_i for bwd); zero is treated as one
 //   bwdx(i)  -> x_i again
 //   emit(i, inv_or_zero)
-// The CTA's total inverse comes from *root_inv when non-null, else it is
-// computed here by thread 0.
-template <class C, class Fwd, class Bwdx, class Emit>
+// The CTA's total inverse comes from *root_inv when non-null; else the product
+// tree stops at 32 nodes and one warp inverts them side by side (the same
+// latency as one inversion, ten tree levels fewer on the way up and down).
+//   side()   -> run by the second warp while the first one inverts
+template <int T, int E, class C, class Fwd, class Bwdx, class Emit, class Side>
 __device__ __forceinline__ void block_mont_trick(uint64_t base, uint64_t n, const Fp<C>* root_inv, Fwd fwd, Bwdx bwdx,
-                                                 Emit emit)
+                                                 Emit emit, Side side)
 {
     using F = Fp<C>;
     extern __shared__ uint4 bi_smem[];
     F* pre = reinterpret_cast<F*>(bi_smem);           // (E-1) x T prefixes
-    F* tree = pre + (BI_E - 1) * BI_T;                 // 2T heap: tree[T + t] = thread total
+    F* tree = pre + (E - 1) * T;                       // 2T heap: tree[T + t] = thread total
     const int t = threadIdx.x;
 
     F acc = F::one();
 #pragma unroll 1
-    for (int j = 0; j < BI_E; j++) {
-        uint64_t i = base + (uint64_t)j * BI_T + t;
+    for (int j = 0; j < E; j++) {
+        uint64_t i = base + (uint64_t)j * T + t;
         F x = F::one();
         if (i < n) {
             x = fwd(i);
             if (x.is_zero()) x = F::one();
         }
         acc = (j == 0) ? x : acc * x;
-        if (j < BI_E - 1) pre[j * BI_T + t] = acc;
+        if (j < E - 1) pre[j * T + t] = acc;
     }
-    tree[BI_T + t] = acc;
+    tree[T + t] = acc;
     __syncthreads();
-    for (int w = BI_T / 2; w >= 1; w >>= 1) {
+    const int top = root_inv ? 1 : 32;
+    for (int w = T / 2; w >= top; w >>= 1) {
         if (t < w) tree[w + t] = tree[2 * (w + t)] * tree[2 * (w + t) + 1];
         __syncthreads();
     }
-    if (t == 0) tree[1] = root_inv ? *root_inv : finv_fast<C>(tree[1]);
+    if (t < top) tree[top + t] = root_inv ? *root_inv : finv_fast<C>(tree[top + t]);
+    if (t >= 32 && t < 64) side();
     __syncthreads();
-    for (int w = 1; w < BI_T; w <<= 1) {
+    for (int w = top; w < T; w <<= 1) {
         if (t < w) {
             int k = w + t;
             F inv = tree[k];
@@ -84,28 +99,28 @@ __device__ __forceinline__ void block_mont_trick(uint64_t base, uint64_t n, cons
     }
     // Backward: x_j^-1 = inv(prefix_j) * prefix_{j-1}; results replace the
     // consumed prefix slots, then are emitted in ascending j.
-    F inv = tree[BI_T + t];
+    F inv = tree[T + t];
     F inv0 = F::zero();
 #pragma unroll 1
-    for (int j = BI_E - 1; j >= 0; j--) {
-        uint64_t i = base + (uint64_t)j * BI_T + t;
+    for (int j = E - 1; j >= 0; j--) {
+        uint64_t i = base + (uint64_t)j * T + t;
         if (i >= n) continue;
         F x = bwdx(i);
         F out;
         if (x.is_zero()) {
             out = x;
         } else {
-            out = (j > 0) ? inv * pre[(j - 1) * BI_T + t] : inv;
+            out = (j > 0) ? inv * pre[(j - 1) * T + t] : inv;
             inv = inv * x;
         }
-        if (j > 0) pre[(j - 1) * BI_T + t] = out;
+        if (j > 0) pre[(j - 1) * T + t] = out;
         else inv0 = out;
     }
 #pragma unroll 1
-    for (int j = 0; j < BI_E; j++) {
-        uint64_t i = base + (uint64_t)j * BI_T + t;
+    for (int j = 0; j < E; j++) {
+        uint64_t i = base + (uint64_t)j * T + t;
         if (i >= n) break;
-        emit(i, j == 0 ? inv0 : pre[(j - 1) * BI_T + t], j);
+        emit(i, j == 0 ? inv0 : pre[(j - 1) * T + t], j);
     }
 }
 
@@ -115,9 +130,9 @@ __global__ void __launch_bounds__(BI_T) k_batch_invert(Fp<C>* __restrict__ d, ui
 {
     using F = Fp<C>;
     uint64_t base = (uint64_t)blockIdx.x * BI_TILE;
-    block_mont_trick<C>(
+    block_mont_trick<BI_T, BI_E, C>(
         base, n, root_inv ? root_inv + blockIdx.x : nullptr, [&](uint64_t i) { return ld(&d[i]); },
-        [&](uint64_t i) { return ld(&d[i]); }, [&](uint64_t i, const F& v, int) { st(&d[i], v); });
+        [&](uint64_t i) { return ld(&d[i]); }, [&](uint64_t i, const F& v, int) { st(&d[i], v); }, [] {});
 }
 
 // Per-CTA product of the (zero-as-one) tile, written to totals[blockIdx.x].
@@ -162,6 +177,7 @@ static RustError batch_invert_local(Fp<C>* d, uint64_t n, cudaStream_t st)
     return ok();
 }
 
+static unsigned pr_tiles(uint64_t n, int E) { return (unsigned)((n + PR_T * E - 1) / (uint64_t)(PR_T * E)); }
 static uint64_t tiles_of(uint64_t n) { return (n + BI_TILE - 1) / BI_TILE; }
 
 static void plan_batch_invert(ScratchPlan& p, uint64_t n)
@@ -394,14 +410,15 @@ static RustError grand_product_inplace(Fr* d, uint64_t n, const Fr* d_prefix, cu
 // lookup product: (A+b)(S+g) / ((A'+b)(S'+g))
 // ---------------------------------------------------------------------------
 
-__global__ void __launch_bounds__(BI_T) k_lookup_product(Fr* __restrict__ out, const Fr* __restrict__ pa,
+template <int E>
+__global__ void __launch_bounds__(PR_T) k_lookup_product(Fr* __restrict__ out, const Fr* __restrict__ pa,
                                                          const Fr* __restrict__ ps, const Fr* __restrict__ ca,
                                                          const Fr* __restrict__ cs, const Fr* __restrict__ pbeta,
                                                          const Fr* __restrict__ pgamma, uint64_t n)
 {
     const Fr beta = ld(pbeta), gamma = ld(pgamma);
-    uint64_t base = (uint64_t)blockIdx.x * BI_TILE;
-    block_mont_trick<FrCfg>(
+    uint64_t base = (uint64_t)blockIdx.x * (PR_T * E);
+    block_mont_trick<PR_T, E, FrCfg>(
         base, n, nullptr,
         [&](uint64_t i) {
             Fr x = (ld(&pa[i]) + beta) * (ld(&ps[i]) + gamma);
@@ -412,7 +429,8 @@ __global__ void __launch_bounds__(BI_T) k_lookup_product(Fr* __restrict__ out, c
         [&](uint64_t i, const Fr& inv, int) {
             Fr v = inv.is_zero() ? inv : inv * (ld(&ca[i]) + beta) * (ld(&cs[i]) + gamma);
             st(&out[i], v);
-        });
+        },
+        [] {});
 }
 
 // ---------------------------------------------------------------------------
@@ -438,17 +456,20 @@ __device__ __forceinline__ Fr pow_u64(const Fr& w, uint64_t e)
 
 // Fused device path: acc_i *= prod_c (b*sigma_c + g + v_c), invert, times
 // prod_c (dw0*delta^c*w^i*b + g + v_c).
-__global__ void __launch_bounds__(BI_T) k_permutation_product(Fr* __restrict__ acc, PermCols cols, int ncols,
+template <int E>
+__global__ void __launch_bounds__(PR_T) k_permutation_product(Fr* __restrict__ acc, PermCols cols, int ncols,
                                                               const Fr* __restrict__ pbeta, const Fr* __restrict__ pgamma,
                                                               const Fr* __restrict__ pdelta, const Fr* __restrict__ pomega,
                                                               const Fr* __restrict__ pdeltaomega, uint64_t n)
 {
     const Fr beta = ld(pbeta), gamma = ld(pgamma), delta = ld(pdelta), omega = ld(pomega);
-    const Fr dw0b = ld(pdeltaomega) * beta;   // the numerator's first column term is dw0 w^i beta
-    const uint64_t base = (uint64_t)blockIdx.x * BI_TILE;
-    Fr wstep = pow_u64(omega, BI_T);   // emit steps i by BI_T
+    const uint64_t base = (uint64_t)blockIdx.x * (PR_T * E);
+    // w^(2^k) for k <= log2 T, then dw0 beta w^base: about 35 dependent
+    // products, by one lane of the warp that would idle during the inversion
+    // (every thread on its own took 30 products for its 8 rows)
+    __shared__ Fr pw[PR_LOG_T + 2];
     Fr wib = Fr::one();
-    block_mont_trick<FrCfg>(
+    block_mont_trick<PR_T, E, FrCfg>(
         base, n, nullptr,
         [&](uint64_t i) {
             Fr x = ld(&acc[i]);
@@ -461,7 +482,14 @@ __global__ void __launch_bounds__(BI_T) k_permutation_product(Fr* __restrict__ a
             // column c's term is dw0 w^i delta^c beta + gamma + v_c: the
             // beta-scaled power is stepped (one product per row) and then
             // by delta per column, so a row takes 2 ncols - 1 products here
-            wib = (j == 0) ? dw0b * pow_u64(omega, i) : wib * wstep;
+            if (j == 0) {
+                wib = pw[PR_LOG_T + 1];
+#pragma unroll 1
+                for (int k = 0; k < PR_LOG_T; k++)
+                    if ((threadIdx.x >> k) & 1) wib = wib * pw[k];
+            } else {
+                wib = wib * pw[PR_LOG_T];
+            }
             if (inv.is_zero()) { st(&acc[i], inv); return; }
             if (ncols == 0) { st(&acc[i], inv); return; }   // no columns: the numerator is 1
             Fr cur = wib;
@@ -471,6 +499,23 @@ __global__ void __launch_bounds__(BI_T) k_permutation_product(Fr* __restrict__ a
                 num = num * (cur + gamma + ld(&cols.value[c][i]));
             }
             st(&acc[i], inv * num);
+        },
+        [&] {
+            if (threadIdx.x != 32) return;
+            Fr p = omega, r = ld(pdeltaomega) * beta;   // the numerator's first column term is dw0 w^i beta
+            pw[0] = p;
+            uint64_t e = base >> PR_LOG_T;               // base is a multiple of T
+#pragma unroll 1
+            for (int k = 1; k <= PR_LOG_T; k++) {
+                p = p * p;
+                pw[k] = p;
+            }
+            while (e) {
+                if (e & 1) r = r * p;
+                e >>= 1;
+                if (e) p = p * p;
+            }
+            pw[PR_LOG_T + 1] = r;
         });
 }
 
@@ -499,13 +544,14 @@ __global__ void k_pp_accumulate(Fr* __restrict__ den, Fr* __restrict__ num, cons
     }
 }
 
-__global__ void __launch_bounds__(BI_T) k_pp_finish(Fr* __restrict__ den, const Fr* __restrict__ num, uint64_t n,
+template <int E>
+__global__ void __launch_bounds__(PR_T) k_pp_finish(Fr* __restrict__ den, const Fr* __restrict__ num, uint64_t n,
                                                     bool have_num)
 {
-    uint64_t base = (uint64_t)blockIdx.x * BI_TILE;
-    block_mont_trick<FrCfg>(
+    uint64_t base = (uint64_t)blockIdx.x * (PR_T * E);
+    block_mont_trick<PR_T, E, FrCfg>(
         base, n, nullptr, [&](uint64_t i) { return ld(&den[i]); }, [&](uint64_t i) { return ld(&den[i]); },
-        [&](uint64_t i, const Fr& inv, int) { st(&den[i], have_num ? inv * ld(&num[i]) : inv); });
+        [&](uint64_t i, const Fr& inv, int) { st(&den[i], have_num ? inv * ld(&num[i]) : inv); }, [] {});
 }
 
 __global__ void k_advance_deltaomega(Fr* __restrict__ dw, const Fr* __restrict__ pdelta, uint64_t batch)
@@ -702,8 +748,11 @@ static RustError lookup_product_run(Fr* out, const Fr* pa, const Fr* ps, const F
                                     const Fr* gamma, uint64_t n, cudaStream_t st)
 {
     if (n == 0) return ok();
-    enable_big_smem(k_lookup_product);
-    k_lookup_product<<<(unsigned)tiles_of(n), BI_T, BI_SMEM, st>>>(out, pa, ps, ca, cs, beta, gamma, n);
+    if (n < PR_SMALL) {
+        k_lookup_product<PR_E_SMALL><<<pr_tiles(n, PR_E_SMALL), PR_T, pr_smem(PR_E_SMALL), st>>>(out, pa, ps, ca, cs, beta, gamma, n);
+    } else {
+        k_lookup_product<PR_E><<<pr_tiles(n, PR_E), PR_T, pr_smem(PR_E), st>>>(out, pa, ps, ca, cs, beta, gamma, n);
+    }
     H2B_LAUNCHED("k_lookup_product");
     return ok();
 }
@@ -807,8 +856,11 @@ extern "C" RustError _halo2_permutation_product(const FFITraitObject* modified_v
         H2B_LAUNCHED("k_advance_deltaomega");
     }
     if (length > 0) {
-        enable_big_smem(k_pp_finish);
-        k_pp_finish<<<(unsigned)tiles_of(length), BI_T, BI_SMEM, stream>>>(den, num, length, batch > 0);
+        if (length < PR_SMALL) {
+            k_pp_finish<PR_E_SMALL><<<pr_tiles(length, PR_E_SMALL), PR_T, pr_smem(PR_E_SMALL), stream>>>(den, num, length, batch > 0);
+        } else {
+            k_pp_finish<PR_E><<<pr_tiles(length, PR_E), PR_T, pr_smem(PR_E), stream>>>(den, num, length, batch > 0);
+        }
         H2B_LAUNCHED("k_pp_finish");
     }
     H2B_CUDA(cudaMemcpyAsync(modified_values->ptr, den, length * 32, cudaMemcpyDeviceToHost, stream));
@@ -838,10 +890,15 @@ extern "C" RustError _halo2_permutation_product_device_inputs(
     }
     Fr* acc = (Fr*)modified_values_device->ptr;
     if (length > 0) {
-        enable_big_smem(k_permutation_product);
-        k_permutation_product<<<(unsigned)tiles_of(length), BI_T, BI_SMEM, stream>>>(
+        if (length < PR_SMALL) {
+            k_permutation_product<PR_E_SMALL><<<pr_tiles(length, PR_E_SMALL), PR_T, pr_smem(PR_E_SMALL), stream>>>(
             acc, cols, (int)batch, (const Fr*)beta_device, (const Fr*)gamma_device, (const Fr*)delta_device,
             (const Fr*)omega_device, (const Fr*)deltaomega_device, length);
+        } else {
+            k_permutation_product<PR_E><<<pr_tiles(length, PR_E), PR_T, pr_smem(PR_E), stream>>>(
+            acc, cols, (int)batch, (const Fr*)beta_device, (const Fr*)gamma_device, (const Fr*)delta_device,
+            (const Fr*)omega_device, (const Fr*)deltaomega_device, length);
+        }
         H2B_LAUNCHED("k_permutation_product");
     }
     k_advance_deltaomega<<<1, 32, 0, stream>>>((Fr*)deltaomega_device, (const Fr*)delta_device, batch);
