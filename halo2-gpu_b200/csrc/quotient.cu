@@ -20,6 +20,9 @@
 // intermediates.  Each thread walks whole rows; every thread of a warp
 // executes the same op, so there is no divergence, and column reads for
 // consecutive rows are coalesced.
+// products inline: the even/odd product is short enough that the fused kernel's
+// body still streams from the instruction cache (a 2^20 part 1.287 -> 1.250 ms)
+#define H2B_INLINE_MUL 1
 #include <algorithm>
 #include <cstring>
 #include <string>
