@@ -559,7 +559,7 @@ __device__ __forceinline__ uint32_t head_pieces(uint32_t m)
 // k_msm_heads.  Latency-bound unless the buckets are many: one lane per bucket
 // took 161 us for 4096 buckets of 19 heads.
 template <int G>
-__global__ void __launch_bounds__(128) k_msm_fixup(const uint32_t* __restrict__ offsets, uint64_t NB, const MsmChunk kc,
+__global__ void __launch_bounds__(128, 4) k_msm_fixup(const uint32_t* __restrict__ offsets, uint64_t NB, const MsmChunk kc,
                                                    G1Xyzz* __restrict__ buckets, const G1Xyzz* __restrict__ heads,
                                                    uint32_t limit, uint32_t* __restrict__ dense, uint64_t max_dense,
                                                    uint2* __restrict__ items, uint64_t max_items)
@@ -717,8 +717,10 @@ __global__ void __launch_bounds__(256) k_msm_heads_merge(const uint32_t* __restr
 // depth is the number of bits: running sums over 8-bucket segments and then
 // per-bit sums of the segments (16 and 16 additions one after the other at
 // c = 16) took 146 + 212 us for 8 windows of 2^15 buckets and 104 + 210 us for
-// one; the two passes here 117 + 60 and 76 + 53 us.
-__global__ void __launch_bounds__(FOLD_THREADS) k_msm_fold(const G1Xyzz* __restrict__ in, uint32_t arrays, uint32_t len,
+// one; the two passes here about 190 + 61 and 84 + 60 us (two CTAs per SM; one,
+// at 150 registers, made the first pass 333 us).
+template <int THREADS, int BLOCKS>
+__global__ void __launch_bounds__(THREADS, BLOCKS) k_msm_fold(const G1Xyzz* __restrict__ in, uint32_t arrays, uint32_t len,
                                                            int m, G1Xyzz* __restrict__ out, uint32_t* __restrict__ ctr,
                                                            uint32_t nctr)
 {
@@ -850,7 +852,7 @@ __global__ void k_write_inf(G1Jac* out)
 // the attribute is the device's, so it is set on every call).
 static cudaError_t fold_smem_ready()
 {
-    return cudaFuncSetAttribute(k_msm_fold, cudaFuncAttributeMaxDynamicSharedMemorySize, 512 * (int)sizeof(G1Xyzz));
+    return cudaFuncSetAttribute(k_msm_fold<256, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, 512 * (int)sizeof(G1Xyzz));
 }
 
 // Steps 5 to 7 from the accumulated buckets: chunk heads, bucket reduction, and
@@ -884,7 +886,8 @@ static RustError msm_reduce(const MsmPlan& p, const MsmScratch& s, int group_win
         const uint32_t tasks = std::max(arrays << (m - 1), arrays + (uint32_t)m);
         const size_t smem = sizeof(G1Xyzz) * ((size_t)(arrays + 1) << (m - 1));
         H2B_CUDA(fold_smem_ready());
-        k_msm_fold<<<(unsigned)p.Wr * (len >> m), (tasks + 31) / 32 * 32, smem, st>>>(
+        const auto fold = k == 0 ? k_msm_fold<256, 2> : k_msm_fold<(int)FOLD_THREADS, 1>;
+        fold<<<(unsigned)p.Wr * (len >> m), (tasks + 31) / 32 * 32, smem, st>>>(
             in, arrays, len, m, s.fold[k & 1], s.tailctr, k == 0 ? (uint32_t)p.leaves : 0u);
         H2B_LAUNCHED("k_msm_fold");
         in = s.fold[k & 1];
