@@ -55,6 +55,9 @@ static constexpr uint32_t ACC_MIN_K = 4;          // smallest chunk
 // 8.14 ms at 64, 8.07 at 96 and 128, 8.12 at 192).
 static constexpr uint32_t ACC_MAX_K = 96;
 static constexpr uint32_t ACC_MAX_K_SHARED = 128; // and of one of several that run at once
+// Lanes that the fixup spreads few buckets over (2^16 table, one MSM: 0.60 ms at
+// 2^15, 0.72 ms at 2^17 lanes; 2^20: 3.37 and 3.42 ms).
+static constexpr uint64_t FIX_THREADS = 32768;
 static constexpr uint32_t HEADS_PIECE = 32;       // chunk heads per warp of a long bucket
 static constexpr uint32_t HEADS_PIECES_MAX = 1024;
 static constexpr uint64_t MSM_PIPE_MIN = 1ull << 18;  // host scalars from here on are copied in pieces
@@ -173,8 +176,8 @@ static MsmPlan plan_core(uint64_t n, int c, uint64_t tn, uint32_t concurrent = 1
     // bucket with more than `limit` heads goes to warps of its own instead.
     const uint64_t avg = p.max_chunks / p.NB + 1;
     p.fix_lanes = 1;
-    while (p.fix_lanes < 32 && p.NB * p.fix_lanes < 32768 && p.fix_lanes < avg) p.fix_lanes *= 2;
-    p.fix_limit = p.fix_lanes * (uint32_t)std::min<uint64_t>(std::max<uint64_t>(2 * avg / p.fix_lanes + 2, 4), 16);
+    while (p.fix_lanes < 32 && p.NB * p.fix_lanes < FIX_THREADS && p.fix_lanes < avg) p.fix_lanes *= 2;
+    p.fix_limit = p.fix_lanes * (uint32_t)std::max<uint64_t>(2 * avg / p.fix_lanes + 2, 4);
     p.max_dense = p.max_chunks / p.fix_limit + 1;
     p.max_items = p.max_chunks / HEADS_PIECE + p.max_dense + 1;
     return p;
