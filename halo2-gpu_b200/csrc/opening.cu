@@ -194,20 +194,22 @@ static __global__ void k_lin_comb(Fr* __restrict__ acc, const __grid_constant__ 
 
 // ---- Kate division ---------------------------------------------------------
 
-// tab[0..7] = v^1..v^8, tab[8 + d] = v^(8 * 2^d) (d = 0..8), from v (one thread).
-static __global__ void k_kd_table(const Fr* __restrict__ v_in, Fr* __restrict__ tab)
+// tab[0..7] = v^1..v^8, tab[8 + d] = v^(8 * 2^d) (d = 0..8), by one thread;
+// returns the last one, v^2048.
+static __device__ Fr kd_table(const Fr& v, Fr* __restrict__ tab)
 {
-    if (blockIdx.x != 0 || threadIdx.x != 0) return;
-    const Fr v = ld(v_in);
     Fr p = v;
+#pragma unroll 1
     for (int k = 0; k < 8; k++) {
         st(&tab[k], p);
         if (k < 7) p = p * v;
     }
+#pragma unroll 1
     for (int d = 0; d <= 8; d++) {
         st(&tab[8 + d], p);
-        p = p * p;
+        if (d < 8) p = p * p;
     }
+    return p;
 }
 
 // Level L value t lives at: level 0 -> q[n-2-t] (reversed, written only below
@@ -300,42 +302,94 @@ static __global__ void __launch_bounds__(KD_T) k_kd_down(KdLevel L, const Fr* __
     }
 }
 
-// u^j and u^-j for j < KD_TILE (U and W), one CTA: thread 0 inverts u (0
-// stays 0) and forms u^(8 * 2^d), u^-(8 * 2^d); thread c then builds
-// entries 8c .. 8c + 7 from u^(8c) and u^-(8c).
-static __global__ void __launch_bounds__(KD_T) k_kd_pow(const Fr* __restrict__ u_in, Fr* __restrict__ U,
-                                                         Fr* __restrict__ W)
+// The top level when it is one tile: 256 values of one per thread or 2048 of two,
+// the scan over thread totals with multipliers v^(E 2^d).  Nine or twelve
+// dependent products instead of the 23 of k_kd_up's eight values per thread
+// (31 us; 10 us here at 128 values).
+template <int E>
+static __global__ void __launch_bounds__(E == 1 ? 256 : 1024) k_kd_top(Fr* __restrict__ arr, uint32_t m,
+                                                                       const Fr* __restrict__ tab)
 {
-    __shared__ Fr base[2][9];  // [0]: u, u^8, u^16, ...; [1]: the same for u^-1
-    const int c = threadIdx.x;
-    if (c == 0) {
-        Fr x[2];
-        x[0] = ld(u_in);
-        x[1] = finv_fast(x[0]);
-        for (int s = 0; s < 2; s++) {
-            base[s][0] = x[s];
-            Fr p = x[s] * x[s];
-            p = p * p;
-            p = p * p;  // x^8
-            for (int d = 0; d < 8; d++) {
-                base[s][1 + d] = p;
-                p = p * p;
-            }
-        }
+    constexpr int T = E == 1 ? 256 : 1024;
+    __shared__ Fr sm[T];
+    const uint32_t c = threadIdx.x, t0 = c * E;
+    Fr y[E];
+#pragma unroll
+    for (int k = 0; k < E; k++) {
+        y[k] = t0 + k < m ? ld(&arr[t0 + k]) : Fr::zero();
+        if (k) y[k] = y[k] + ldg(&tab[0]) * y[k - 1];
     }
+    Fr s = y[E - 1];
+#pragma unroll 1
+    for (int d = 0; (1u << d) * E < m; d++) {
+        const int e = d + E - 1;                        // multiplier v^(2^e)
+        sm[c] = s;
+        __syncthreads();
+        if (c >= (1u << d)) s = s + ldg(&tab[e < 3 ? (1 << e) - 1 : 5 + e]) * sm[c - (1u << d)];
+        __syncthreads();
+    }
+    sm[c] = s;
     __syncthreads();
-    for (int s = 0; s < 2; s++) {
+#pragma unroll
+    for (int k = 0; k < E; k++) {
+        if (t0 + k >= m) break;
+        if (k == E - 1) y[k] = s;
+        else if (c > 0) y[k] = y[k] + ldg(&tab[k]) * sm[c - 1];
+        st(&arr[t0 + k], y[k]);
+    }
+}
+
+// All power tables of one division, one CTA: u^j and u^-j for j < KD_TILE (U
+// and W) and the tables of the levels above (level l from v = u^(2048^l)).
+// The chains are serial, so they run side by side: warp 0 inverts u (0 stays
+// 0) and forms u^-(8 * 2^d); warp 1 forms u^(8 * 2^d), and behind the barrier of
+// warps 1 to 7 warp 2 the level tables and warps 3 to 7 U (thread by thread
+// entries 8c .. 8c + 7 from u^(8c)); at the end the whole CTA forms W.
+// One kernel of about 38 us; a table kernel per level and the chains one after
+// the other took 69 us.
+static __global__ void __launch_bounds__(KD_T) k_kd_pow(const Fr* __restrict__ u_in, Fr* __restrict__ U,
+                                                         Fr* __restrict__ W, Fr* __restrict__ tabs, int levels)
+{
+    __shared__ Fr base[2][10];  // [0]: u, u^8, u^16, .., u^2048; [1]: the same for u^-1 (up to u^-1024)
+    const int t = threadIdx.x;
+    auto chain = [&](int s, const Fr& x, int n) {
+        base[s][0] = x;
+        Fr p = x * x;
+        p = p * p;
+        p = p * p;
+#pragma unroll 1
+        for (int d = 0; d < n; d++) {
+            base[s][1 + d] = p;
+            if (d + 1 < n) p = p * p;
+        }
+    };
+    auto entries = [&](int s, int c, Fr* out) {
         Fr p = Fr::one();
+#pragma unroll 1
         for (int d = 0; d < 8; d++)
             if ((c >> d) & 1) p = p * base[s][1 + d];
-        Fr* out = s ? W : U;
         const Fr x = base[s][0];
 #pragma unroll 1
         for (int k = 0; k < KD_E; k++) {
             st(&out[c * KD_E + k], p);
             if (k + 1 < KD_E) p = p * x;
         }
+    };
+    if (t < 32) {
+        if (t == 0) chain(1, finv_fast(ld(u_in)), 8);
+    } else {
+        if (t == 32) chain(0, ld(u_in), 9);
+        __syncwarp();
+        asm volatile("bar.sync 1, 224;" ::: "memory");
+        if (t == 64) {
+            Fr v = base[0][9];
+            for (int l = 1; l <= levels; l++) v = kd_table(v, tabs + (uint64_t)KD_TAB * l);
+        } else if (t >= 96) {
+            for (int c = t - 96; c < KD_T; c += KD_T - 96) entries(0, c, U);
+        }
     }
+    __syncthreads();
+    entries(1, t, W);
 }
 
 // Level 0 up: P_j = sum_{s <= j} r_{kT+s} u^-s within the tile, written to q
@@ -449,13 +503,6 @@ static RustError kd_run(const Fr* a, Fr* q, const Fr* u, uint64_t n, uint64_t ql
         return scratch_too_small(who, bytes, sp.used);
     }
     lv[P.levels + 1] = top;
-    // power tables: level 0 from u, level l from table l-1's v^2048
-    k_kd_table<<<1, 32, 0, st>>>(u, tabs);
-    H2B_LAUNCHED("k_kd_table");
-    for (int l = 1; l <= P.levels; l++) {
-        k_kd_table<<<1, 32, 0, st>>>(tabs + (uint64_t)KD_TAB * (l - 1) + 16, tabs + (uint64_t)KD_TAB * l);
-        H2B_LAUNCHED("k_kd_table");
-    }
     auto level = [&](int l) {
         KdLevel L;
         L.arr = l == 0 ? q : lv[l];
@@ -465,13 +512,20 @@ static RustError kd_run(const Fr* a, Fr* q, const Fr* u, uint64_t n, uint64_t ql
         L.qlim = qlim;
         return L;
     };
-    k_kd_pow<<<1, KD_T, 0, st>>>(u, upow, wpow);
+    k_kd_pow<<<1, KD_T, 0, st>>>(u, upow, wpow, tabs, P.levels);
     H2B_LAUNCHED("k_kd_pow");
     const unsigned tiles0 = (unsigned)((P.m[0] + KD_TILE - 1) / KD_TILE);
     k_kd0_up<<<tiles0, KD_T, 0, st>>>(level(0), a, upow, wpow, lv[1]);
     H2B_LAUNCHED("k_kd0_up");
     for (int l = 1; l <= P.levels; l++) {
         const uint64_t tiles = (P.m[l] + KD_TILE - 1) / KD_TILE;
+        if (l == P.levels && P.m[l] <= 2048) {
+            const uint32_t m = (uint32_t)P.m[l];
+            if (m <= 256) k_kd_top<1><<<1, 256, 0, st>>>(lv[l], m, tabs + (uint64_t)KD_TAB * l);
+            else k_kd_top<2><<<1, 1024, 0, st>>>(lv[l], m, tabs + (uint64_t)KD_TAB * l);
+            H2B_LAUNCHED("k_kd_top");
+            break;
+        }
         k_kd_up<<<(unsigned)tiles, KD_T, 0, st>>>(level(l), a, tabs + (uint64_t)KD_TAB * l, lv[l + 1]);
         H2B_LAUNCHED("k_kd_up");
     }
