@@ -76,6 +76,46 @@ __global__ void __launch_bounds__(TW_T) k_twiddles(const Fr* __restrict__ lut, F
     }
 }
 
+// The two small tables behind k_twiddles_fill (below), lo[j] = w^j and
+// hi[j] = w^(2^TW2_LOG j), in one launch without a power table in memory: every
+// CTA squares w down in shared memory (dependent products, 0.45 us each) and
+// then makes 1024 entries of one table, four per thread.  A squaring kernel and
+// a kernel of 16 serial entries per table took 24 us; this one 12 us at 2^16.
+constexpr int TW_PAIR_K = 4;
+__global__ void __launch_bounds__(TW_T) k_twiddle_tables(const Fr* __restrict__ omega, int bits, Fr* __restrict__ lo,
+                                                         uint64_t nlo, Fr* __restrict__ hi, uint64_t nhi, int hi_bit)
+{
+    __shared__ Fr lut[40];
+    const uint32_t tiles_lo = (uint32_t)((nlo + TW_T * TW_PAIR_K - 1) / (TW_T * TW_PAIR_K));
+    const bool second = blockIdx.x >= tiles_lo;
+    if (threadIdx.x == 0) {
+        Fr cur = ld(omega);
+#pragma unroll 1
+        for (int i = 0; i < bits; i++) {
+            lut[i] = cur;
+            if (i + 1 < bits) cur = cur * cur;
+        }
+    }
+    __syncthreads();
+    const uint64_t n = second ? nhi : nlo;
+    const Fr* base = lut + (second ? hi_bit : 0);
+    Fr* out = second ? hi : lo;
+    uint64_t e = (blockIdx.x - (second ? tiles_lo : 0u)) * (uint64_t)(TW_T * TW_PAIR_K) + threadIdx.x;
+    if (e >= n) return;
+    Fr p = Fr::one();
+    int i = 0;
+#pragma unroll 1
+    for (uint64_t x = e; x; x >>= 1, i++)
+        if (x & 1) p = p * base[i];
+#pragma unroll 1
+    for (int j = 0; j < TW_PAIR_K; j++) {
+        st(&out[e], p);
+        e += TW_T;
+        if (e >= n) break;
+        p = p * base[TW_LOGT];
+    }
+}
+
 // tw[e] = lo[e mod 2^TW2_LOG] * hi[e >> TW2_LOG] with lo[j] = w^j and
 // hi[j] = w^(2^TW2_LOG j): one independent product per twiddle, both factors
 // from small tables that stay in cache.
@@ -114,13 +154,23 @@ constexpr int SC_CHUNK = 8;
 struct Zeta3 {
     Fr f[3];
 };
+// z3.f[i mod 3] by selects: an index that differs between lanes would read the
+// kernel parameters once per distinct address, word by word (n <= 2^28).
+__device__ __forceinline__ Fr zeta_pick(const Zeta3& z3, uint64_t i)
+{
+    const uint32_t m = (uint32_t)i % 3u;
+    Fr r;
+#pragma unroll
+    for (int w = 0; w < 8; w++) r.v[w] = m == 0 ? z3.f[0].v[w] : m == 1 ? z3.f[1].v[w] : z3.f[2].v[w];
+    return r;
+}
 __device__ __forceinline__ Fr twist_in(const Fr* __restrict__ in, uint64_t i, uint64_t n_in, int mode,
                                        const Fr* __restrict__ cpow, const Zeta3& z3)
 {
     if (i >= n_in) return Fr::zero();
     const Fr v = ldg(&in[i]);
     if (mode == 1) return v * ldg(&cpow[i]);
-    if (mode == 2) return v * z3.f[i % 3];
+    if (mode == 2) return v * zeta_pick(z3, i);
     return v;
 }
 __global__ void k_twist_bitrev_stage0(NttBatch B, uint64_t n_in, int log_out, int mode,
@@ -156,7 +206,7 @@ __global__ void k_coset_spread(NttBatch B, int log_in, int e, Zeta3 z3)
     for (uint64_t r = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; r < n_in;
          r += (uint64_t)gridDim.x * blockDim.x) {
         const uint64_t i = bitrev(r, log_in);
-        Fr v = ldg(&in[i]) * z3.f[i % 3];
+        Fr v = ldg(&in[i]) * zeta_pick(z3, i);
         Fr* dst = out + (r << e);
         for (uint64_t j = 0; j < g; j++) st(&dst[j], v);
     }
@@ -173,7 +223,7 @@ __global__ void k_twist_inplace(NttBatch B, uint64_t n, int mode, const Fr* __re
         for (int j = 0; j < SC_CHUNK && i0 + j < n; j++) {
             uint64_t i = i0 + j;
             Fr v = ld(&a[i]);
-            v = v * (mode == 1 ? ldg(&cpow[i]) : z3.f[i % 3]);
+            v = v * (mode == 1 ? ldg(&cpow[i]) : zeta_pick(z3, i));
             st(&a[i], v);
         }
     }
@@ -190,14 +240,14 @@ __global__ void k_bitrev_inplace(NttBatch B, int k, bool scale, Zeta3 z3)
         if (i < j) {
             Fr x = ld(&a[i]), y = ld(&a[j]);
             if (scale) {
-                y = y * z3.f[i % 3];
-                x = x * z3.f[j % 3];
+                y = y * zeta_pick(z3, i);
+                x = x * zeta_pick(z3, j);
             }
             st(&a[i], y);
             st(&a[j], x);
         } else if (i == j && scale) {
             Fr x = ld(&a[i]);
-            st(&a[i], x * z3.f[i % 3]);
+            st(&a[i], x * zeta_pick(z3, i));
         }
     }
 }
@@ -236,15 +286,19 @@ __global__ void __launch_bounds__(BR_THREADS) k_bitrev_tiled(NttBatch B, int k, 
     Fr* tile = reinterpret_cast<Fr*>(br_sh);
     Fr* __restrict__ a = B.dst[blockIdx.y];
     const int km = k - BR_MIN_LOG;
-    const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = BR_THREADS / 32;
+    const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    constexpr uint32_t nw = BR_THREADS / 32;
     for (uint64_t m = blockIdx.x; m < (1ull << km); m += gridDim.x) {
         const uint64_t mr = bitrev(m, km);
         if (m > mr) continue;  // the CTA of the partner tile moves both
         const int nt = (m == mr) ? 1 : 2;
         for (int t = 0; t < nt; t++) {
             const uint64_t mm = t ? mr : m;
-            for (uint32_t h = warp; h < BR_SIDE; h += nw)
-                st(&tile[t * BR_TILE + br_slot(h, lane)], ld(&a[br_index(h, mm, lane, k)]));
+            Fr v[BR_SIDE / nw];                  // all loads of a tile in flight together
+#pragma unroll
+            for (uint32_t r = 0; r < BR_SIDE / nw; r++) v[r] = ld(&a[br_index(warp + r * nw, mm, lane, k)]);
+#pragma unroll
+            for (uint32_t r = 0; r < BR_SIDE / nw; r++) st(&tile[t * BR_TILE + br_slot(warp + r * nw, lane)], v[r]);
         }
         __syncthreads();
         // tile t holds middle index mm; its element (h, l) lands at
@@ -255,7 +309,7 @@ __global__ void __launch_bounds__(BR_THREADS) k_bitrev_tiled(NttBatch B, int k, 
             for (uint32_t h = warp; h < BR_SIDE; h += nw) {
                 Fr v = ld(&tile[t * BR_TILE + br_slot(rev5(lane), rev5(h))]);
                 const uint64_t j = br_index(h, md, lane, k);
-                if (scale) v = v * z3.f[j % 3];
+                if (scale) v = v * zeta_pick(z3, j);
                 st(&a[j], v);
             }
         }
@@ -275,11 +329,15 @@ __global__ void __launch_bounds__(BR_THREADS) k_twist_bitrev_stage0_tiled(NttBat
     const Fr* __restrict__ in = B.src[blockIdx.y];
     Fr* __restrict__ out = B.dst[blockIdx.y];
     const int km = L - BR_MIN_LOG;
-    const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = BR_THREADS / 32;
+    const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    constexpr uint32_t nw = BR_THREADS / 32;
     for (uint64_t m = blockIdx.x; m < (1ull << km); m += gridDim.x) {
         const uint64_t mi = bitrev(m, km);
-        for (uint32_t h = warp; h < BR_SIDE; h += nw)
+#pragma unroll
+        for (uint32_t r = 0; r < BR_SIDE / nw; r++) {
+            const uint32_t h = warp + r * nw;
             st(&tile[br_slot(h, lane)], twist_in(in, br_index(h, mi, lane, L), n_in, mode, cpow, z3));
+        }
         __syncthreads();
         for (uint32_t h = warp; h < BR_SIDE; h += nw) {
             // output (h, m, l) holds input (rev5(l), mi, rev5(h)); DIT stage 0
@@ -687,27 +745,22 @@ static NttScratch carve_ntt(ScratchArena& ar, int log_size, bool data_slot, int 
     return s;
 }
 
-// Builds tw[] (and lut_w) for transforms of size 2^logn from a device omega.
+// Builds tw[] for transforms of size 2^logn from a device omega.
 static RustError make_twiddles(const Fr* d_omega, NttScratch& s, int logn, cudaStream_t st)
 {
     if (logn == 0) return ok();
-    k_pow2_lut<<<1, 32, 0, st>>>(d_omega, s.lut_w, logn);
-    H2B_LAUNCHED("k_pow2_lut");
-    uint64_t half = 1ull << (logn - 1);
-    const uint64_t tile = (uint64_t)TW_T * TW_K;
+    const uint64_t half = 1ull << (logn - 1), tile = (uint64_t)TW_T * TW_PAIR_K;
     if (half < (4ull << TW2_LOG)) {
-        k_twiddles<<<(unsigned)((half + tile - 1) / tile), TW_T, 0, st>>>(s.lut_w, s.tw, half);
-        H2B_LAUNCHED("k_twiddles");
+        k_twiddle_tables<<<(unsigned)((half + tile - 1) / tile), TW_T, 0, st>>>(d_omega, logn, s.tw, half, nullptr, 0, 0);
+        H2B_LAUNCHED("k_twiddle_tables");
         return ok();
     }
-    // lo[j] = w^j, j < 2^TW2_LOG; hi[j] = (w^(2^TW2_LOG))^j from the same power table shifted by TW2_LOG
     const uint64_t nlo = 1ull << TW2_LOG, nhi = half >> TW2_LOG;
     Fr* lo = s.tw2;
     Fr* hi = s.tw2 + nlo;
-    k_twiddles<<<(unsigned)((nlo + tile - 1) / tile), TW_T, 0, st>>>(s.lut_w, lo, nlo);
-    H2B_LAUNCHED("k_twiddles");
-    k_twiddles<<<(unsigned)((nhi + tile - 1) / tile), TW_T, 0, st>>>(s.lut_w + TW2_LOG, hi, nhi);
-    H2B_LAUNCHED("k_twiddles");
+    k_twiddle_tables<<<(unsigned)((nlo + tile - 1) / tile + (nhi + tile - 1) / tile), TW_T, 0, st>>>(
+        d_omega, logn, lo, nlo, hi, nhi, TW2_LOG);
+    H2B_LAUNCHED("k_twiddle_tables");
     k_twiddles_fill<<<grid_for(half, 256, 148u * 16u), 256, 0, st>>>(lo, hi, s.tw, half);
     H2B_LAUNCHED("k_twiddles_fill");
     return ok();
