@@ -368,6 +368,13 @@ constexpr int NTT_THREADS = 512;
 // spills).  Coset extension 2^22 -> 2^24 3.98 ms at two blocks, 3.83 ms at three;
 // ten inverse transforms at 2^16 264 -> 260 us (320 blocks in one wave).
 constexpr int NTT4_BLOCKS = 3;
+// Tiles that a pass should make at least (two rounds of the resident CTAs), and
+// the fewest groups a tile may be cut down to for it: a warp's global run is
+// then 64 bytes, which L2 still serves in full sectors.  Ten 2^16 transforms
+// 229 us with full tiles, 208 us down to 128-byte runs, 194 us down to 64; one
+// 2^12 transform 104, 80, 78 us.
+constexpr int NTT4_MIN_LG = 1;
+constexpr uint64_t NTT4_TILES = 888;
 constexpr int NTT_MIN_BLOCKS = 2;  // blocks per SM of the radix-2 pass
 
 template <bool DIT>
@@ -684,7 +691,11 @@ static RustError run_passes(NttBatch B, int count, const Fr* tw, int logn, bool 
         const int lS = dit ? s0 : logn - s0 - nst;
         // a one-stage pass runs the radix-2 kernel, whose tile stays at 2^10
         const bool pass4 = r4 && nst >= 2;
-        const int lG = std::min((pass4 ? tile_log : NTT_LOG_TILE) - nst, logn - nst);
+        int lG = std::min((pass4 ? tile_log : NTT_LOG_TILE) - nst, logn - nst);
+        // Fewer groups per tile while the tiles do not fill the GPU twice over:
+        // ten 2^16 transforms made 320 tiles of 2^11 (three on some SMs, two on
+        // others).
+        while (pass4 && lG > NTT4_MIN_LG && ((uint64_t)count << (logn - nst - lG)) < NTT4_TILES) lG--;
         const dim3 grid((unsigned)(1ull << (logn - nst - lG)), (unsigned)count);
         size_t smem = (size_t)(1ull << (lG + nst)) * sizeof(Fr);
         int threads = (int)std::min<uint64_t>(NTT_THREADS, std::max<uint64_t>(32, 1ull << (lG + nst - 1)));
