@@ -259,6 +259,28 @@ H2B_DEV Fq qsqr(const Fq& a)
 H2B_DEV Fq qadd(const Fq& a, const Fq& b) { return add2p<FqCfg>(a, b); }
 H2B_DEV Fq qsub(const Fq& a, const Fq& b) { return sub2p<FqCfg>(a, b); }
 
+// 2p - a (a <= 2p): the complement that turns a subtraction into an addition
+H2B_DEV Fq qneg2(const Fq& a)
+{
+    Fq r;
+    asm("sub.cc.u32 %0, %16, %8;\n\tsubc.cc.u32 %1, %17, %9;\n\tsubc.cc.u32 %2, %18, %10;\n\t"
+        "subc.cc.u32 %3, %19, %11;\n\tsubc.cc.u32 %4, %20, %12;\n\tsubc.cc.u32 %5, %21, %13;\n\t"
+        "subc.cc.u32 %6, %22, %14;\n\tsubc.u32 %7, %23, %15;"
+        : "=&r"(r.v[0]), "=&r"(r.v[1]), "=&r"(r.v[2]), "=&r"(r.v[3]), "=&r"(r.v[4]), "=&r"(r.v[5]), "=&r"(r.v[6]),
+          "=&r"(r.v[7])
+        : "r"(a.v[0]), "r"(a.v[1]), "r"(a.v[2]), "r"(a.v[3]), "r"(a.v[4]), "r"(a.v[5]), "r"(a.v[6]), "r"(a.v[7]),
+          "n"(m2word<FqCfg>(0)), "n"(m2word<FqCfg>(1)), "n"(m2word<FqCfg>(2)), "n"(m2word<FqCfg>(3)),
+          "n"(m2word<FqCfg>(4)), "n"(m2word<FqCfg>(5)), "n"(m2word<FqCfg>(6)), "n"(m2word<FqCfg>(7)));
+    return r;
+}
+
+// a b - c d, one reduction when the products are inline
+template <bool INL>
+H2B_DEV Fq qmulsub(const Fq& a, const Fq& b, const Fq& c, const Fq& d)
+{
+    return INL ? mont_mul_add_eo_lazy<FqCfg>(a, b, c, qneg2(d)) : qsub(qmul<INL>(a, b), qmul<INL>(c, d));
+}
+
 // the canonical memory image (infinity stays ZZ = 0)
 H2B_DEV G1Xyzz xyzze_canonical(const G1Xyzz& a)
 {
@@ -317,7 +339,7 @@ H2B_DEV void xyzze_madd(G1Xyzz& acc, const Fq& qx, const Fq& qy)
     acc.ZZ = qmul<INL>(acc.ZZ, PP);
     acc.ZZZ = qmul<INL>(acc.ZZZ, PPP);
     acc.X = qsub(qsub(qsqr<INL>(R), PPP), qadd(Q, Q));
-    acc.Y = qsub(qmul<INL>(R, qsub(Q, acc.X)), qmul<INL>(acc.Y, PPP));
+    acc.Y = qmulsub<INL>(R, qsub(Q, acc.X), acc.Y, PPP);
 }
 
 // add-2008-s: acc += q
@@ -402,21 +424,6 @@ H2B_DEV Fq qlin(uint32_t ca, const Fq& a, uint32_t cb, const Fq& b, uint32_t cc,
           "=&r"(r.v[7])
         : "r"(w[0]), "r"(w[1]), "r"(w[2]), "r"(w[3]), "r"(w[4]), "r"(w[5]), "r"(w[6]), "r"(w[7]), "r"(lo[0]), "r"(lo[1]),
           "r"(lo[2]), "r"(lo[3]), "r"(lo[4]), "r"(lo[5]), "r"(lo[6]), "r"(lo[7]));
-    return r;
-}
-
-// 2p - a (a <= 2p): the complement that turns a subtraction into an addition for qlin
-H2B_DEV Fq qneg2(const Fq& a)
-{
-    Fq r;
-    asm("sub.cc.u32 %0, %16, %8;\n\tsubc.cc.u32 %1, %17, %9;\n\tsubc.cc.u32 %2, %18, %10;\n\t"
-        "subc.cc.u32 %3, %19, %11;\n\tsubc.cc.u32 %4, %20, %12;\n\tsubc.cc.u32 %5, %21, %13;\n\t"
-        "subc.cc.u32 %6, %22, %14;\n\tsubc.u32 %7, %23, %15;"
-        : "=&r"(r.v[0]), "=&r"(r.v[1]), "=&r"(r.v[2]), "=&r"(r.v[3]), "=&r"(r.v[4]), "=&r"(r.v[5]), "=&r"(r.v[6]),
-          "=&r"(r.v[7])
-        : "r"(a.v[0]), "r"(a.v[1]), "r"(a.v[2]), "r"(a.v[3]), "r"(a.v[4]), "r"(a.v[5]), "r"(a.v[6]), "r"(a.v[7]),
-          "n"(m2word<FqCfg>(0)), "n"(m2word<FqCfg>(1)), "n"(m2word<FqCfg>(2)), "n"(m2word<FqCfg>(3)),
-          "n"(m2word<FqCfg>(4)), "n"(m2word<FqCfg>(5)), "n"(m2word<FqCfg>(6)), "n"(m2word<FqCfg>(7)));
     return r;
 }
 

@@ -727,6 +727,53 @@ H2B_DEV void eo_mont_sqr(uint32_t (&w)[8], const uint32_t (&a)[8])
     eo_close(w, e, o, t[15]);
 }
 
+// (e, o) += a b (no shift)
+template <class C>
+H2B_DEV void eo_mad(uint32_t (&e)[8], uint32_t (&o)[8], const uint32_t (&a)[8], uint32_t b)
+{
+    asm("mad.lo.cc.u32 %0, %8, %12, %0;\n\t"
+        "madc.hi.cc.u32 %1, %8, %12, %1;\n\t"
+        "madc.lo.cc.u32 %2, %9, %12, %2;\n\t"
+        "madc.hi.cc.u32 %3, %9, %12, %3;\n\t"
+        "madc.lo.cc.u32 %4, %10, %12, %4;\n\t"
+        "madc.hi.cc.u32 %5, %10, %12, %5;\n\t"
+        "madc.lo.cc.u32 %6, %11, %12, %6;\n\t"
+        "madc.hi.u32 %7, %11, %12, %7;"
+        : "+r"(o[0]), "+r"(o[1]), "+r"(o[2]), "+r"(o[3]), "+r"(o[4]), "+r"(o[5]), "+r"(o[6]), "+r"(o[7])
+        : "r"(a[1]), "r"(a[3]), "r"(a[5]), "r"(a[7]), "r"(b));
+    asm("mad.lo.cc.u32 %0, %9, %13, %0;\n\t"
+        "madc.hi.cc.u32 %1, %9, %13, %1;\n\t"
+        "madc.lo.cc.u32 %2, %10, %13, %2;\n\t"
+        "madc.hi.cc.u32 %3, %10, %13, %3;\n\t"
+        "madc.lo.cc.u32 %4, %11, %13, %4;\n\t"
+        "madc.hi.cc.u32 %5, %11, %13, %5;\n\t"
+        "madc.lo.cc.u32 %6, %12, %13, %6;\n\t"
+        "madc.hi.cc.u32 %7, %12, %13, %7;\n\t"
+        "addc.u32 %8, %8, 0;"
+        : "+r"(e[0]), "+r"(e[1]), "+r"(e[2]), "+r"(e[3]), "+r"(e[4]), "+r"(e[5]), "+r"(e[6]), "+r"(e[7]), "+r"(o[7])
+        : "r"(a[0]), "r"(a[2]), "r"(a[4]), "r"(a[6]), "r"(b));
+}
+
+// (a b + c d) 2^-256 mod p, below (a b + c d) / 2^256 + p, with one reduction
+// (200 wide multiply-adds instead of 272).  Between rows the value is below
+// a + c + p, so a + c < 2^256 - p (4.29 p).
+template <class C>
+H2B_DEV void eo_mont2(uint32_t (&w)[8], const uint32_t (&a)[8], const uint32_t (&b)[8], const uint32_t (&c)[8],
+                      const uint32_t (&d)[8])
+{
+    uint32_t e[8], o[8];
+    eo_mul_first<C>(e, o, a, b[0]);
+    eo_mad<C>(e, o, c, d[0]);
+    eo_redc<C>(e, o);
+#pragma unroll
+    for (int i = 1; i < 8; i++) {
+        eo_mad_shift<C>(e, o, a, b[i]);
+        eo_mad<C>(e, o, c, d[i]);
+        eo_redc<C>(e, o);
+    }
+    eo_close(w, e, o, 0u);
+}
+
 template <class C>
 H2B_DEV Fp<C> mont_mul_eo(const Fp<C>& a, const Fp<C>& b)
 {
@@ -1009,6 +1056,33 @@ H2B_DEV Fp<C> sub2p(const Fp<C>& a, const Fp<C>& b)
         : "+r"(r.v[0]), "+r"(r.v[1]), "+r"(r.v[2]), "+r"(r.v[3]), "+r"(r.v[4]), "+r"(r.v[5]), "+r"(r.v[6]),
           "+r"(r.v[7])
         : "r"(q0), "r"(q1), "r"(q2), "r"(q3), "r"(q4), "r"(q5), "r"(q6), "r"(q7));
+    return r;
+}
+
+// (a b + c d) 2^-256 mod p in [0, 2p) for a, b, c, d <= 2p: the sum's reduction
+// leaves less than (8 p / 2^256 + 1) p < 2.52 p, one correction by 2p
+template <class C>
+H2B_DEV Fp<C> mont_mul_add_eo_lazy(const Fp<C>& a, const Fp<C>& b, const Fp<C>& c, const Fp<C>& d)
+{
+    uint32_t t[8], s[8], bw;
+    eo_mont2<C>(t, a.v, b.v, c.v, d.v);
+    asm("sub.cc.u32  %0, %9, %17;\n\t"
+        "subc.cc.u32 %1, %10, %18;\n\t"
+        "subc.cc.u32 %2, %11, %19;\n\t"
+        "subc.cc.u32 %3, %12, %20;\n\t"
+        "subc.cc.u32 %4, %13, %21;\n\t"
+        "subc.cc.u32 %5, %14, %22;\n\t"
+        "subc.cc.u32 %6, %15, %23;\n\t"
+        "subc.cc.u32 %7, %16, %24;\n\t"
+        "subc.u32    %8, 0, 0;"
+        : "=r"(s[0]), "=r"(s[1]), "=r"(s[2]), "=r"(s[3]), "=r"(s[4]), "=r"(s[5]), "=r"(s[6]), "=r"(s[7]),
+          "=r"(bw)
+        : "r"(t[0]), "r"(t[1]), "r"(t[2]), "r"(t[3]), "r"(t[4]), "r"(t[5]), "r"(t[6]), "r"(t[7]),
+          "n"(m2word<C>(0)), "n"(m2word<C>(1)), "n"(m2word<C>(2)), "n"(m2word<C>(3)), "n"(m2word<C>(4)),
+          "n"(m2word<C>(5)), "n"(m2word<C>(6)), "n"(m2word<C>(7)));
+    Fp<C> r;
+#pragma unroll
+    for (int i = 0; i < 8; i++) r.v[i] = bw ? t[i] : s[i];
     return r;
 }
 
