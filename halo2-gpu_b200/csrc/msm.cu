@@ -231,7 +231,7 @@ void msm_plan_scratch(const MsmPlan& p, ScratchPlan& sp, bool scalar_host, bool 
     for (int k = 0; k < 2; k++) sp.add_n<G1Xyzz>(msm_fold_points(p, k));  // outputs of the reduction passes
     sp.add_n<uint32_t>(p.leaves);                     // counters of the last reduction step
     sp.add_n<G1Jac>(1);                               // result
-    if (p.tn == 0) sp.add_n<G1Affine>(2 * p.n);  // P_i and phi(P_i) in the lazy form (x 2^261)
+    if (p.tn == 0) sp.add_n<Fq>((g_msm_acc_variant == 6 ? 1 : 4) * p.n);  // x of phi(P_i); form 0: P_i, phi(P_i) x 2^261
 }
 
 MsmScratch msm_carve(const MsmPlan& p, ScratchArena& ar, bool scalar_host, bool bases_host)
@@ -252,7 +252,7 @@ MsmScratch msm_carve(const MsmPlan& p, ScratchArena& ar, bool scalar_host, bool 
     for (int k = 0; k < 2; k++) s.fold[k] = ar.take_n<G1Xyzz>(msm_fold_points(p, k));
     s.tailctr = ar.take_n<uint32_t>(p.leaves);
     s.result = ar.take_n<G1Jac>(1);
-    s.rbases = p.tn == 0 ? ar.take_n<G1Affine>(2 * p.n) : nullptr;
+    s.phix = p.tn == 0 ? ar.take_n<Fq>((g_msm_acc_variant == 6 ? 1 : 4) * p.n) : nullptr;
     return s;
 }
 
@@ -263,28 +263,13 @@ MsmScratch msm_carve(const MsmPlan& p, ScratchArena& ar, bool scalar_host, bool 
 // Virtual scalars: vs[2i] = k1, vs[2i+1] = k2 of the GLV split of scalar i
 // (128-bit magnitudes, sign in bit 127), so entry v stands for point i = v/2,
 // taken as P_i (v even) or phi(P_i) (v odd).
-// GLV split of each scalar; with `rb` set, base i is also converted to the
-// lazy x 2^261 form the accumulation reads (same index space, one launch):
-// rb[i] = P_i and rb[n + i] = phi(P_i) = (beta x, y), so the accumulation
-// multiplies by beta nowhere.
-__global__ void k_msm_glv(const Fr* __restrict__ sc, uint4* __restrict__ vs, uint64_t lo, uint64_t hi,
-                          const G1Affine* __restrict__ bases, G1Affine* __restrict__ rb, uint64_t n)
+__global__ void k_msm_glv(const Fr* __restrict__ sc, uint4* __restrict__ vs, uint64_t n)
 {
-    const Fq beta = glv::beta();
-    for (uint64_t i = lo + blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < hi;
-         i += (uint64_t)gridDim.x * blockDim.x) {
+    for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < n; i += (uint64_t)gridDim.x * blockDim.x) {
         uint4 a, b;
         glv::decompose(from_mont(ldg(&sc[i])), a, b);
         vs[2 * i] = a;
         vs[2 * i + 1] = b;
-        if (rb) {
-            const G1Affine q = ld_affine(&bases[i]);
-            const Fq y = to_r261(q.y);
-            st(&rb[i].x, to_r261(q.x));
-            st(&rb[i].y, y);
-            st(&rb[n + i].x, to_r261(q.x * beta));     // infinity (0, 0) stays (0, 0)
-            st(&rb[n + i].y, y);
-        }
     }
 }
 
@@ -355,14 +340,15 @@ __global__ void k_msm_sort(const uint4* __restrict__ vsc, uint64_t v0, uint64_t 
     }
 }
 
-// The GLV split and base conversion of k_msm_glv fused with the digit
+// The GLV split of each scalar and, over plain bases, the x coordinate beta x of
+// phi(P) = (beta x, y), fused with the digit
 // histogram of k_msm_sort<false> for the two halves of each scalar: the
 // histogram's atomics overlap the split's memory traffic, and the halves are
 // counted from registers instead of re-read.  Loops are block-uniform so
 // that every lane reaches the warp-wide match.
 __global__ void k_msm_glv_hist(const Fr* __restrict__ sc, uint4* __restrict__ vs, uint64_t lo, uint64_t hi,
-                               const G1Affine* __restrict__ bases, G1Affine* __restrict__ rb, uint64_t n, int c,
-                               int W, uint32_t H, uint32_t* __restrict__ counts, uint64_t tn)
+                               const G1Affine* __restrict__ bases, Fq* __restrict__ phix, int c, int W, uint32_t H,
+                               uint32_t* __restrict__ counts, uint64_t tn)
 {
     const Fq beta = glv::beta();
     for (uint64_t base = lo + blockIdx.x * (uint64_t)blockDim.x; base < hi; base += (uint64_t)gridDim.x * blockDim.x) {
@@ -373,14 +359,7 @@ __global__ void k_msm_glv_hist(const Fr* __restrict__ sc, uint4* __restrict__ vs
             glv::decompose(from_mont(ldg(&sc[i])), a, b);
             vs[2 * i] = a;
             vs[2 * i + 1] = b;
-            if (rb) {
-                const G1Affine q = ld_affine(&bases[i]);
-                const Fq y = to_r261(q.y);
-                st(&rb[i].x, to_r261(q.x));
-                st(&rb[i].y, y);
-                st(&rb[n + i].x, to_r261(q.x * beta));     // infinity (0, 0) stays (0, 0)
-                st(&rb[n + i].y, y);
-            }
+            if (phix) st(&phix[i], ldg(&bases[i].x) * beta);   // infinity (0, 0) stays (0, 0)
         }
         uint32_t ca = 0, cb = 0;
         for (int w = 0; w < W; w++) {
@@ -497,14 +476,20 @@ __device__ __forceinline__ Fq from_r261(const Fq& v)
     return r;
 }
 
-// The same accumulation with coordinates in [0, 2p) on the even/odd product:
-// bases are read in the x 2^261 storage form and divided by 32 on load;
-// buckets leave in the canonical memory image.
+// The accumulation with coordinates in [0, 2p) on the even/odd product (default).
+// TABLE: points in a window table's x 2^261 form, divided by 32 on load, phi(P)
+// at phi_off; else the caller's bases as they are, with the x coordinate of
+// phi(P) from phix (its y is P's).  Buckets leave in the canonical memory image.
+// Ten products an addition (two of them squares, two sharing a reduction) bound
+// it: 2^22 witness mix (39.7 M additions) 5.8 ms, against 8.6 ms with the FP64
+// form; 128 registers, 16 warps per SM (three CTAs measured 6.18 against 6.09 ms).
+template <bool TABLE>
 __global__ void __launch_bounds__(128, 4) k_msm_accumulate_e(const uint32_t* __restrict__ sorted,
                                                              const uint32_t* __restrict__ offsets, uint64_t NB,
                                                              const MsmChunk kc, const G1Affine* __restrict__ bases,
-                                                             uint64_t phi_off, G1Xyzz* __restrict__ buckets,
-                                                             G1Xyzz* __restrict__ heads, uint32_t pf)
+                                                             uint64_t phi_off, const Fq* __restrict__ phix,
+                                                             G1Xyzz* __restrict__ buckets, G1Xyzz* __restrict__ heads,
+                                                             uint32_t pf)
 {
     const uint32_t M = offsets[NB];
     const uint32_t K = chunk_entries(kc, M);
@@ -531,23 +516,29 @@ __global__ void __launch_bounds__(128, 4) k_msm_accumulate_e(const uint32_t* __r
             }
             if (pf && e + pf < end) {   // bring the point pf entries ahead into L2 (no registers held)
                 const uint32_t vn = sorted[e + pf] & ~SIGN_BIT;
-                const G1Affine* pn = &bases[(vn >> 1) + ((vn & 1u) ? phi_off : 0)];
+                const G1Affine* pn = &bases[(vn >> 1) + (TABLE && (vn & 1u) ? phi_off : 0)];
                 asm volatile("prefetch.global.L2 [%0];" ::"l"(pn));
+                if (!TABLE && (vn & 1u)) asm volatile("prefetch.global.L2 [%0];" ::"l"(&phix[vn >> 1]));
             }
             const uint32_t ent = sorted[e];
             const uint32_t v = ent & ~SIGN_BIT;
             const bool phi = (v & 1u) != 0;
-            const G1Affine P = ld_affine(&bases[(v >> 1) + (phi ? phi_off : 0)]);    // phi(P) precomputed
+            G1Affine P;
+            if (TABLE) {
+                P = ld_affine(&bases[(v >> 1) + (phi ? phi_off : 0)]);
+            } else {
+                P.x = ldg(phi ? &phix[v >> 1] : &bases[v >> 1].x);
+                P.y = ldg(&bases[v >> 1].y);
+            }
             if (is_inf(P)) continue;
-            const Fq qx = from_r261(P.x);
-            Fq qy = from_r261(P.y);
+            const Fq qx = TABLE ? from_r261(P.x) : P.x;
+            Fq qy = TABLE ? from_r261(P.y) : P.y;
             if (ent & SIGN_BIT) qy = qsub(Fq::zero(), qy);
             xyzze_madd<true>(acc, qx, qy);
         }
         st_xyzze(head ? &heads[t] : &buckets[b], acc);
     }
 }
-
 
 // pieces of a long bucket with m chunk heads (one warp each)
 __device__ __forceinline__ uint32_t head_pieces(uint32_t m)
@@ -923,22 +914,36 @@ static RustError msm_split(const MsmPlan& p, const MsmScratch& s, const Fr* d_sc
     const unsigned sm_cap = 148u * 16u;
     uint4* vsc = reinterpret_cast<uint4*>(s.canon);  // 2n x 16 B in the n x 32 B slot
     k_msm_glv_hist<<<grid_for(hi - lo, 256, sm_cap), 256, 0, st>>>(
-        d_scalars, vsc, lo, hi, d_bases, p.tn == 0 ? s.rbases : nullptr, p.n, p.c, p.W, p.H, s.counts,
-        p.tn);
+        d_scalars, vsc, lo, hi, d_bases, p.tn == 0 && g_msm_acc_variant == 6 ? s.phix : nullptr, p.c, p.W, p.H,
+        s.counts, p.tn);
     H2B_LAUNCHED("k_msm_glv_hist");
     return ok();
 }
 
-// The bucket accumulation over points in the x 2^261 form.
-static void msm_accumulate(const MsmPlan& p, const MsmScratch& s, const G1Affine* pts, cudaStream_t st)
+// The bucket accumulation over a window table (p.tn > 0) or plain bases.
+static RustError msm_accumulate(const MsmPlan& p, const MsmScratch& s, const G1Affine* pts, cudaStream_t st)
 {
-    const uint64_t phi = p.tn ? (uint64_t)p.W * p.tn : p.n;
     const unsigned grid = grid_for(p.max_chunks, 128, 148u * 32u);
-    if (g_msm_acc_variant == 6)
-        k_msm_accumulate_e<<<grid, 128, 0, st>>>(s.sorted, s.offsets, p.NB, p.chunk, pts, phi, s.buckets, s.heads,
-                                                 g_msm_prefetch);
-    else
-        k_msm_accumulate_z<<<grid, 128, 0, st>>>(s.sorted, s.offsets, p.NB, p.chunk, pts, phi, s.buckets, s.heads);
+    const uint64_t phi = (uint64_t)p.W * p.tn;
+    if (g_msm_acc_variant == 6) {
+        if (p.tn)
+            k_msm_accumulate_e<true><<<grid, 128, 0, st>>>(s.sorted, s.offsets, p.NB, p.chunk, pts, phi, nullptr,
+                                                           s.buckets, s.heads, g_msm_prefetch);
+        else
+            k_msm_accumulate_e<false><<<grid, 128, 0, st>>>(s.sorted, s.offsets, p.NB, p.chunk, pts, 0, s.phix,
+                                                            s.buckets, s.heads, g_msm_prefetch);
+        H2B_LAUNCHED("k_msm_accumulate");
+        return ok();
+    }
+    G1Affine* rb = (G1Affine*)s.phix;
+    if (!p.tn) {
+        k_to_r261<<<grid_for(p.n, 256, 148u * 8u), 256, 0, st>>>(pts, rb, p.n, rb + p.n);
+        H2B_LAUNCHED("k_to_r261");
+    }
+    k_msm_accumulate_z<<<grid, 128, 0, st>>>(s.sorted, s.offsets, p.NB, p.chunk, p.tn ? pts : rb, p.tn ? phi : p.n,
+                                             s.buckets, s.heads);
+    H2B_LAUNCHED("k_msm_accumulate");
+    return ok();
 }
 
 static RustError msm_finish(const MsmPlan& p, const MsmScratch& s, const G1Affine* d_bases, cudaStream_t st)
@@ -951,9 +956,8 @@ static RustError msm_finish(const MsmPlan& p, const MsmScratch& s, const G1Affin
                                                                     s.sorted, p.tn, 0u);
     H2B_LAUNCHED("k_msm_sort<scatter>");
     prof_begin(PROF_MSM_ACCUMULATE, st);
-    msm_accumulate(p, s, p.tn ? d_bases : s.rbases, st);
+    H2B_TRY(msm_accumulate(p, s, d_bases, st));
     prof_end(PROF_MSM_ACCUMULATE, st);
-    H2B_LAUNCHED("k_msm_accumulate");
     MsmOuts o;
     o.p[0] = s.result;
     H2B_TRY(msm_reduce(p, s, p.Wr, p.c, o, st));
@@ -987,8 +991,7 @@ RustError msm_run_merged(const MsmPlan& p, const MsmScratch& s, uint32_t J, cons
     uint64_t at = 0;   // job j's virtual scalars start at vsc + 2 * at
     for (uint32_t j = 0; j < J; j++) {
         if (ns[j] == 0) continue;
-        k_msm_glv<<<grid_for(ns[j], 256, sm_cap), 256, 0, st>>>(scalars[j], vsc + 2 * at, 0, ns[j], nullptr, nullptr,
-                                                                ns[j]);
+        k_msm_glv<<<grid_for(ns[j], 256, sm_cap), 256, 0, st>>>(scalars[j], vsc + 2 * at, ns[j]);
         H2B_LAUNCHED("k_msm_glv");
         k_msm_sort<false><<<grid_for(2 * ns[j], 256, sm_cap), 256, 0, st>>>(vsc + 2 * at, 0, 2 * ns[j], p.c, p.W,
                                                                               p.H, s.counts, nullptr, p.tn, j * p.H);
@@ -1006,9 +1009,8 @@ RustError msm_run_merged(const MsmPlan& p, const MsmScratch& s, uint32_t J, cons
         at += ns[j];
     }
     prof_begin(PROF_MSM_ACCUMULATE, st);
-    msm_accumulate(p, s, table, st);
+    H2B_TRY(msm_accumulate(p, s, table, st));
     prof_end(PROF_MSM_ACCUMULATE, st);
-    H2B_LAUNCHED("k_msm_accumulate");
     MsmOuts o;
     for (uint32_t j = 0; j < J; j++) o.p[j] = outs[j];
     H2B_TRY(msm_reduce(p, s, 1, 0, o, st));

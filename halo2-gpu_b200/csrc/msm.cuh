@@ -52,7 +52,7 @@ struct MsmScratch {
     G1Xyzz* fold[2];     // outputs of the reduction passes, alternating
     uint32_t* tailctr;   // arrival counters of the last reduction step
     G1Jac* result;
-    G1Affine* rbases;    // plain bases P_i, then phi(P_i), in the x 2^261 form
+    Fq* phix;            // plain bases: x of phi(P_i) (form 0: P_i, then phi(P_i), as points x 2^261)
 };
 
 // Plan for an MSM that runs beside `concurrent` - 1 others (batches): same
