@@ -997,11 +997,11 @@ Fr fr_from(const void* p)
 } // namespace
 
 // Register budget of the fused kernel, in blocks of 128 threads per SM: 3
-// (162 registers, no spills; the default), 4 (128 registers, a few spills)
-// or 5 (96 registers, more spills).  2^20 rows of a config-3 part: 1.416,
-// 1.500 and 1.489 ms (1.54 ms uncapped at 198 registers; the reference's
-// four per-part launches 1.50 ms).  Same results.
-static int g_fq_blocks = 3;
+// (168 registers), 4 (128; the default) or 5 (96).  Config-3 part on even/odd
+// products: 2^20 rows 1247, 1205 and 1224 us, 2^16 rows 145, 135 and 136 us.
+// The products of its [0, 2p) formulas stay out of line: inline they took 1399,
+// 1458 and 1519 us at 2^20 rows.  Same results.
+static int g_fq_blocks = 4;
 extern "C" void h2b_quotient_fused_set_blocks(int blocks_per_sm)
 {
     if (blocks_per_sm >= 3 && blocks_per_sm <= 5) g_fq_blocks = blocks_per_sm;

@@ -436,7 +436,7 @@ RustError h2b_quotient_fused(const void* const* fixed, uint64_t num_fixed, const
                              uint64_t rotation_scale, uint64_t row_start, uint64_t row_end, void* out,
                              uint64_t out_stride, uint64_t out_offset, const void* scale /* nullable */,
                              h2b_stream_t stream);
-/* register budget of the fused kernel: 3 (default), 4 or 5 blocks of 128 threads per SM; same results */
+/* register budget of the fused kernel: 3, 4 (default) or 5 blocks of 128 threads per SM; same results */
 void h2b_quotient_fused_set_blocks(int blocks_per_sm);
 int h2b_quotient_fused_get_blocks(void);
 /* culib.rs:603-617 ; quotient_lookups.cu:16-53 -- all device pointers */
@@ -463,16 +463,13 @@ RustError h2b_msm_device(const void* d_scalar, const void* d_bases, void* d_out,
 /* Window bits (0 = automatic; 4..22 accepted, other values also mean automatic) and sorted entries per
  * accumulation chunk (0 = automatic). */
 void h2b_msm_set_tuning(int window_bits, int chunk);
-/* Form of the MSM bucket-accumulation kernel: 6 = lazy R' = 2^260 limbs of 52 bits on the FP64 pipe
- * (default; window-table MSMs use it too); 0 = lazy R = 2^261 limbs of 29 bits with one-step carries on the
- * integer multiply pipe (window-table MSMs use it for every choice but 6).  A library built with
- * H2B_EXPERIMENTS=1 also has the normalised R = 2^256 forms 1..5 (slower; A/B comparisons only).  A value
- * that is not built leaves the setting unchanged.  Same results; tuning only. */
+/* Form of the MSM bucket-accumulation kernel: 6 = coordinates below 2p as eight 32-bit words, products in
+ * even and odd word rows (default); 0 = lazy R = 2^261 limbs of 29 bits with one-step carries (its workspace
+ * is larger: set it before sizing scratch).  Any other value leaves the setting unchanged.  Same results;
+ * tuning only. */
 void h2b_msm_set_accumulate_variant(int variant);
 int h2b_msm_get_accumulate_variant(void);
-/* Batch-affine pairing rounds before the XYZZ bucket accumulation (default 0; 1..3 only in a library built
- * with H2B_EXPERIMENTS=1, where they measured slower).  Same results; the MSM workspace-size queries depend on
- * it (set it before sizing scratch). */
+/* Batch-affine pairing rounds before the XYZZ bucket accumulation: not built, the setting stays 0. */
 void h2b_msm_set_pair_rounds(int rounds);
 int h2b_msm_get_pair_rounds(void);
 
@@ -588,7 +585,8 @@ int h2b_prof_read(int id, double* total_ms, int* count);
 RustError h2b_probe_imad(int blocks, int threads, int iters, void* d_sink, h2b_stream_t stream);
 RustError h2b_probe_modmul(int blocks, int threads, int iters, void* d_sink, h2b_stream_t stream);
 /* out[i] = a[i] * b[i] with product implementation `impl` (tests: 0-2 Fr CIOS lo/hi, CIOS wide,
- * 29-bit; 3 Fr square; 4 Fq product; 5 Fq square; 6 Fr, 7 Fq with the FP64 form). */
+ * 29-bit; 3 Fr square; 4 Fq product; 5 Fq square; 6 Fr, 7 Fq with the FP64 form; the
+ * even/odd forms 8 Fr, 9 Fq, 10 Fr square, 11 Fq square, 12 Fq a b + b a, operands below 2p). */
 RustError h2b_fr_mul_batch(int impl, const void* d_a, const void* d_b, void* d_out, uint64_t n,
                            h2b_stream_t stream);
 /* MSM accumulation: prefetch into L2 the point this many sorted entries ahead (0..64, default 2;
