@@ -146,6 +146,19 @@ __global__ void k_fq_mul_batch(const Fq* __restrict__ a, const Fq* __restrict__ 
                                 : mont_sqr_29<FqCfg>(ld(&a[i])));
 }
 
+// The even/odd forms: FORM 0 a b, 1 a^2, 2 a b + b a with one reduction; the
+// results of the lazy forms made canonical.
+template <class C, int FORM>
+__global__ void k_eo_batch(const Fp<C>* __restrict__ a, const Fp<C>* __restrict__ b, Fp<C>* __restrict__ out, uint64_t n)
+{
+    for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < n; i += (uint64_t)gridDim.x * blockDim.x) {
+        const Fp<C> x = ld(&a[i]), y = ld(&b[i]);
+        st(&out[i], canon2p<C>(FORM == 0   ? mont_mul_eo_lazy<C>(x, y)
+                               : FORM == 1 ? mont_sqr_eo_lazy<C>(x)
+                                           : mont_mul_add_eo_lazy<C>(x, y, y, x)));
+    }
+}
+
 // Four independent chains of 29-bit-limb products that stay in limb form.
 #if H2B_EXPERIMENTS
 __global__ void k_probe_mul29_chain(uint32_t* sink, int iters)
@@ -273,7 +286,9 @@ extern "C" RustError h2b_probe_modmul_impl(int impl, int blocks, int threads, in
 
 // out[i] = a[i] * b[i] with the chosen product implementation (tests):
 // 0-2 Fr products (CIOS lo/hi, CIOS wide, 29-bit), 3 Fr square (29-bit),
-// 4 Fq product, 5 Fq square (29-bit), 6 Fr product, 7 Fq product (FP64).
+// 4 Fq product, 5 Fq square (29-bit), 6 Fr product, 7 Fq product (FP64), and the
+// even/odd forms 8 Fr product, 9 Fq product, 10 Fr square, 11 Fq square, 12 Fq
+// a b + b a (operands of these may be anything below 2p).
 #endif  // H2B_EXPERIMENTS
 
 extern "C" RustError h2b_fr_mul_batch(int impl, const void* d_a, const void* d_b, void* d_out, uint64_t n,
@@ -294,6 +309,16 @@ extern "C" RustError h2b_fr_mul_batch(int impl, const void* d_a, const void* d_b
         k_fr_mul_batch<6><<<grid_for(n, 256), 256, 0, stream>>>((const Fr*)d_a, (const Fr*)d_b, (Fr*)d_out, n);
     else if (impl == 7)
         k_fq_mul_batch<7><<<grid_for(n, 256), 256, 0, stream>>>((const Fq*)d_a, (const Fq*)d_b, (Fq*)d_out, n);
+    else if (impl == 8)
+        k_eo_batch<FrCfg, 0><<<grid_for(n, 256), 256, 0, stream>>>((const Fr*)d_a, (const Fr*)d_b, (Fr*)d_out, n);
+    else if (impl == 9)
+        k_eo_batch<FqCfg, 0><<<grid_for(n, 256), 256, 0, stream>>>((const Fq*)d_a, (const Fq*)d_b, (Fq*)d_out, n);
+    else if (impl == 10)
+        k_eo_batch<FrCfg, 1><<<grid_for(n, 256), 256, 0, stream>>>((const Fr*)d_a, (const Fr*)d_b, (Fr*)d_out, n);
+    else if (impl == 11)
+        k_eo_batch<FqCfg, 1><<<grid_for(n, 256), 256, 0, stream>>>((const Fq*)d_a, (const Fq*)d_b, (Fq*)d_out, n);
+    else if (impl == 12)
+        k_eo_batch<FqCfg, 2><<<grid_for(n, 256), 256, 0, stream>>>((const Fq*)d_a, (const Fq*)d_b, (Fq*)d_out, n);
     else
         k_fq_mul_batch<5><<<grid_for(n, 256), 256, 0, stream>>>((const Fq*)d_a, (const Fq*)d_b, (Fq*)d_out, n);
     H2B_LAUNCHED("k_fr_mul_batch");
