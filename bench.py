@@ -20,14 +20,13 @@ mix), and its value is the points/s those steps measured; the coset NTT
 2^22 -> 2^24 and the batch inversion of 2^24 elements are each timed once at
 full size beside it (`cpu_rows`).
 
-The dominant kernel's roofline is its binding resource, the field products:
-the FP64-form product (five 52-bit limbs, exact FMA splits) issues, per 32
-products, 430 warp instructions of which 211 go to the integer ALU pipe and
-155 to the FP64 pipe (ncu, profiles/product_probe_fp64.md); with B200's 4
-issue slots and 2 ALU and 2 FP64 warp instructions per clock per SM, issue
-bounds it at 148 x 4 / 430 x 32 products per clock (the ALU pipe within 2 %).
-That ceiling, at the SM clock sampled during the run, is `roofline.peak`;
-the HBM figures sit beside it in `roofline.hbm`.
+The dominant kernel's roofline is its binding resource, the multiply pipe: a
+mixed addition of the bucket accumulation makes 1160 wide multiply-adds with
+carry (six products of 128, one two-product sum with a single reduction of
+192, two squares of 100) and 72 digit products of half the cost, and a
+scheduler's pipe takes a warp's wide multiply-add every four cycles (32 per
+clock per SM).  That ceiling, at the SM clock sampled during the run, is
+`roofline.peak`; the HBM figures sit beside it in `roofline.hbm`.
 """
 import argparse
 import ctypes
@@ -82,26 +81,17 @@ def whole_job_points_per_s(world, points_per_rank, ms):
     return world * points_per_rank / (ms * 1e-3)
 
 
-# Per 32 products of the FP64-form field product (ncu on h2b_probe_modmul's
-# kernel, profiles/product_probe_fp64.md): warp instructions issued, and those
-# executed by the integer ALU pipe and the FP64 pipe.
-PRODUCT_WARP_INST = {"issue": 430, "alu": 211, "fp64": 155}
-# B200 warp instructions per clock per SM: issue slots (4 schedulers), ALU and
-# FP64 pipes (16 lanes per scheduler each)
-SM_RATE = {"issue": 4, "alu": 2, "fp64": 2}
+# Wide multiply-adds (32 x 32 + 64 bits with carry) of one mixed addition, the
+# digit products (mad.lo, half a wide one's cycles) counted as halves
+ADD_WIDE = 6 * 128 + 192 + 2 * 100 + 72 / 2
+# lanes of wide multiply-adds per clock per SM: four schedulers, a warp every four cycles
+WIDE_PER_CLK = 32
 NUM_SMS = 148
 
 
-def product_ceiling(sm_mhz):
-    """Products/s ceilings of the FP64-form field product at `sm_mhz`: per
-    resource, SMs x rate / (warp instructions per 32 products) x 32; the
-    lowest binds."""
-    ceilings = {r: NUM_SMS * SM_RATE[r] / PRODUCT_WARP_INST[r] * 32 * sm_mhz * 1e6 / 1e9 for r in SM_RATE}
-    bind = min(ceilings, key=ceilings.get)
-    return {"peak_gproducts_per_s": ceilings[bind], "binding": bind,
-            "ceilings": {r: round(v, 2) for r, v in ceilings.items()},
-            "source": f"{bind} pipe: {NUM_SMS} SMs x {SM_RATE[bind]} warp instr/clk / "
-                      f"{PRODUCT_WARP_INST[bind]} per 32 products at {sm_mhz:.0f} MHz (sampled SM clock)"}
+def multiply_ceiling(sm_mhz):
+    """Wide multiply-adds per second (in 1e9) of the multiply pipes at `sm_mhz`."""
+    return NUM_SMS * WIDE_PER_CLK * sm_mhz * 1e6 / 1e9
 
 
 def peaks():
@@ -1116,17 +1106,16 @@ def main():
     acc_avg_ms = acc_ms / max(acc_cnt, 1)
     acc_bytes = entries * (4 + 64) + (1 << 19) * 128          # sorted ids + affine points + bucket sums
     acc_modmul = entries * 10                                  # XYZZ mixed add 8M + 2S
-    # the accumulation is bound by its field products (about 0.25 products per
-    # byte of traffic), so the roofline is the FP64-form product's pipe ceiling
+    # the accumulation is bound by its field products (about 0.15 products per
+    # byte of traffic), so the roofline is the multiply pipe's rate
     sm_mhz = clk.get("sm_mhz") or 1965.0
-    ceil = product_ceiling(sm_mhz)
-    acc_gps = acc_modmul / (acc_avg_ms * 1e-3) / 1e9
+    ceil = multiply_ceiling(sm_mhz)
+    acc_gws = entries * ADD_WIDE / (acc_avg_ms * 1e-3) / 1e9
     hbm_achieved = acc_bytes / (acc_avg_ms * 1e-3) / 1e9
-    roofline = {"bound": f"{ceil['binding']} (FP64-form field products)", "kernel": "k_msm_accumulate_d",
-                "achieved": acc_gps, "peak": ceil["peak_gproducts_per_s"], "unit": "G products/s",
-                "frac": acc_gps / ceil["peak_gproducts_per_s"],
-                "peak_source": ceil["source"], "ceilings_gproducts_per_s": ceil["ceilings"],
-                "traffic": ncu_traffic("msm_accumulate_d_k22.md"),
+    roofline = {"bound": "multiply pipe (wide multiply-adds with carry)", "kernel": "k_msm_accumulate_e",
+                "achieved": acc_gws, "peak": ceil, "unit": "G wide multiply-adds/s", "frac": acc_gws / ceil,
+                "peak_source": f"{NUM_SMS} SMs x {WIDE_PER_CLK} lanes/clk at {sm_mhz:.0f} MHz (sampled SM clock)",
+                "traffic": ncu_traffic("msm_accumulate_e_k22.md"),
                 "products_per_launch": acc_modmul, "launch_ms": acc_avg_ms,
                 "hbm": {"achieved_GB_per_s": hbm_achieved, "peak_GB_per_s": hbm,
                         "frac": hbm_achieved / hbm,
@@ -1134,10 +1123,10 @@ def main():
                                         "fallback: MEASURED_PEAKS.json absent, 6.65 TB/s measured earlier on this pool"),
                         "algorithmic_bytes_per_launch": acc_bytes}}
     # beside it: the same product in register-resident chains (h2b_probe_modmul)
-    products = {"kernel": "k_msm_accumulate_d", "modmul_per_launch": acc_modmul,
+    products = {"kernel": "k_msm_accumulate_e", "modmul_per_launch": acc_modmul,
                 "achieved_products_per_s": acc_modmul / (acc_avg_ms * 1e-3),
                 "peak_products_per_s": probe["h2b_probe_modmul"],
-                "peak_source": "measured h2b_probe_modmul (operator*, FP64 product, four chains per thread)",
+                "peak_source": "measured h2b_probe_modmul (operator*, four chains per thread)",
                 "imad_ops_per_s_probe": probe["h2b_probe_imad"]}
     products["frac"] = products["achieved_products_per_s"] / products["peak_products_per_s"]
     ntt_kernel_ms = nttp_ms / max(nttp_cnt, 1)
@@ -1146,7 +1135,7 @@ def main():
     line = {
         "metric": METRIC, "value": value, "unit": UNIT, "n_gpus": world, "steps": args.steps,
         "warmup": max(args.warmup, 3), "ms_per_step": step_ms, "higher_is_better": True, "scaling": "weak",
-        "vs_baseline": None, "dtype": "Montgomery Fr/Fq, exact integer (52-bit limbs in f64 for products, u32 words in memory)",
+        "vs_baseline": None, "dtype": "Montgomery Fr/Fq, exact integer (eight u32 words)",
         "data": "synthetic (seeded SRS [tau^i]G and scalars; generated on device)",
         "config": dict(WORKLOAD, parallelism=f"replicas x{world}"),
         "msm": {"ms": msm_ms, "points_per_s": n_msm / (msm_ms * 1e-3), "entries": entries,

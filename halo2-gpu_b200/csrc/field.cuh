@@ -833,10 +833,13 @@ H2B_DEV Fp<C> mont_sqr_eo_lazy(const Fp<C>& a)
 // so the result is below (p / 2^256 + 1) p < 1.19 p; one conditional
 // subtraction makes it canonical.  Column values stay below 2^57.
 //
-// Throughput measured on B200 (two independent product chains per thread):
-// 53-54 G products/s against 41-42 G for mont_mul_29.  The products use the
-// FP64 pipe and the column sums the integer ALU, leaving the multiply pipe
-// (which the 29-bit form saturates) almost idle.
+// Measured on B200: 55 G products/s at 64 to 72 registers (the even/odd form
+// 67.5 G at 40).  A limb product with its split and sums takes 10.4 cycles per
+// scheduler however many warps run, about what its 20 register words read take
+// at two words a cycle, so neither fewer ALU instructions (the carry of a digit
+// folded into the column's bias) nor a shorter digit chain (a multiple of p
+// that is -1 mod 2^52) made it faster.  Kept as an independent second product
+// for the tests of the first.
 
 namespace f64 {
 constexpr uint64_t M52 = (1ull << 52) - 1;
@@ -974,12 +977,10 @@ H2B_DEV Fp<C> mont_mul_f64(const Fp<C>& a, const Fp<C>& b)
 
 // ---- residues in [0, 2p) ----------------------------------------------------
 // A chain of products and sums (an NTT pass) can keep its values in [0, 2p)
-// and make them canonical once at the end.  The FP64 product's bound with
-// a, b < 2p: 16 a b + Q p < 64 p^2 + 2^260 p, so the result is below
-// (64 p / 2^260 + 1) p < 1.76 p for both BN254 moduli (p < 2^253.6), and its closing
-// subtraction can be left out; a sum below 4p (< 2^256) or a difference in
-// (-2p, 2p) takes one correction by 2p.  Column bounds of the product do not
-// depend on the operands' size (every limb is below 2^52 and 16 a < 2^260).
+// and make them canonical once at the end.  A product of a, b < 2p is below
+// (4 p / 2^256 + 1) p < 1.76 p for both BN254 moduli (p < 2^253.6), so its
+// closing subtraction can be left out; a sum below 4p (< 2^256) or a difference
+// in (-2p, 2p) takes one correction by 2p.
 
 // word w of 2m (8 x 32 grid)
 template <class C>

@@ -1,4 +1,4 @@
-// Lazy 29-bit limb arithmetic for the MSM bucket accumulation.
+// Lazy 29-bit limb arithmetic for the MSM bucket accumulation (accumulate form 0).
 //
 // The accumulation runs one mixed XYZZ addition per sorted entry; in the
 // normalised limb form (field.cuh, R = 2^256) each of its seven additions and

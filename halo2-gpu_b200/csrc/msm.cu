@@ -650,8 +650,7 @@ __global__ void __launch_bounds__(128) k_msm_heads(const uint32_t* __restrict__ 
 }
 
 // CTA-wide tree sum of n XYZZ values produced by get(i); result valid in
-// thread 0.  The partial sums stay in 29-bit limb form (latency-oriented
-// products: every level of the tree is one dependent addition per thread).
+// thread 0 (coordinates below 2p).
 template <class Get>
 __device__ G1Xyzz block_sum_xyzz(uint64_t n, Get get)
 {

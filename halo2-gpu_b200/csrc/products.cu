@@ -309,8 +309,8 @@ static RustError batch_invert_groups(Fp<C>* d, uint64_t n, ScratchArena& ar, cud
     return ok();
 }
 
-// In-place Fq batch inversion for other kernels of this library (the MSM's
-// pairing rounds): zeros stay zero; scratch from fq_batch_invert_scratch().
+// In-place Fq batch inversion for other kernels of this library (window
+// tables): zeros stay zero; scratch from fq_batch_invert_scratch().
 uint64_t fq_batch_invert_scratch(uint64_t n)
 {
     ScratchPlan p;
