@@ -39,14 +39,6 @@ H2B_DEV G1Xyzz xyzz_inf()
     return r;
 }
 
-H2B_DEV G1Xyzz xyzz_from_affine(const G1Affine& p)
-{
-    if (is_inf(p)) return xyzz_inf();
-    G1Xyzz r;
-    r.X = p.x; r.Y = p.y; r.ZZ = Fq::one(); r.ZZZ = Fq::one();
-    return r;
-}
-
 H2B_DEV G1Affine ld_affine(const G1Affine* p)
 {
     G1Affine r;
@@ -127,32 +119,6 @@ H2B_DEV void xyzz_madd(G1Xyzz& acc, const G1Affine& q)
     acc.X = X3;
     acc.ZZ = acc.ZZ * PP;
     acc.ZZZ = acc.ZZZ * PPP;
-}
-
-// add-2008-s: acc += q (both XYZZ).
-H2B_DEV void xyzz_add(G1Xyzz& acc, const G1Xyzz& q)
-{
-    if (is_inf(q)) return;
-    if (is_inf(acc)) { acc = q; return; }
-    Fq U1 = acc.X * q.ZZ;
-    Fq U2 = q.X * acc.ZZ;
-    Fq S1 = acc.Y * q.ZZZ;
-    Fq S2 = q.Y * acc.ZZZ;
-    Fq P = U2 - U1;
-    Fq R = S2 - S1;
-    if (P.is_zero()) {
-        if (R.is_zero()) acc = xyzz_dbl(acc);
-        else acc = xyzz_inf();
-        return;
-    }
-    Fq PP = fsqr(P);
-    Fq PPP = P * PP;
-    Fq Q = U1 * PP;
-    Fq X3 = fsqr(R) - PPP - fdbl(Q);
-    acc.Y = R * (Q - X3) - S1 * PPP;
-    acc.X = X3;
-    acc.ZZ = acc.ZZ * q.ZZ * PP;
-    acc.ZZZ = acc.ZZZ * q.ZZZ * PPP;
 }
 
 // ---- XYZZ in the lazy form (R = 2^261), for the bucket accumulation -------
@@ -518,21 +484,6 @@ H2B_DEV void sl_add(Fq* sl)
 }
 #undef SL6
 
-H2B_DEV G1Affine affine_neg(const G1Affine& p)
-{
-    G1Affine r;
-    r.x = p.x;
-    r.y = p.y.is_zero() ? p.y : fneg(p.y);
-    return r;
-}
-
-H2B_DEV G1Xyzz xyzz_neg(const G1Xyzz& p)
-{
-    G1Xyzz r = p;
-    if (!is_inf(p)) r.Y = fneg(p.Y);
-    return r;
-}
-
 // XYZZ -> reference Jacobian image (affine with Z = 1; infinity = (0, 1, 0)).
 H2B_DEV G1Jac xyzz_to_jac_affine(const G1Xyzz& p)
 {
@@ -547,20 +498,6 @@ H2B_DEV G1Jac xyzz_to_jac_affine(const G1Xyzz& p)
     r.X = p.X * izz;
     r.Y = p.Y * izzz;
     r.Z = Fq::one();
-    return r;
-}
-
-// Scalar multiplication by a small non-negative integer (double-and-add).
-H2B_DEV G1Xyzz xyzz_mul_u32(const G1Xyzz& p, uint32_t k)
-{
-    G1Xyzz r = xyzz_inf();
-    if (k == 0 || is_inf(p)) return r;
-    int top = 31 - __clz(k);
-#pragma unroll 1
-    for (int i = top; i >= 0; i--) {
-        r = xyzz_dbl(r);
-        if ((k >> i) & 1u) xyzz_add(r, p);
-    }
     return r;
 }
 

@@ -1096,133 +1096,6 @@ H2B_DEV Fp<C> canon2p(const Fp<C>& a)
     return r;
 }
 
-// ---- Fl arithmetic kept in limb form (values < 2p, limbs < 2^29) ---------
-
-// limb i of 2m (m2word above) in the 29-bit grid
-template <class C>
-__host__ __device__ constexpr uint32_t p2_29(int i)
-{
-    return (uint32_t)((((uint64_t)m2word<C>((29 * i) / 32)) | ((uint64_t)m2word<C>((29 * i) / 32 + 1) << 32)) >>
-                      ((29 * i) % 32)) & M29;
-}
-
-// Signed limbs -> normalised limbs, carries/borrows moved up (top limb keeps the sign).
-H2B_DEV void fl_normalise(int32_t (&d)[9])
-{
-#pragma unroll
-    for (int i = 0; i < 8; i++) {
-        const int32_t c = d[i] >> 29;
-        d[i] &= (int32_t)M29;
-        d[i + 1] += c;
-    }
-}
-
-// a - b (+ 2m when negative); inputs and output < 2m.
-template <class C>
-H2B_DEV Fl<C> fl_sub(const Fl<C>& a, const Fl<C>& b)
-{
-    int32_t d[9];
-#pragma unroll
-    for (int i = 0; i < 9; i++) d[i] = (int32_t)a.l[i] - (int32_t)b.l[i];
-    fl_normalise(d);
-    const int32_t neg = d[8] >> 31;
-#pragma unroll
-    for (int i = 0; i < 9; i++) d[i] += (int32_t)(p2_29<C>(i) & (uint32_t)neg);
-    fl_normalise(d);
-    Fl<C> r;
-#pragma unroll
-    for (int i = 0; i < 9; i++) r.l[i] = (uint32_t)d[i];
-    return r;
-}
-
-// a + b (- 2m when >= 2m); inputs and output < 2m.
-template <class C>
-H2B_DEV Fl<C> fl_add(const Fl<C>& a, const Fl<C>& b)
-{
-    int32_t s[9], t[9];
-#pragma unroll
-    for (int i = 0; i < 9; i++) s[i] = (int32_t)(a.l[i] + b.l[i]);
-    fl_normalise(s);
-#pragma unroll
-    for (int i = 0; i < 9; i++) t[i] = s[i] - (int32_t)p2_29<C>(i);
-    fl_normalise(t);
-    const bool keep = t[8] < 0;
-    Fl<C> r;
-#pragma unroll
-    for (int i = 0; i < 9; i++) r.l[i] = (uint32_t)(keep ? s[i] : t[i]);
-    return r;
-}
-
-// a == 0 (mod m) for a < 2m: a is 0 or m.
-template <class C>
-H2B_DEV bool fl_is_zero_mod(const Fl<C>& a)
-{
-    uint32_t z = 0, e = 0;
-#pragma unroll
-    for (int i = 0; i < 9; i++) {
-        z |= a.l[i];
-        e |= a.l[i] ^ p29<C>(i);
-    }
-    return z == 0 || e == 0;
-}
-
-template <class C>
-H2B_DEV bool fl_is_zero(const Fl<C>& a)
-{
-    uint32_t z = 0;
-#pragma unroll
-    for (int i = 0; i < 9; i++) z |= a.l[i];
-    return z == 0;
-}
-
-template <class C>
-H2B_DEV Fl<C> fl_zero()
-{
-    Fl<C> r;
-#pragma unroll
-    for (int i = 0; i < 9; i++) r.l[i] = 0;
-    return r;
-}
-
-// Out-of-line products for kernels that chain many of them.  A call costs
-// about a fifth of a product (measured: 42 G/s out of line against 54.7 G/s
-// inline), so the paired forms compute two independent products per call,
-// which also gives the scheduler two dependency chains to interleave.
-template <class C>
-__device__ __noinline__ Fl<C> fl_mul(const Fl<C> a, const Fl<C> b)
-{
-    return mul29<C>(a, b);
-}
-
-template <class C>
-__device__ __noinline__ Fl<C> fl_sqr(const Fl<C> a)
-{
-    return sqr29<C>(a);
-}
-
-template <class C>
-struct Fl2 {
-    Fl<C> a, b;
-};
-
-template <class C>
-__device__ __noinline__ Fl2<C> fl_mul2(const Fl<C> a0, const Fl<C> b0, const Fl<C> a1, const Fl<C> b1)
-{
-    Fl2<C> r;
-    r.a = mul29<C>(a0, b0);
-    r.b = mul29<C>(a1, b1);
-    return r;
-}
-
-template <class C>
-__device__ __noinline__ Fl2<C> fl_sqr2(const Fl<C> a0, const Fl<C> a1)
-{
-    Fl2<C> r;
-    r.a = sqr29<C>(a0);
-    r.b = sqr29<C>(a1);
-    return r;
-}
-
 // operator* and fsqr.  One out-of-line body per field by default: kernels that
 // chain many products (curve formulas, the quotient interpreter) otherwise
 // inline hundreds of instructions per product and starve on instruction
@@ -1376,33 +1249,6 @@ H2B_DEV Fp<C> from_mont(const Fp<C>& a)
 }
 template <class C>
 H2B_DEV Fp<C> to_mont(const Fp<C>& a) { return a * Fp<C>::r2(); }
-
-// a^e for a 256-bit exponent given as 8 little-endian words; 4-bit fixed window.
-template <class C>
-H2B_DEV Fp<C> fpow(const Fp<C>& a, const uint32_t (&e)[8])
-{
-    Fp<C> tbl[16];
-    tbl[0] = Fp<C>::one();
-    tbl[1] = a;
-#pragma unroll 1
-    for (int i = 2; i < 16; i++) tbl[i] = tbl[i - 1] * a;
-    Fp<C> r = Fp<C>::one();
-#pragma unroll 1
-    for (int w = 63; w >= 0; w--) {
-        r = r * r; r = r * r; r = r * r; r = r * r;
-        uint32_t d = (e[w >> 3] >> ((w & 7) * 4)) & 15u;
-        if (d) r = r * tbl[d];
-    }
-    return r;
-}
-
-// Fermat inverse a^(m-2); inverse of zero is zero.
-template <class C>
-H2B_DEV Fp<C> finv(const Fp<C>& a)
-{
-    const uint32_t e[8] = {C::M0 - 2u, C::M1, C::M2, C::M3, C::M4, C::M5, C::M6, C::M7};
-    return fpow<C>(a, e);
-}
 
 template <class C>
 H2B_DEV Fp<C> ldg(const Fp<C>* p)

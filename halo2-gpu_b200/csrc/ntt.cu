@@ -717,13 +717,12 @@ static RustError run_passes(NttBatch B, int count, const Fr* tw, int logn, bool 
     return ok();
 }
 
-// Scratch layout for one transform family: twiddles (n/2), lut_w (64), lut_c
+// Scratch layout for one transform family: twiddles (n/2), lut_c
 // (64), omega staging, (host-input variants) one data slot, then (coset
 // parts) the coset powers c^i, i < n.
 struct NttScratch {
     Fr* tw = nullptr;
     Fr* tw2 = nullptr;   // lo and hi factors of the two-level twiddle fill
-    Fr* lut_w = nullptr;
     Fr* lut_c = nullptr;
     Fr* omega = nullptr;
     Fr* data = nullptr;
@@ -736,7 +735,6 @@ static void plan_ntt(ScratchPlan& p, int log_size, bool data_slot, int log_data,
     p.add_n<Fr>(half);
     p.add_n<Fr>((1ull << TW2_LOG) + (half >> TW2_LOG) + 1);
     p.add_n<Fr>(64);
-    p.add_n<Fr>(64);
     p.add_n<Fr>(1);
     if (data_slot) p.add_n<Fr>(1ull << log_data);
     if (coset_powers) p.add_n<Fr>(1ull << log_size);
@@ -748,7 +746,6 @@ static NttScratch carve_ntt(ScratchArena& ar, int log_size, bool data_slot, int 
     uint64_t half = log_size == 0 ? 1 : (1ull << (log_size - 1));
     s.tw = ar.take_n<Fr>(half);
     s.tw2 = ar.take_n<Fr>((1ull << TW2_LOG) + (half >> TW2_LOG) + 1);
-    s.lut_w = ar.take_n<Fr>(64);
     s.lut_c = ar.take_n<Fr>(64);
     s.omega = ar.take_n<Fr>(1);
     if (data_slot) s.data = ar.take_n<Fr>(1ull << log_data);
