@@ -182,6 +182,8 @@ static uint64_t batch_slot(const h2b_msm_job* jobs, uint64_t count, uint32_t con
 extern "C" uint64_t h2b_msm_batch_workspace_size(const h2b_msm_job* jobs, uint64_t count, uint32_t streams)
 {
     if (streams == 0 || streams > EXEC_MAX_STREAMS) return 0;
+    for (uint64_t i = 0; i < count; i++)
+        if (!msm_plan_fits(job_plan(jobs[i].n, jobs[i].table_n, 1))) return 0;
     return (uint64_t)streams * batch_slot(jobs, count, batch_concurrency(count, streams));
 }
 
@@ -197,6 +199,8 @@ extern "C" RustError h2b_msm_batch(const h2b_msm_job* jobs, uint64_t count, uint
         if (!jobs[i].d_out) return err((int)cudaErrorInvalidValue, "h2b_msm_batch: null output pointer");
         if (jobs[i].table_n && jobs[i].n > jobs[i].table_n)
             return err((int)cudaErrorInvalidValue, "h2b_msm_batch: job longer than its table");
+        if (!msm_plan_fits(job_plan(jobs[i].n, jobs[i].table_n, 1)))
+            return err((int)cudaErrorInvalidValue, "h2b_msm_batch: job or table too long");
     }
     const uint32_t conc = batch_concurrency(count, streams);
     const uint64_t slot = batch_slot(jobs, count, conc);
@@ -226,12 +230,21 @@ extern "C" RustError h2b_msm_batch(const h2b_msm_job* jobs, uint64_t count, uint
 // prover commits one polynomial per `_halo2_multiexp*` call): every job must
 // name the same table (d_bases, table_n > 0); up to 64 jobs of any lengths
 // up to table_n run as one MSM whose bucket sets are the jobs'.  Results are
-// those of h2b_msm_device_table per job.
-static RustError merged_check(const h2b_msm_job* jobs, uint64_t count, uint64_t& n_total)
+// those of h2b_msm_device_table per job.  Jobs that would make 2^32 entries or
+// more between them (at 16 bits 2^28 scalars) run in groups, one after another
+// in the same scratch; a single job of a table always fits.
+namespace {
+struct MergedRun {
+    uint64_t first, count;
+    MsmPlan plan;
+};
+}  // namespace
+
+static RustError merged_runs(const h2b_msm_job* jobs, uint64_t count, MergedRun (&runs)[MSM_MERGE_MAX], uint32_t& nruns,
+                             uint64_t& scratch)
 {
     if (count == 0 || count > MSM_MERGE_MAX)
         return err((int)cudaErrorInvalidValue, "h2b_msm_merged: 1 to 64 jobs");
-    n_total = 0;
     for (uint64_t i = 0; i < count; i++) {
         if (jobs[i].table_n == 0 || jobs[i].d_bases != jobs[0].d_bases || jobs[i].table_n != jobs[0].table_n)
             return err((int)cudaErrorInvalidValue, "h2b_msm_merged: jobs must share one window table");
@@ -239,44 +252,67 @@ static RustError merged_check(const h2b_msm_job* jobs, uint64_t count, uint64_t&
             return err((int)cudaErrorInvalidValue, "h2b_msm_merged: job longer than its table");
         if (!jobs[i].d_out || (jobs[i].n > 0 && !jobs[i].d_scalars))
             return err((int)cudaErrorInvalidValue, "h2b_msm_merged: null pointer");
-        n_total += jobs[i].n;
+    }
+    nruns = 0;
+    scratch = 0;
+    for (uint64_t i = 0; i < count;) {
+        uint64_t n = 0, end = i;
+        MergedRun& r = runs[nruns];
+        while (end < count) {
+            const MsmPlan p = msm_plan_merged(std::max<uint64_t>(n + jobs[end].n, 1), jobs[0].table_n,
+                                              (uint32_t)(end - i + 1));
+            if (!msm_plan_fits(p)) break;
+            n += jobs[end++].n;
+            r.plan = p;
+        }
+        if (end == i) return err((int)cudaErrorInvalidValue, "h2b_msm_merged: table too long");
+        r.first = i;
+        r.count = end - i;
+        ScratchPlan sp;
+        msm_plan_scratch(r.plan, sp, false, false);
+        scratch = std::max(scratch, sp.used);
+        nruns++;
+        i = end;
     }
     return ok();
 }
 
 extern "C" uint64_t h2b_msm_merged_workspace_size(const h2b_msm_job* jobs, uint64_t count)
 {
-    uint64_t n_total = 0;
-    RustError e = merged_check(jobs, count, n_total);
+    MergedRun runs[MSM_MERGE_MAX];
+    uint32_t nruns = 0;
+    uint64_t need = 0;
+    RustError e = merged_runs(jobs, count, runs, nruns, need);
     if (e.code) {
         free(e.message);
         return 0;
     }
-    const MsmPlan p = msm_plan_merged(std::max<uint64_t>(n_total, 1), jobs[0].table_n, (uint32_t)count);
-    ScratchPlan sp;
-    msm_plan_scratch(p, sp, false, false);
-    return sp.used;
+    return need;
 }
 
 extern "C" RustError h2b_msm_merged(const h2b_msm_job* jobs, uint64_t count, void* scratch, uint64_t scratch_bytes,
                                     cudaStream_t stream)
 {
-    uint64_t n_total = 0;
-    H2B_TRY(merged_check(jobs, count, n_total));
-    const MsmPlan p = msm_plan_merged(std::max<uint64_t>(n_total, 1), jobs[0].table_n, (uint32_t)count);
-    ScratchPlan sp;
-    msm_plan_scratch(p, sp, false, false);
-    if (!scratch || scratch_bytes < sp.used) return scratch_too_small("h2b_msm_merged", scratch_bytes, sp.used);
-    ScratchArena ar(scratch, scratch_bytes);
-    const MsmScratch s = msm_carve(p, ar, false, false);
-    if (!ar.good()) return err((int)cudaErrorInvalidValue, "h2b_msm_merged: scratch carving failed");
-    const Fr* sc[MSM_MERGE_MAX];
-    uint64_t ns[MSM_MERGE_MAX];
-    G1Jac* outs[MSM_MERGE_MAX];
-    for (uint64_t i = 0; i < count; i++) {
-        sc[i] = (const Fr*)jobs[i].d_scalars;
-        ns[i] = jobs[i].n;
-        outs[i] = (G1Jac*)jobs[i].d_out;
+    MergedRun runs[MSM_MERGE_MAX];
+    uint32_t nruns = 0;
+    uint64_t need = 0;
+    H2B_TRY(merged_runs(jobs, count, runs, nruns, need));
+    if (!scratch || scratch_bytes < need) return scratch_too_small("h2b_msm_merged", scratch_bytes, need);
+    for (uint32_t k = 0; k < nruns; k++) {
+        const MergedRun& r = runs[k];
+        ScratchArena ar(scratch, scratch_bytes);
+        const MsmScratch s = msm_carve(r.plan, ar, false, false);
+        if (!ar.good()) return err((int)cudaErrorInvalidValue, "h2b_msm_merged: scratch carving failed");
+        const Fr* sc[MSM_MERGE_MAX];
+        uint64_t ns[MSM_MERGE_MAX];
+        G1Jac* outs[MSM_MERGE_MAX];
+        for (uint64_t i = 0; i < r.count; i++) {
+            const h2b_msm_job& j = jobs[r.first + i];
+            sc[i] = (const Fr*)j.d_scalars;
+            ns[i] = j.n;
+            outs[i] = (G1Jac*)j.d_out;
+        }
+        H2B_TRY(msm_run_merged(r.plan, s, (uint32_t)r.count, sc, ns, (const G1Affine*)jobs[0].d_bases, outs, stream));
     }
-    return msm_run_merged(p, s, (uint32_t)count, sc, ns, (const G1Affine*)jobs[0].d_bases, outs, stream);
+    return ok();
 }

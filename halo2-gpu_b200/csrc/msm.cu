@@ -41,7 +41,7 @@ extern "C" RustError h2b_exec_fork(cudaStream_t parent, uint32_t n, cudaStream_t
 namespace h2b {
 
 static constexpr int GLV_BITS = 127;
-// 32-bit sorted-entry offsets: 2 halves x 8 windows x n < 2^32
+// longest MSM: 2 halves x 8 windows x n entries stay below 2^32 (msm_plan_fits)
 static constexpr uint64_t MSM_MAX_LENGTH = 1ull << 27;
 static constexpr uint32_t SIGN_BIT = 0x80000000u;
 // widest window the tuning override accepts (22 bits: 6 windows per GLV half)
@@ -86,9 +86,18 @@ static int floor_log2(uint64_t n)
     return lg;
 }
 
-// `plain`: an MSM over plain bases, whose window width may come from the
-// per-size tuning table; a window table's width is fixed when it is built.
-static int choose_c(uint64_t n, bool plain = false)
+// Windows of c bits over the GLV halves (magnitudes < 2^GLV_BITS); the top one
+// must leave room for the signed-digit carry (its width <= c - 1).
+static int window_count(int c)
+{
+    const int W = (GLV_BITS + c - 1) / c;
+    return GLV_BITS - c * (W - 1) > c - 1 ? W + 1 : W;
+}
+
+// The width an MSM over n points would like, before widen_c.  `plain`: over
+// plain bases, whose window width may come from the per-size tuning table; a
+// window table's width is fixed when it is built.
+static int wanted_c(uint64_t n, bool plain = false)
 {
     const int lg = floor_log2(n);
     if (g_msm_window_override >= 4 && g_msm_window_override <= MSM_MAX_WINDOW) return g_msm_window_override;
@@ -122,6 +131,16 @@ static int choose_c(uint64_t n, bool plain = false)
     return 7;
 }
 
+// A width set by hand can be too narrow for the 32-bit entry count (4 bits
+// from 2^26 points on): plain bases then take the next one that fits.  A table
+// keeps the width it was built with, at which table_fits holds.
+static int choose_c(uint64_t n, bool plain = false)
+{
+    int c = wanted_c(n, plain);
+    while (plain && c < MSM_MAX_WINDOW && 2 * n * (uint64_t)window_count(c) >= (1ull << 32)) c++;
+    return c;
+}
+
 // tn > 0: precomputed window table of tn points per window; all windows then
 // share one bucket set and the reduction has a single window (one per job of
 // a merged run).
@@ -131,10 +150,7 @@ static MsmPlan plan_core(uint64_t n, int c, uint64_t tn, uint32_t concurrent = 1
     p.n = n;
     p.tn = tn;
     p.c = c;
-    // GLV halves: magnitudes < 2^GLV_BITS; the top window must leave room
-    // for the signed-digit carry (its width <= c - 1).
-    p.W = (GLV_BITS + c - 1) / c;
-    if (GLV_BITS - c * (p.W - 1) > c - 1) p.W++;
+    p.W = window_count(c);
     p.H = 1u << (c - 1);
     p.Wr = tn ? (int)jobs : p.W;
     p.NB = (uint64_t)p.Wr * p.H;

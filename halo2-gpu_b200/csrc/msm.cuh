@@ -71,6 +71,13 @@ RustError msm_run(const MsmPlan& p, const MsmScratch& s, const Fr* d_scalars, co
 // bucket set j; each job's 96-byte result goes to outs[j].
 constexpr uint32_t MSM_MERGE_MAX = 64;
 MsmPlan msm_plan_merged(uint64_t n_total, uint64_t tn, uint32_t J);
+// Bucket offsets, scatter cursors and chunk starts count sorted entries in 32
+// bits, and an entry names its point in 31.
+inline bool msm_plan_fits(const MsmPlan& p)
+{
+    return p.n < (1ull << 30) && p.max_entries < (1ull << 32) && p.tn < (1ull << 30) &&
+           2 * (uint64_t)p.W * p.tn < (1ull << 31);
+}
 RustError msm_run_merged(const MsmPlan& p, const MsmScratch& s, uint32_t J, const Fr* const* scalars,
                          const uint64_t* ns, const G1Affine* table, G1Jac* const* outs, cudaStream_t st);
 void msm_set_tuning(int window_bits, int chunk);

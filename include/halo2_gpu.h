@@ -460,8 +460,9 @@ RustError _halo2_quotient_permutation(void* values, const void* l0, const void* 
  * result to d_out on `stream` without synchronising. */
 RustError h2b_msm_device(const void* d_scalar, const void* d_bases, void* d_out, uint64_t length, void* scratch,
                          uint64_t scratch_bytes, h2b_stream_t stream);
-/* Window bits (0 = automatic; 4..22 accepted, other values also mean automatic) and sorted entries per
- * accumulation chunk (0 = automatic). */
+/* Window bits (0 = automatic; 4..22 accepted, other values also mean automatic; an MSM over plain bases
+ * takes the next width that keeps its digits below 2^32) and sorted entries per accumulation chunk (0 =
+ * automatic). */
 void h2b_msm_set_tuning(int window_bits, int chunk);
 /* Form of the MSM bucket-accumulation kernel: 6 = coordinates below 2p as eight 32-bit words, products in
  * even and odd word rows (default); 0 = lazy R = 2^261 limbs of 29 bits with one-step carries (its workspace
@@ -518,8 +519,9 @@ RustError h2b_msm_batch(const h2b_msm_job* jobs, uint64_t count, uint32_t stream
  * differ, each <= table_n) run as one MSM: one counting sort with job j's entries in bucket set j, one
  * accumulation, one bucket reduction, one final kernel writing each job's 96-byte result to its d_out.
  * Same results as h2b_msm_device_table per job (no counterpart in the reference, which commits one
- * polynomial per _halo2_multiexp* call).  Scratch: h2b_msm_merged_workspace_size (0 if the jobs do not
- * qualify).  No host synchronisation; device outputs. */
+ * polynomial per _halo2_multiexp* call).  Jobs of 2^32 digits or more between them (2^28 scalars over a
+ * 16-bit table) run in groups, one after another.  Scratch: h2b_msm_merged_workspace_size (0 if the jobs do
+ * not qualify).  No host synchronisation; device outputs. */
 uint64_t h2b_msm_merged_workspace_size(const h2b_msm_job* jobs, uint64_t count);
 RustError h2b_msm_merged(const h2b_msm_job* jobs, uint64_t count, void* scratch, uint64_t scratch_bytes,
                          h2b_stream_t stream);

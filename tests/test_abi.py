@@ -176,3 +176,38 @@ def test_fused_quotient_and_merged_msm_reject_on_the_host(h2b, built_lib):
     bad(L.h2b_msm_merged(jobs, 2, fake[30], 1 << 30, None), "job longer than its table")
     jobs[1].n = 8
     bad(L.h2b_msm_merged(jobs, 2, fake[30], 16, None), "h2b_msm_merged")      # scratch too small
+
+
+def test_msm_entries_stay_below_32_bits(h2b, built_lib):
+    """Bucket offsets and chunk starts are 32-bit, so no plan may make 2^32
+    digits: merged jobs beyond that run in groups (their scratch is that of the
+    largest group), and plain bases take a wider window than the one set by
+    hand.  Pure host; the pointers are stand-ins."""
+    L = built_lib
+    fake = [ctypes.c_void_p(0x10000 + 0x1000 * i) for i in range(3)]
+
+    def merged_ws(count, n):
+        jobs = (h2b.MsmJob * count)()
+        for j in jobs:
+            j.d_scalars, j.d_bases, j.d_out, j.n, j.table_n = fake[0], fake[1], fake[2], n, n
+        return L.h2b_msm_merged_workspace_size(jobs, count)
+
+    n = 1 << 23                                        # 16-bit windows: 2 x 8 digits a scalar
+    assert merged_ws(30, n) < merged_ws(31, n)
+    assert merged_ws(32, n) == merged_ws(64, n) == merged_ws(31, n)       # 32 n digits x 16 = 2^32
+    assert merged_ws(64, n // 4) > merged_ws(63, n // 4)
+    # no table of 2^27 points can be built, so none can be used
+    assert merged_ws(1, 1 << 27) == 0
+    job = (h2b.MsmJob * 1)()
+    job[0].d_scalars, job[0].d_bases, job[0].d_out, job[0].n, job[0].table_n = *fake, 1 << 30, 0
+    assert L.h2b_msm_batch_workspace_size(job, 1, 1) == 0
+    try:
+        for c, length, got in ((4, (1 << 26) - 1, 4), (4, 1 << 26, 5), (4, 1 << 27, 9), (8, 1 << 27, 9),
+                               (9, 1 << 27, 9), (16, 1 << 27, 16)):
+            L.h2b_msm_set_tuning(c, 0)
+            assert L.h2b_msm_window_bits(length) == got, (c, length)
+            windows = (127 + got - 1) // got
+            windows += 127 - got * (windows - 1) > got - 1
+            assert 2 * windows * length < 1 << 32
+    finally:
+        L.h2b_msm_set_tuning(0, 0)

@@ -163,6 +163,35 @@ def test_merged_64_jobs_k16_match_the_batch(h2b, cuda):
     assert [_bytes(o) for o in outs_m] == [_bytes(o) for o in outs_b]
 
 
+def test_merged_jobs_in_groups(h2b, cuda):
+    """64 jobs of 2^20 scalars at 4-bit windows make 2^32 digits, which run as
+    a group of 63 and one job: the bytes of h2b_msm_device_table on both sides
+    of the cut."""
+    L = h2b.lib()
+    n = 1 << 20
+    try:
+        L.h2b_msm_set_tuning(4, 0)
+        table = h2b.msm_table_precompute(h2b.srs_device(0x6409, n), n)
+        scs = [torch.zeros(32 * n, dtype=torch.uint8, device="cuda") for _ in range(2)]
+        for i, sc in enumerate(scs):
+            sc.view(n, 32)[i::4099] = h2b.random_fr_device(len(range(i, n, 4099)), 61 + i, 0).view(-1, 32)
+        which = [i % 2 for i in range(64)]
+        outs = [h2b.dev_empty(96) for _ in which]
+        jobs = h2b.msm_batch_jobs([scs[w] for w in which], [table] * 64, outs, [n] * 64, table_n=n)
+        need = h2b.msm_merged_workspace_bytes(jobs, 64)
+        assert need == h2b.msm_merged_workspace_bytes(jobs, 63)
+        h2b.msm_merged(jobs, 64, h2b.dev_empty(need))
+        want = []
+        for sc in scs:
+            one = h2b.dev_empty(96)
+            h2b.msm_device_table(sc, table, n, one, n)
+            want.append(_bytes(one))
+        assert want[0] != want[1]
+        assert [_bytes(o) for o in outs] == [want[w] for w in which]
+    finally:
+        L.h2b_msm_set_tuning(0, 0)
+
+
 def test_merged_argument_errors(h2b, cuda, table4k):
     srs, d_srs, table = table4k
     tn = 1 << 12
