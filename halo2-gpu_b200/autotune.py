@@ -8,10 +8,11 @@ Here those choices are entries of a table inside libhalo2_gpu.so
 times candidate settings on the GPU it runs on and keeps the fastest:
 
 * op "msm", k = log2 of the MSM length: the signed-digit window width
-  (automatic width - 1, automatic, + 1, within 10..16), then the sorted
-  entries per accumulation chunk (automatic, 32, 64, 128, 256) at the chosen
-  width.  Timed on the witness-like scalar mix (50 % uniform, 30 % < 2^64,
-  20 % {0, 1}) over a prefix of a synthetic SRS.
+  (automatic width - 1, automatic, + 1, within 10..16; below 2^14 points,
+  where 8 bits is automatic, 8, 10, 11, 12 and 13), then the sorted entries
+  per accumulation chunk (automatic, 32, 64, 128, 256) at the chosen width.
+  Timed on the witness-like scalar mix (50 % uniform, 30 % < 2^64, 20 %
+  {0, 1}) over a prefix of a synthetic SRS.
 * op "ntt", k = log2 of the transform size: stages per shared-memory pass
   (6..11; 11 only with the radix-4 pass kernel, whose tiles hold 2^11
   elements), timed on a forward FFT of uniform random coefficients; the
@@ -36,6 +37,10 @@ import statistics
 
 PARAM_WINDOW, PARAM_CHUNK, PARAM_STAGES = 0, 1, 2
 WINDOW_RANGE = (10, 16)
+# instead of the automatic width's neighbours below 2^14 points: 7 and 9 bits
+# leave one bit of the 127 to a window of its own, whose bucket holds half of
+# all entries
+SMALL_WINDOWS = (8, 10, 11, 12, 13)
 CHUNK_CANDIDATES = (0, 32, 64, 128, 256)
 STAGE_CANDIDATES = (6, 7, 8, 9, 10, 11)
 CACHE_VERSION = 1
@@ -91,6 +96,8 @@ def pick(timings, auto, margin=0.01):
 
 def window_candidates(auto_c):
     lo, hi = WINDOW_RANGE
+    if auto_c < lo:
+        return list(SMALL_WINDOWS)
     return [c for c in (auto_c - 1, auto_c, auto_c + 1) if lo <= c <= hi]
 
 

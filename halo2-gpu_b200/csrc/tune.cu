@@ -20,11 +20,12 @@ constexpr int TUNE_PARAMS = 3;   // 0 MSM window bits, 1 MSM chunk entries, 2 NT
 constexpr int TUNE_MAX_LOG = 32;
 static std::atomic<int> g_tune[TUNE_PARAMS][TUNE_MAX_LOG + 1];
 
-static bool tune_valid(uint32_t param, int32_t v)
+static bool tune_valid(uint32_t param, uint32_t log_n, int32_t v)
 {
     if (v == 0) return true;
     switch (param) {
-    case 0: return v >= 10 && v <= 16;   // windows the default plans also use (sizes 2^10 .. 2^27)
+    // the widths that plain MSMs use by themselves: 8 bits below 2^14 points, 13 and 16 above
+    case 0: return v >= (log_n < 14 ? 8 : 10) && v <= 16;
     case 1: return v >= 8 && v <= 512;   // sorted entries per accumulation thread
     case 2: return v >= 1 && v <= 11;    // radix-2 stages per shared-memory pass (11: radix-4 passes only)
     default: return false;
@@ -41,7 +42,7 @@ int tune_value(int param, int log_n)
 
 extern "C" int32_t h2b_tune_set(uint32_t param, uint32_t log_n, int32_t value)
 {
-    if (param >= (uint32_t)h2b::TUNE_PARAMS || log_n > (uint32_t)h2b::TUNE_MAX_LOG || !h2b::tune_valid(param, value))
+    if (param >= (uint32_t)h2b::TUNE_PARAMS || log_n > (uint32_t)h2b::TUNE_MAX_LOG || !h2b::tune_valid(param, log_n, value))
         return -1;
     h2b::g_tune[param][log_n].store(value, std::memory_order_relaxed);
     return 0;

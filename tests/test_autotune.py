@@ -95,6 +95,32 @@ def test_table_drives_plain_msm_plan_only(clean_table):
     assert L._halo2_multiexp_device_scalars_device_bases_workspace_size(n) == ws_auto
 
 
+@pytest.mark.parametrize("k", [10, 11, 12, 13, 14, 18, 19, 22])
+def test_built_in_width_has_rivals(at, clean_table, k):
+    """At every size the tuner compares the built-in width with others, and the
+    table takes each of them (the built-in one too)."""
+    L = clean_table
+    auto = L.h2b_msm_window_bits(1 << k)
+    cands = at.window_candidates(auto)
+    assert auto in cands and len(cands) >= 2
+    for c in cands:
+        assert L.h2b_tune_set(0, k, c) == 0 and L.h2b_msm_window_bits(1 << k) == c
+    assert L.h2b_tune_set(0, k, 9 if k >= 14 else 7) == -1
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("c", [8, 9])
+def test_narrow_msm_settings_are_bit_exact(h2b, orc, cuda, clean_table, c):
+    n = 1500
+    bases = orc.srs(h2b.fields.fr_mont_limbs([0x5154]), n)
+    sc = orc.chacha_fr(0x5155, n)
+    d_b, d_s = h2b.to_dev(bases), h2b.to_dev(sc)
+    for chunk in (0, 8, 256):
+        assert clean_table.h2b_tune_set(0, 10, c) == 0 and clean_table.h2b_tune_set(1, 10, chunk) == 0
+        got = h2b.multiexp_gpu_device_scalars_device_bases(d_s, d_b, n)
+        assert_limbs_equal(got, orc.msm(sc, bases), f"window {c} chunk {chunk}")
+
+
 @pytest.mark.gpu
 def test_every_msm_setting_is_bit_exact(h2b, orc, cuda, clean_table):
     L = clean_table
