@@ -796,7 +796,7 @@ struct MsmFold {
 __global__ void __launch_bounds__(32) k_msm_tail(G1Xyzz* sums, uint32_t per, MsmFold f, int c, uint32_t leaves,
                                                  uint32_t* ctr, const __grid_constant__ MsmOuts outs)
 {
-    __shared__ Fq sl[20];
+    __shared__ __align__(16) Fq sl[20];   // read and written as uint4
     const int lane = (int)threadIdx.x;
     const uint32_t group = blockIdx.x / leaves;
     uint32_t i = blockIdx.x % leaves;
