@@ -1096,10 +1096,14 @@ H2B_DEV Fp<C> canon2p(const Fp<C>& a)
     return r;
 }
 
-// operator* and fsqr.  One out-of-line body per field by default: kernels that
-// chain many products (curve formulas, the quotient interpreter) otherwise
-// inline hundreds of instructions per product and starve on instruction
-// fetch.  H2B_INLINE_MUL=1 restores full inlining for kernels that want it.
+// operator* and fsqr.  The first factor must be below 2^256 - p (4.29 p; every
+// canonical residue and every value below 2p is): beyond it a carry out of the
+// ninth word is dropped.  The second may be any 256-bit value, and the product
+// is canonical when the first is, so a value that comes from outside as it is
+// (a caller's element, random words) stands second.
+// One out-of-line body per field by default: kernels that chain many products
+// (curve formulas) would inline two hundred instructions per product.
+// H2B_INLINE_MUL=1 inlines them in a file.
 #ifndef H2B_INLINE_MUL
 #define H2B_INLINE_MUL 0
 #endif
@@ -1239,16 +1243,17 @@ H2B_DEV Fp<C> fsqr(const Fp<C>& a)
 #endif
 }
 
-// Montgomery residue -> canonical integer (multiply by 1).
+// Montgomery residue (any 256-bit value of its class) -> canonical integer (multiply by 1).
 template <class C>
 H2B_DEV Fp<C> from_mont(const Fp<C>& a)
 {
     Fp<C> one_int = Fp<C>::zero();
     one_int.v[0] = 1;
-    return a * one_int;
+    return one_int * a;
 }
+// any 256-bit integer -> its residue
 template <class C>
-H2B_DEV Fp<C> to_mont(const Fp<C>& a) { return a * Fp<C>::r2(); }
+H2B_DEV Fp<C> to_mont(const Fp<C>& a) { return Fp<C>::r2() * a; }
 
 template <class C>
 H2B_DEV Fp<C> ldg(const Fp<C>* p)

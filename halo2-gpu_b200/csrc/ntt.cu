@@ -169,8 +169,8 @@ __device__ __forceinline__ Fr twist_in(const Fr* __restrict__ in, uint64_t i, ui
 {
     if (i >= n_in) return Fr::zero();
     const Fr v = ldg(&in[i]);
-    if (mode == 1) return v * ldg(&cpow[i]);
-    if (mode == 2) return v * zeta_pick(z3, i);
+    if (mode == 1) return ldg(&cpow[i]) * v;
+    if (mode == 2) return zeta_pick(z3, i) * v;
     return v;
 }
 __global__ void k_twist_bitrev_stage0(NttBatch B, uint64_t n_in, int log_out, int mode,
@@ -206,7 +206,7 @@ __global__ void k_coset_spread(NttBatch B, int log_in, int e, Zeta3 z3)
     for (uint64_t r = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; r < n_in;
          r += (uint64_t)gridDim.x * blockDim.x) {
         const uint64_t i = bitrev(r, log_in);
-        Fr v = ldg(&in[i]) * zeta_pick(z3, i);
+        Fr v = zeta_pick(z3, i) * ldg(&in[i]);
         Fr* dst = out + (r << e);
         for (uint64_t j = 0; j < g; j++) st(&dst[j], v);
     }
@@ -223,7 +223,7 @@ __global__ void k_twist_inplace(NttBatch B, uint64_t n, int mode, const Fr* __re
         for (int j = 0; j < SC_CHUNK && i0 + j < n; j++) {
             uint64_t i = i0 + j;
             Fr v = ld(&a[i]);
-            v = v * (mode == 1 ? ldg(&cpow[i]) : zeta_pick(z3, i));
+            v = (mode == 1 ? ldg(&cpow[i]) : zeta_pick(z3, i)) * v;
             st(&a[i], v);
         }
     }

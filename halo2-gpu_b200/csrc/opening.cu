@@ -405,7 +405,7 @@ static __global__ void __launch_bounds__(KD_T, 2) k_kd0_up(KdLevel L, const Fr* 
 #pragma unroll
     for (int k = 0; k < KD_E; k++) {
         const uint64_t t = t0 + k;
-        y[k] = t < L.m ? ld(&a[L.n - 1 - t]) * ldg(&W[c * KD_E + k]) : Fr::zero();
+        y[k] = t < L.m ? ldg(&W[c * KD_E + k]) * ld(&a[L.n - 1 - t]) : Fr::zero();
     }
 #pragma unroll
     for (int k = 1; k < KD_E; k++) y[k] = y[k] + y[k - 1];

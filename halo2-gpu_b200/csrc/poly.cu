@@ -34,7 +34,7 @@ __global__ void k_extended_from_parts(Fr* __restrict__ out, const Fr* const* __r
 
 __global__ void k_divide_by_vanishing(Fr* __restrict__ a, const Fr* __restrict__ t, uint32_t tl, uint64_t n)
 {
-    H2B_GRID_STRIDE(i, n) { st(&a[i], ld(&a[i]) * ldg(&t[i % tl])); }
+    H2B_GRID_STRIDE(i, n) { st(&a[i], ldg(&t[i % tl]) * ld(&a[i])); }
 }
 
 __global__ void k_distribute_powers(Fr* __restrict__ a, const Fr* __restrict__ c, uint32_t L, uint64_t n)
@@ -43,13 +43,13 @@ __global__ void k_distribute_powers(Fr* __restrict__ a, const Fr* __restrict__ c
     H2B_GRID_STRIDE(i, n)
     {
         uint32_t r = (uint32_t)(i % mod);
-        if (r != 0) st(&a[i], ld(&a[i]) * ldg(&c[r - 1]));
+        if (r != 0) st(&a[i], ldg(&c[r - 1]) * ld(&a[i]));
     }
 }
 
 __global__ void k_mul(Fr* out, const Fr* a, const Fr* b, uint64_t n)
 {
-    H2B_GRID_STRIDE(i, n) { st(&out[i], ld(&a[i]) * ld(&b[i])); }
+    H2B_GRID_STRIDE(i, n) { st(&out[i], canon2p<FrCfg>(ld(&a[i])) * ld(&b[i])); }
 }
 
 __global__ void k_fill_one(Fr* __restrict__ out, uint64_t n)
@@ -60,7 +60,7 @@ __global__ void k_fill_one(Fr* __restrict__ out, uint64_t n)
 __global__ void k_mul_add(Fr* __restrict__ acc, const Fr* __restrict__ in, const Fr* __restrict__ s, uint64_t n)
 {
     const Fr k = ld(s);
-    H2B_GRID_STRIDE(i, n) { st(&acc[i], ld(&acc[i]) + ld(&in[i]) * k); }
+    H2B_GRID_STRIDE(i, n) { st(&acc[i], ld(&acc[i]) + k * ld(&in[i])); }
 }
 
 __global__ void k_sub_short(Fr* __restrict__ acc, const Fr* __restrict__ sh, uint64_t n)

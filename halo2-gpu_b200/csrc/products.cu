@@ -473,7 +473,7 @@ __global__ void __launch_bounds__(PR_T) k_permutation_product(Fr* __restrict__ a
         base, n, nullptr,
         [&](uint64_t i) {
             Fr x = ld(&acc[i]);
-            for (int c = 0; c < ncols; c++) x = x * (beta * ld(&cols.sigma[c][i]) + gamma + ld(&cols.value[c][i]));
+            for (int c = 0; c < ncols; c++) x = (beta * ld(&cols.sigma[c][i]) + gamma + ld(&cols.value[c][i])) * x;
             st(&acc[i], x);
             return x;
         },
@@ -536,7 +536,7 @@ __global__ void k_pp_accumulate(Fr* __restrict__ den, Fr* __restrict__ num, cons
         for (int j = 0; j < PP_CHUNK && i0 + j < n; j++) {
             uint64_t i = i0 + j;
             Fr v = ld(&value[i]);
-            st(&den[i], ld(&den[i]) * (beta * ld(&sigma[i]) + gamma + v));
+            st(&den[i], (beta * ld(&sigma[i]) + gamma + v) * ld(&den[i]));
             Fr f = cur * beta + gamma + v;
             st(&num[i], first ? f : ld(&num[i]) * f);
             cur = cur * omega;
@@ -652,7 +652,7 @@ __global__ void k_bia_apply(BiaCols cols, uint64_t n, AssignedRec L, const Fr* _
     for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < n; i += (uint64_t)gridDim.x * blockDim.x) {
         const uint8_t* rec = raw + i * L.stride_bytes;
         Fr v = Fr::zero();
-        if (rec[0] != 0) v = ld_words_fr(rec + L.num_offset) * ld(&inv[c * n + i]);
+        if (rec[0] != 0) v = ld(&inv[c * n + i]) * ld_words_fr(rec + L.num_offset);
         st(&out[i], v);
     }
 }

@@ -10,8 +10,11 @@
  *
  * Conventions (halo2_proofs/cuda/include/common/halo2_ffi.h:1-62):
  *  - Field elements are 32-byte Montgomery-form BN254 Fr/Fq, little-endian
- *    64-bit limbs (the halo2curves memory image).  G1 affine points are 64
- *    bytes {x, y}, infinity = (0, 0).  MSM results are the 96-byte Jacobian
+ *    64-bit limbs (the halo2curves memory image), canonical: below the modulus.
+ *    MSM scalars and the inputs of the entries that first multiply each element
+ *    by a factor of their own (the forward coset transforms, Kate division, the
+ *    element-wise products) may be any 256-bit value of the class.  G1 affine
+ *    points are 64 bytes {x, y}, infinity = (0, 0).  MSM results are the 96-byte Jacobian
  *    image {X, Y, Z} with Z = 1, or (0, 1, 0) for infinity.
  *  - `void*` arguments named d_* are device pointers; FFITraitObject carries a
  *    host or device address as documented per entry.
