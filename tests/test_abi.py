@@ -211,3 +211,16 @@ def test_msm_entries_stay_below_32_bits(h2b, built_lib):
             assert 2 * windows * length < 1 << 32
     finally:
         L.h2b_msm_set_tuning(0, 0)
+
+
+def test_settings_that_are_not_built_change_nothing(h2b, built_lib):
+    """Accumulation forms other than 0 and 6 and batch-affine pairing rounds are
+    not built: their setters leave the setting as it is."""
+    L = built_lib
+    before = L.h2b_msm_get_accumulate_variant()
+    for v in (1, 5, 7, -1):
+        L.h2b_msm_set_accumulate_variant(v)
+        assert L.h2b_msm_get_accumulate_variant() == before == 6
+    for rounds in (1, 3):
+        L.h2b_msm_set_pair_rounds(rounds)
+        assert L.h2b_msm_get_pair_rounds() == 0

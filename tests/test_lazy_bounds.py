@@ -1,12 +1,10 @@
-"""The value bounds behind the lazy accumulation forms (csrc/lazy.cuh with
-csrc/curve.cuh xyzzz_madd / xyzzz_dbl_affine, R = 2^261; csrc/lazy64.cuh with
-xyzzd_madd / xyzzd_dbl_affine, R' = 2^260), re-derived with exact rational
-arithmetic: every subtraction a - b + K p must see b below (K - 0.001) p,
+"""The value bounds behind the lazy accumulation form (csrc/lazy.cuh with
+csrc/curve.cuh xyzzz_madd / xyzzz_dbl_affine, R = 2^261), re-derived with exact
+rational arithmetic: every subtraction a - b + K p must see b below (K - 0.001) p,
 every product input must keep the column sums exact, and the accumulator
-bounds (R = 2^261: X < 5.39p, Y < 3.34p, ZZ, ZZZ < 2p; R' = 2^260: X < 5.4p,
-Y < 3.45p, ZZ, ZZZ < 1.2p) must be stable from one addition to the next.
-Also checks the borrow-adjusted K p limbs of the 29-bit form and the K p
-limbs of the 52-bit form."""
+bounds (X < 5.39p, Y < 3.34p, ZZ, ZZZ < 2p) must be stable from one addition to
+the next.  Also checks the borrow-adjusted K p limbs, and the residues below 2p
+that the NTT passes and the default accumulation keep."""
 from fractions import Fraction as Q
 
 P = 0x30644E72E131A029B85045B68181585D97816A916871CA8D3C208C16D87CFD47
@@ -14,12 +12,8 @@ R = 1 << 261
 EPS = Q(P, R)                   # product of a p and b p is below (1 + EPS a b) p
 
 
-EPS_260 = Q(P, 1 << 260)        # the FP64 form's R'
-_eps = [EPS]
-
-
 def mul(a, b):
-    return 1 + _eps[0] * a * b
+    return 1 + EPS * a * b
 
 
 def sub(a, b, K):
@@ -102,50 +96,19 @@ def test_column_sums_fit_64_bits():
     assert _p29(8) < (1 << 29)
 
 
-def test_fp64_form_bounds_are_stable():
-    _eps[0] = EPS_260
-    try:
-        qx, qy = Q(1), Q(2)              # canonical (halved from the stored form); negated 2p - y
-        B = (Q(54, 10), Q(345, 100), Q(12, 10), Q(12, 10))
-        X3, Y3, ZZ3, ZZZ3, inner = madd(*B, qx, qy)
-        assert all(a <= b for a, b in zip((X3, Y3, ZZ3, ZZZ3), B))
-        assert qx <= B[0] and qy <= B[1]  # the infinity start (acc = q, ZZ = ZZZ = 1)
-        assert max(inner) < Q(72, 10)     # largest product input, below 2^257 / p
-        assert max(inner) * P < 1 << 257
-        dX, dY, dZZ, dZZZ = dbl_affine(qx, qy)
-        assert dX <= B[0] and dY <= B[1] and dZZ <= B[2] and dZZZ <= B[3]
-        assert mul(B[0], 1) < 2          # the store product by 2^256 mod p
-    finally:
-        _eps[0] = EPS
-
-
-def _p52(i):
-    return (P >> (52 * i)) & ((1 << 52) - 1)
-
-
-def test_fp64_form_limbs():
-    # K p in the 52-bit grid (kp52): normalised, the top limb holding the rest
-    for K in (2, 3, 4, 5, 6):
-        limbs = [((K * P) >> (52 * i)) & ((1 << 52) - 1) if i < 4 else (K * P) >> 208 for i in range(5)]
-        assert sum(l << (52 * i) for i, l in enumerate(limbs)) == K * P
-        assert limbs[4] < 1 << 52
-    # every lazy value stays below 2^257, so its top limb is below 2^49 and
-    # the signed limb sums of a - b + K p stay far inside 64 bits
-    assert 8 * P < 1 << 257
-    assert sum(_p52(i) << (52 * i) for i in range(5)) == P
-
-
 def test_ntt_residues_below_2p():
-    """The radix-4 NTT pass keeps values in [0, 2p) (field.cuh: mont_mul_f64_lazy,
-    add2p, sub2p, canon2p): for both BN254 moduli a product of operands below
-    2p leaves (16 a b + Q p) / 2^260 < (64 p / 2^260 + 1) p < 1.76 p < 2p
-    (Q < 2^260), a sum of two such values is below 4p < 2^256 (no carry out of
+    """The radix-4 NTT pass and the MSM keep values in [0, 2p) (field.cuh:
+    mont_mul_eo_lazy, add2p, sub2p, canon2p): for both BN254 moduli a product of
+    operands below 2p leaves (a b + Q p) / 2^256 < (4 p / 2^256 + 1) p < 1.76 p
+    (Q < 2^256), the sum of two such products less than 2.52 p, which one
+    subtraction of 2p brings below 2p, a sum of two such values is below 4p < 2^256 (no carry out of
     the 8 words), one subtraction of 2p brings a sum or a borrowed difference
     back below 2p, and one subtraction of p makes a value below 2p canonical.
     Exhaustive over the interval ends with exact integers."""
     r = 0x30644E72E131A029B85045B68181585D2833E84879B9709143E1F593F0000001
     for m in (P, r):
-        assert Q(64 * m, 1 << 260) + 1 < Q(176, 100)
+        assert Q(4 * m, 1 << 256) + 1 < Q(176, 100)
+        assert Q(8 * m, 1 << 256) + 1 < Q(252, 100)
         assert 4 * m < 1 << 256
         two = 2 * m
         words = [(two >> (32 * w)) & 0xFFFFFFFF for w in range(8)]

@@ -216,10 +216,10 @@ def test_merged_argument_errors(h2b, cuda, table4k):
         h2b.msm_merged(ok, 1, h2b.dev_empty(need - 256))
 
 
-def test_wide_windows_split_bit_sums(h2b, orc, cuda):
-    """Window widths 17-19 give bucket reductions whose bit sums span more
-    than 4096 segment sums, split over several CTAs and summed by a second
-    kernel: a table MSM and a plain MSM at those widths equal the oracle."""
+def test_wide_windows(h2b, orc, cuda):
+    """Window widths whose bucket reduction folds in three passes (17, 19 bits)
+    and in four (22, the widest): a table MSM and a plain MSM at those widths
+    equal the oracle."""
     L = h2b.lib()
     n = 1 << 12
     tau = h2b.fields.fr_mont_limbs([0x51DE])
@@ -230,7 +230,7 @@ def test_wide_windows_split_bit_sums(h2b, orc, cuda):
     want = orc.msm(sc, srs)
     d_sc = h2b.to_dev(sc)
     try:
-        for c in (17, 19):
+        for c in (17, 19, 22):
             L.h2b_msm_set_tuning(c, 0)
             assert L.h2b_msm_window_bits(n) == c
             table = h2b.msm_table_precompute(d_srs, n)
