@@ -305,80 +305,16 @@ H2B_DEV Fp<C> from_l(const Fl<C>& a)
     return r;
 }
 
-// Column sums T_k = sum_{i+j=k} a_i b_j (k < 17) of two 9-limb operands by
-// one Karatsuba step (5 + 4 limbs): z0 = a0 b0 and z2 = a1 b1 schoolbook,
-// the middle term as (a0 + a1)(b0 + b1) - z0 - z2 with 30-bit limb sums, so 66
-// limb products instead of 81.  Every column is the exact integer sum
-// (no carries between columns), so the reduction that consumes them is
-// unchanged.  Bounds: limbs below 2^29 + 8 give sums below 2^30.1, middle
-// products below 2^60.1, five of them below 2^62.5.
-// Off by default: measured on B200 it is slower despite the fewer multiplies
-// (MSM at 2^22 13.59 -> 13.92 ms, 8 coset parts at 2^22 12.98 -> 13.28 ms, 8
-// inverse NTTs 14.31 -> 15.80 ms): the limb sums, the 64-bit column
-// subtractions and the extra live registers cost more than the 15 products,
-// and the interleaved product-scanning form overlaps better.
-#ifndef H2B_MUL_KARATSUBA
-#define H2B_MUL_KARATSUBA 0
-#endif
-H2B_DEV void kcols29(const uint32_t (&a)[9], const uint32_t (&b)[9], uint64_t (&T)[17])
-{
-    uint32_t sa[5], sb[5];
-#pragma unroll
-    for (int i = 0; i < 5; i++) {
-        sa[i] = a[i] + (i < 4 ? a[5 + i] : 0u);
-        sb[i] = b[i] + (i < 4 ? b[5 + i] : 0u);
-    }
-#pragma unroll
-    for (int k = 0; k < 17; k++) T[k] = 0;
-    uint64_t z0[9], z2[7];
-#pragma unroll
-    for (int k = 0; k < 9; k++) {
-        uint64_t acc = 0;
-#pragma unroll
-        for (int i = 0; i < 5; i++)
-            if (k - i >= 0 && k - i < 5) acc = madw(a[i], b[k - i], acc);
-        z0[k] = acc;
-    }
-#pragma unroll
-    for (int k = 0; k < 7; k++) {
-        uint64_t acc = 0;
-#pragma unroll
-        for (int i = 0; i < 4; i++)
-            if (k - i >= 0 && k - i < 4) acc = madw(a[5 + i], b[5 + k - i], acc);
-        z2[k] = acc;
-    }
-#pragma unroll
-    for (int k = 0; k < 9; k++) {
-        uint64_t acc = 0;
-#pragma unroll
-        for (int i = 0; i < 5; i++)
-            if (k - i >= 0 && k - i < 5) acc = madw(sa[i], sb[k - i], acc);
-        acc -= z0[k];
-        if (k < 7) acc -= z2[k];
-        T[k] += z0[k];
-        T[k + 5] += acc;
-        if (k < 7) T[k + 10] += z2[k];
-    }
-}
-
 template <class C>
 H2B_DEV Fl<C> mul29(const Fl<C>& a, const Fl<C>& b)
 {
-#if H2B_MUL_KARATSUBA
-    uint64_t T[17];
-    kcols29(a.l, b.l, T);
-#endif
     const uint32_t np = C::N0 & M29;
     uint32_t m[9];
     uint64_t acc = 0;
 #pragma unroll
     for (int k = 0; k < 9; k++) {
-#if H2B_MUL_KARATSUBA
-        acc += T[k];
-#else
 #pragma unroll
         for (int i = 0; i <= k; i++) acc = madw(a.l[i], b.l[k - i], acc);
-#endif
 #pragma unroll
         for (int i = 0; i < k; i++) acc = madw(m[i], p29<C>(k - i), acc);
         const uint32_t mk = ((uint32_t)acc * np) & (k < 8 ? M29 : 0xffffffu);
@@ -392,12 +328,8 @@ H2B_DEV Fl<C> mul29(const Fl<C>& a, const Fl<C>& b)
     uint32_t h[9];
 #pragma unroll
     for (int k = 9; k < 17; k++) {
-#if H2B_MUL_KARATSUBA
-        acc += T[k];
-#else
 #pragma unroll
         for (int i = k - 8; i <= 8; i++) acc = madw(a.l[i], b.l[k - i], acc);
-#endif
 #pragma unroll
         for (int i = k - 8; i <= 8; i++) acc = madw(m[i], p29<C>(k - i), acc);
         h[k - 9] = (uint32_t)acc & M29;

@@ -35,18 +35,6 @@ namespace h2b {
 // kernels
 // ---------------------------------------------------------------------------
 
-// lut[i] = base^(2^i), i < k.  One thread: k sequential squarings.
-__global__ void k_pow2_lut(const Fr* __restrict__ base, Fr* __restrict__ lut, int k)
-{
-    if (blockIdx.x == 0 && threadIdx.x == 0) {
-        Fr cur = ld(base);
-        for (int i = 0; i < k; i++) {
-            st(&lut[i], cur);
-            cur = cur * cur;
-        }
-    }
-}
-
 __device__ __forceinline__ Fr pow_from_lut(const Fr* __restrict__ lut, uint64_t e)
 {
     Fr r = Fr::one();
