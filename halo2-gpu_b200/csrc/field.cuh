@@ -410,7 +410,10 @@ H2B_DEV Fp<C> mont_sqr_29(const Fp<C>& a)
 // the same operands), and no carry is handled by an instruction of its own but
 // the last one of the chain.  After a reduction row e[0] is zero; dividing by
 // 2^32 swaps the roles: o becomes the even words (e[1] joins its word 0) and
-// e[2..7] the odd ones, which the next row's chains read as addends.
+// e[2..7] the odd ones, which the next row's chains read as addends.  Keeping
+// even and odd limb products apart is a known arrangement for GPU multiply-add
+// chains (CGBN and sppark's Montgomery fields use it); the rows, the square and
+// the two-product sum below are written out for eight words here.
 //
 // 128 wide multiply-adds and 8 digit products; about 205 instructions and 40
 // registers.  Measured on B200 (one chain of products per thread, 16 warps per

@@ -5,8 +5,10 @@
 // constant-time gcd computation and modular inversion", 2019) with delta
 // starting at 1/2, 30 at a time on the low words of f and g alone (a 2 x 2
 // matrix of 31-bit entries), then one pass that applies the matrix to f, g and
-// to the cofactors d, e (reduced modulo m by a 30-bit Montgomery digit).  At
-// most 590 steps are needed for 256-bit inputs; the loop ends when g is zero.
+// to the cofactors d, e (reduced modulo m by a 30-bit Montgomery digit).  The
+// start at 1/2, its bound of 590 steps for 256-bit inputs and the digit update
+// of d and e follow Wuille's write-up of the algorithm for libsecp256k1
+// (doc/safegcd_implementation.md there).  The loop ends when g is zero.
 // d starts at 0 and e at R^2, so the result is (a R)^-1 R^2 = a^-1 R without a
 // closing product.  |d| and |e| grow by at most m per pass (below 21 m; limbs
 // and sums fit 64 bits).  Inverse of zero is zero.

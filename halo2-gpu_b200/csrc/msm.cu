@@ -726,8 +726,8 @@ __global__ void __launch_bounds__(256) k_msm_heads_merge(const uint32_t* __restr
 // depth is the number of bits: running sums over 8-bucket segments and then
 // per-bit sums of the segments (16 and 16 additions one after the other at
 // c = 16) took 146 + 212 us for 8 windows of 2^15 buckets and 104 + 210 us for
-// one; the two passes here about 190 + 61 and 84 + 60 us (two CTAs per SM; one,
-// at 150 registers, made the first pass 333 us).
+// one; the two passes here 245 + 61 and 81 + 60 us (two CTAs per SM; one, at 150
+// registers, made the first pass 333 us).
 template <int THREADS, int BLOCKS>
 __global__ void __launch_bounds__(THREADS, BLOCKS) k_msm_fold(const G1Xyzz* __restrict__ in, uint32_t arrays, uint32_t len,
                                                            int m, G1Xyzz* __restrict__ out, uint32_t* __restrict__ ctr,
@@ -792,7 +792,7 @@ struct MsmFold {
 // child's leaf index.  Counters start at zero (k_msm_fold).
 // The chain is bound by product latency, two per doubling.  Measured at
 // c = 16, 8 windows: Horner over bit sums per window, then the window
-// doublings with one warp per window on one SM, 567 us; this kernel 290 us.
+// doublings with one warp per window on one SM, 567 us; this kernel 214 us.
 __global__ void __launch_bounds__(32) k_msm_tail(G1Xyzz* sums, uint32_t per, MsmFold f, int c, uint32_t leaves,
                                                  uint32_t* ctr, const __grid_constant__ MsmOuts outs)
 {
@@ -1291,7 +1291,7 @@ extern "C" void h2b_msm_set_tuning(int window_bits, int chunk) { msm_set_tuning(
 // Form of the bucket-accumulation kernel: 6 = coordinates in [0, 2p) on the
 // even/odd product (default), 0 = the lazy R = 2^261 form of 29-bit limbs with
 // one-step carries.  Measured at 2^22 with the witness-like scalar mix, the
-// whole MSM: 6 8.07 ms, 0 13.6 ms.  Results are identical; only speed differs.
+// whole MSM: 6 7.57 ms, 0 13.6 ms.  Results are identical; only speed differs.
 // Any other value leaves the setting unchanged (read it back with
 // h2b_msm_get_accumulate_variant).
 extern "C" void h2b_msm_set_accumulate_variant(int v)

@@ -20,8 +20,11 @@
 // intermediates.  Each thread walks whole rows; every thread of a warp
 // executes the same op, so there is no divergence, and column reads for
 // consecutive rows are coalesced.
-// products inline: the even/odd product is short enough that the fused kernel's
-// body still streams from the instruction cache (a 2^20 part 1.287 -> 1.250 ms)
+// operator* inline: all products of the three kernels that the reference also
+// has (2^20 rows: gates 242 -> 235 us, permutation 666 -> 617 us, lookup 282 ->
+// 257 us), and in the fused kernel the power of omega that a thread steps from
+// row to row, whose call made it spill (a 2^20 part 1.235 -> 1.186 ms).  The
+// fused kernel's formulas call one out-of-line body (zm below).
 #define H2B_INLINE_MUL 1
 #include <algorithm>
 #include <cstring>
@@ -997,7 +1000,7 @@ Fr fr_from(const void* p)
 } // namespace
 
 // Register budget of the fused kernel, in blocks of 128 threads per SM: 3
-// (168 registers), 4 (128; the default) or 5 (96).  Config-3 part on even/odd
+// (142 registers), 4 (126; the default) or 5 (96).  Config-3 part on even/odd
 // products: 2^20 rows 1247, 1205 and 1224 us, 2^16 rows 145, 135 and 136 us.
 // The products of its [0, 2p) formulas stay out of line: inline they took 1399,
 // 1458 and 1519 us at 2^20 rows.  Same results.
