@@ -121,10 +121,14 @@ static int wanted_c(uint64_t n, bool plain = false)
     // buckets, so a narrow window makes few, long buckets (2^18 points at 13
     // bits: 4096 buckets of about 1300 entries).
     // Widths from a sweep of c in 10..18 on B200 (bench.py --case
-    // table_widths; uniform / witness-mix scalars, n = table size): 2^18
-    // table 11.57 / 3.07 ms at 13 bits -> 1.80 / 1.48 ms at 16, 2^20 6.32 /
-    // 4.64 ms at 15 -> 4.91 / 3.46 ms at 16, 2^16 4.48 / 1.20 ms at 12 ->
-    // 1.02 / 0.85 ms at 13.
+    // table_widths; uniform / witness-mix scalars, n = table size, ms):
+    //   2^12: 10 bits 0.29 / 0.29, 13 bits 0.30 / 0.34
+    //   2^13: 13 bits 0.32 / 0.36, 10 bits 0.34 / 0.38
+    //   2^16: 13 bits 0.58 / 0.53, 10 bits 0.99 / 0.82, 16 bits 0.49 / 0.52
+    //   2^17: 16 bits 0.69 / 0.63, 13 bits 0.84 / 0.71
+    //   2^20: 16 bits 3.26 / 2.19, 13 bits 4.62 / 2.93
+    // (16 bits would serve 2^15 and 2^16 too; a table's layout follows this
+    // rule, and a caller may hold tables of the present one.)
     if (lg >= 17) return 16;
     if (lg >= 13) return 13;
     if (lg >= 10) return 10;
