@@ -185,3 +185,24 @@ def test_msm_accumulate_forms(h2b, orc, cuda, srs_small, variant):
         assert_limbs_equal(h2b.to_host(out, (12,)), orc.msm(mix, srs[:n]), f"table, variant {variant}")
     finally:
         L.h2b_msm_set_accumulate_variant(before)
+
+
+@pytest.mark.parametrize("c", [10, 11, 16])
+def test_msm_blocks_of_empty_buckets(h2b, orc, cuda, srs_small, c):
+    """The first folding pass leaves blocks of 512 buckets without an entry: one
+    digit at either edge of a block (the window's first and last ones, and both
+    sides of a block's border), alone or in several windows."""
+    _, srs = srs_small
+    L = h2b.lib()
+    H = 1 << (c - 1)
+    digits = sorted({1, 2, min(512, H), min(513, H), H - 1, H})
+    L.h2b_msm_set_tuning(c, 0)
+    try:
+        for d in digits:
+            for vals in ([d], [d, 0, d << (3 * c)], [1 + (H << c), 512]):
+                sc = h2b.fields.fr_mont_limbs([v % h2b.fields.R_MOD for v in vals] * 5)
+                n = sc.shape[0]
+                got = h2b.multiexp_gpu_device_scalars_device_bases(h2b.to_dev(sc), h2b.to_dev(srs[:n]), n)
+                assert_limbs_equal(got, orc.msm(sc, srs[:n]), f"c={c} digit {d}")
+    finally:
+        L.h2b_msm_set_tuning(0, 0)
